@@ -157,6 +157,17 @@ Op r_to_last_prefix(Ctx* ctx, const Op& in, const Label& r) {
   return permuted(ctx, in, perm_r_last(in->P(), in->N(), ax));
 }
 
+// The same reorder as a key-sorted view (prefix axes only move, so no block
+// changes): no copy and no launch.  Not when `written` is the operand itself:
+// its payload is overwritten while the view would still be read.
+Op r_to_last_prefix_view(Ctx* ctx, const Op& in, const Label& r, const Tensor& written) {
+  if (&in.t->owner() == &written) return r_to_last_prefix(ctx, in, r);
+  const int ax = find(in.labels, r) + 1;
+  require(ax >= 1 && ax <= in->P(), SB_ERR_LABEL, "rlab must be in prefix to use prefix kernel");
+  if (ax == in->P()) return view(*in.t, in.labels);
+  return permuted_keys_only(ctx, in, perm_r_last(in->P(), in->N(), ax));
+}
+
 enum class Mode { AthenB, BthenA, Interleaved };
 
 // _cdense_grouping_and_orders (contract_bs_bs.jl:470-505)
@@ -2000,9 +2011,9 @@ void coo_bs_prefix(Ctx* ctx, Tensor& C, const Labels& lC, const Op& A, const Op&
   AxpyPlan ap;
   for (size_t c = 0; c < ord.size(); ++c) {
     ap.add_seg(static_cast<int64_t>(c) * blk, blk);
-    for (int ci : ck.contribs[ord[c]]) ap.add(pr[ci].second * blk, pr[ci].first);
+    for (int ci : ck.contribs[ord[c]]) ap.add(B->block_off(pr[ci].second), pr[ci].first);
   }
-  ap.launch(ctx, B->data.d(), A->data.d(), C.data.d());
+  ap.launch(ctx, B->payload(), A->data.d(), C.data.d());
 }
 
 void coo_bs_dense_index(Ctx* ctx, Tensor& C, const Labels& lC, const Op& A, const Op& B0, const Label& r) {
@@ -2616,7 +2627,7 @@ void contract(Ctx* ctx, Tensor& C, const Labels& lC, const Tensor& A, const Labe
     if (c == BS && a == COO && b == BS) {
       Op A2 = coo_r_last_sorted(ctx, oA, r);
       if (find(lB, r) < B.P()) {
-        Op B2 = r_to_last_prefix(ctx, oB, r);
+        Op B2 = r_to_last_prefix_view(ctx, oB, r, C);
         return coo_bs_prefix(ctx, C, lC, A2, B2, r);
       }
       return coo_bs_dense_index(ctx, C, lC, A2, oB, r);

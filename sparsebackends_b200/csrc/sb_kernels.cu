@@ -48,20 +48,36 @@ __global__ void k_outer_acc(const double* __restrict__ A, const double* __restri
 }
 
 // ── segmented scaled accumulation ─────────────────────────────────────────
+// HBM-bound.  Each thread takes four elements a CTA stride apart, so four
+// loads per entry are in flight and an entry's descriptor and factor are read
+// once per four elements.
 __global__ void k_axpy_seg(const double* __restrict__ src, const double* __restrict__ alpha,
                            double* __restrict__ C, const AxpySeg* __restrict__ segs, int64_t nsegs,
                            const AxpyEntry* __restrict__ ents) {
+  constexpr int kPer = 4;
   for (int64_t g = blockIdx.y; g < nsegs; g += gridDim.y) {
     const AxpySeg sg = segs[g];
-    for (int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; t < sg.len;
-         t += (int64_t)gridDim.x * blockDim.x) {
-      double acc = 0.0;
+    for (int64_t t0 = (int64_t)blockIdx.x * (kPer * blockDim.x); t0 < sg.len;
+         t0 += (int64_t)gridDim.x * (kPer * blockDim.x)) {
+      const int64_t t = t0 + threadIdx.x;
+      double acc[kPer] = {0.0, 0.0, 0.0, 0.0};
       for (int e = sg.e_begin; e < sg.e_end; ++e) {
         const AxpyEntry en = ents[e];
         const double a = en.alpha_idx >= 0 ? alpha[en.alpha_idx] : 1.0;
-        acc = __dadd_rn(acc, __dmul_rn(a, src[en.src_off + t]));
+        double v[kPer];
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) {
+          const int64_t i = t + r * static_cast<int64_t>(blockDim.x);
+          v[r] = i < sg.len ? src[en.src_off + i] : 0.0;
+        }
+#pragma unroll
+        for (int r = 0; r < kPer; ++r) acc[r] = __dadd_rn(acc[r], __dmul_rn(a, v[r]));
       }
-      C[sg.c_off + t] = acc;
+#pragma unroll
+      for (int r = 0; r < kPer; ++r) {
+        const int64_t i = t + r * static_cast<int64_t>(blockDim.x);
+        if (i < sg.len) C[sg.c_off + i] = acc[r];
+      }
     }
   }
 }
@@ -88,27 +104,32 @@ __global__ void k_permute_general(const double* __restrict__ src, double* __rest
 
 // Contiguous runs: output axis 0 has unit source stride too, so every run of
 // the leading output axes that are contiguous in both layouts (len doubles) is
-// a straight copy.  One warp per run: the source offset of a run is computed
-// once, then the lanes copy it with coalesced accesses, four loads in flight
-// per lane.
+// a straight copy.  One warp per segment of a run (seg doubles, the whole run
+// when there are runs enough for every warp slot of the chip): the source
+// offset of a segment is computed once, then the lanes copy it with coalesced
+// accesses, eight loads in flight per lane.  Bound by HBM; with one warp per
+// run a reorder of two 2 MB blocks was two warps' work and took 403 us.
 __global__ void k_permute_runs(const double* __restrict__ src, double* __restrict__ dst,
                                const int64_t* __restrict__ src_off, int64_t blk, int64_t len, int64_t runs_per_block,
-                               int64_t total_runs, PermDesc d, int first_outer) {
+                               int64_t seg, int64_t segs_per_run, int64_t total, PermDesc d, int first_outer) {
   const int lane = threadIdx.x & 31;
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
-  for (int64_t run = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; run < total_runs;
-       run += warps) {
+  for (int64_t task = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; task < total;
+       task += warps) {
+    const int64_t run = segs_per_run == 1 ? task : task / segs_per_run;
+    const int64_t e0 = segs_per_run == 1 ? 0 : (task - run * segs_per_run) * seg;
+    const int64_t n = len - e0 < seg ? len - e0 : seg;
     const int64_t b = run / runs_per_block;
     int64_t rr = run - b * runs_per_block;
-    const double* s = src + src_off[b];
-    double* o = dst + b * blk + rr * len;
+    const double* s = src + src_off[b] + e0;
+    double* o = dst + b * blk + rr * len + e0;
     for (int r = first_outer; r < d.rank; ++r) {
       const int64_t c = rr % d.out_dims[r];
       rr /= d.out_dims[r];
       s += c * d.in_strides[r];
     }
-#pragma unroll 4
-    for (int64_t e = lane; e < len; e += 32) o[e] = s[e];
+#pragma unroll 8
+    for (int64_t e = lane; e < n; e += 32) o[e] = s[e];
   }
 }
 
@@ -498,7 +519,7 @@ cudaError_t launch_outer_acc(const double* A, const double* B, double* C, const 
 cudaError_t launch_axpy_seg(const double* src, const double* d_alpha, double* C, const AxpySeg* d_segs,
                             int64_t nsegs, const AxpyEntry* d_entries, int64_t max_len, cudaStream_t s) {
   if (nsegs <= 0 || max_len <= 0) return cudaSuccess;
-  dim3 grid(grid_for(max_len), static_cast<unsigned>(nsegs < 65535 ? nsegs : 65535));
+  dim3 grid(grid_for(max_len, 4 * kThreads), static_cast<unsigned>(nsegs < 65535 ? nsegs : 65535));
   if ((int64_t)grid.x * grid.y > 148LL * 64) grid.x = static_cast<unsigned>(std::max<int64_t>(1, 148LL * 64 / grid.y));
   k_axpy_seg<<<grid, kThreads, 0, s>>>(src, d_alpha, C, d_segs, nsegs, d_entries);
   return cudaGetLastError();
@@ -518,10 +539,15 @@ cudaError_t launch_permute_blocks(const double* src, double* dst, const int64_t*
     int64_t len = desc.out_dims[0];
     while (j < desc.rank && desc.in_strides[j] == len) len *= desc.out_dims[j++];
     if (len >= 32) {
-      const int64_t runs = blk / len, total = nblocks * runs;
+      // long runs are cut (not below 1024 doubles) until every warp slot of
+      // the chip has a segment
+      const int64_t runs = blk / len, nruns = nblocks * runs;
+      int64_t seg = len;
+      while (nruns * ((len + seg - 1) / seg) < 148LL * 64 && seg >= 2048) seg = (seg / 2 + 31) / 32 * 32;
+      const int64_t spr = (len + seg - 1) / seg, total = nruns * spr;
       const int64_t ctas = std::min<int64_t>((total + 7) / 8, 148LL * 8);
       k_permute_runs<<<static_cast<unsigned>(std::max<int64_t>(ctas, 1)), kThreads, 0, s>>>(
-          src, dst, d_src_off, blk, len, runs, total, desc, j);
+          src, dst, d_src_off, blk, len, runs, seg, spr, total, desc, j);
       return cudaGetLastError();
     }
   }

@@ -1,0 +1,49 @@
+"""The streaming kernels at the sizes where their work split changes: run
+copies cut into segments, and scaled accumulation with four elements per
+thread.  Both only move or add values in a fixed order, so results equal the
+oracle's bit for bit."""
+import numpy as np
+import pytest
+
+from oracle import sparse_oracle as so
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("nblocks", [1, 2, 7])
+@pytest.mark.parametrize("tail", [(31, 1), (32, 3), (1023, 2), (2049, 1), (4999, 7), (70001, 1)])
+def test_prefix_reorder_copies_long_runs(nblocks, tail):
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(tail[0] + nblocks))
+    pre = (3, 3)
+    keys = sorted([(1 + i % 3, 1 + i // 3) for i in range(nblocks)], key=lambda k: k[::-1])
+    data = rng.standard_normal(nblocks * tail[0] * tail[1])
+    A = sb.NewBlockSparseSorted(pre + tail, 2, keys, None, data)
+    R = so.BS(pre + tail, 2, keys, list(range(1, nblocks + 1)), data)
+    P, W = sb.permutedims(A, [2, 1, 3, 4]), so.bs_permutedims(R, [2, 1, 3, 4])
+    assert P.keys == W.keys
+    got, want = P.blocks_by_key(), W.blocks_by_key()
+    assert all(np.array_equal(got[k], np.ravel(want[k], order="F")) for k in want)
+
+
+@pytest.mark.parametrize("length", [1, 255, 1023, 1024, 1025, 4097])
+@pytest.mark.parametrize("first", [True, False])  # the reduced label last in the prefix, or reordered by a view
+def test_coo_times_blocks_bit_exact(length, first):
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(length))
+    ck = [(a, s) for s in (1, 2, 3) for a in (1, 2, 4)]
+    cv = rng.standard_normal(len(ck))
+    bk = [(q, s) for s in (1, 2, 3) for q in (1, 2)]
+    data = rng.standard_normal(len(bk) * length)
+    A, RA = sb.COOTensor((4, 3), ck, cv), so.COO((4, 3), ck, cv)
+    B = sb.NewBlockSparseSorted((2, 3, length), 1, bk, None, data)
+    RB = so.BS((2, 3, length), 1, bk, list(range(1, len(bk) + 1)), data)
+    lB = ["q", "s", "x"]
+    if not first:
+        B, RB, lB = sb.permutedims(B, [2, 1, 3]), so.bs_permutedims(RB, [2, 1, 3]), ["s", "q", "x"]
+    C = sb.NewBlockSparseSorted.empty((4, 2, length), 1)
+    sb.contract_(C, ["a", "q", "x"], A, ["a", "s"], B, lB)
+    W = so.contract(so.BS.empty((4, 2, length), 1), ["a", "q", "x"], RA, ["a", "s"], RB, lB)
+    assert C.keys == W.keys
+    got, want = C.blocks_by_key(), W.blocks_by_key()
+    assert all(np.array_equal(got[k], np.ravel(want[k], order="F")) for k in want)
