@@ -657,28 +657,31 @@ cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* 
 // ext[b*n2 + r] = 1 + the largest axis-r coordinate of a nonzero element
 // (ext holds 1s on entry).  A block is a column-major matrix of d0 rows
 // (axis 0) and cols columns (the other axes, flattened).  Work comes in warp
-// tasks, task_begin[b] .. task_begin[b+1] for block b, in one of three forms
-// fixed by (d0, cols) alone (ext_task_shape): rows of one column split into
-// 8192-long segments (cols == 1); a run of columns, one at a time by the whole
-// warp (d0 >= 32); 2048 columns, one lane per column (d0 < 32).  A column with
-// a nonzero entry has its other coordinates decomposed once; the maxima go to
-// ext with one atomicMax per axis and task.
-__host__ __device__ inline int64_t ext_task_cols(int64_t d0, int64_t cols) {
+// tasks of about `budget` elements, task_begin[b] .. task_begin[b+1] for block
+// b, in one of three forms fixed by (d0, cols): rows of one column split into
+// segments (cols == 1); a run of columns, one at a time by the whole warp
+// (d0 >= 32); one lane per column (d0 < 32).  A column with a nonzero entry
+// has its other coordinates decomposed once; the maxima go to ext with one
+// atomicMax per axis and task.  The scan is HBM-bound on large operands and a
+// chain of dependent column loads on small ones, so the budget shrinks until
+// every warp slot has a task (block_extent_budget): four 256 x 256 blocks took
+// 47 us as 32 warps of 32 columns each.
+__host__ __device__ inline int64_t ext_task_cols(int64_t d0, int64_t cols, int64_t budget) {
   if (cols == 1) return 1;
-  if (d0 < 32) return 2048;
-  const int64_t per = 8192 / d0;
+  if (d0 < 32) return budget / 4 < 32 ? 32 : budget / 4 / 32 * 32;
+  const int64_t per = budget / d0;
   return per < 1 ? 1 : per > 32 ? 32 : per;
 }
-__host__ __device__ inline int64_t ext_tasks(int64_t d0, int64_t cols) {
+__host__ __device__ inline int64_t ext_tasks(int64_t d0, int64_t cols, int64_t budget) {
   if (d0 == 0 || cols == 0) return 0;
-  if (cols == 1) return (d0 + 8191) / 8192;
-  const int64_t per = ext_task_cols(d0, cols);
+  if (cols == 1) return (d0 + budget - 1) / budget;
+  const int64_t per = ext_task_cols(d0, cols, budget);
   return (cols + per - 1) / per;
 }
 
 __global__ void k_block_extents(const double* __restrict__ src, const int64_t* __restrict__ off,
                                 const int64_t* __restrict__ dims, const int64_t* __restrict__ task_begin,
-                                int64_t nblocks, int n2, int* __restrict__ ext) {
+                                int64_t nblocks, int n2, int64_t budget, int* __restrict__ ext) {
   const int lane = threadIdx.x & 31;
   const int64_t ntasks = task_begin[nblocks];
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
@@ -706,13 +709,13 @@ __global__ void k_block_extents(const double* __restrict__ src, const int64_t* _
       }
     };
     if (cols == 1 || d0 >= 32) {
-      const int64_t per = ext_task_cols(d0, cols);
+      const int64_t per = ext_task_cols(d0, cols, budget);
       const int64_t c0 = cols == 1 ? 0 : t * per, c1 = cols == 1 ? 1 : (c0 + per < cols ? c0 + per : cols);
-      const int64_t r0 = cols == 1 ? t * 8192 : 0, r1 = cols == 1 ? (r0 + 8192 < d0 ? r0 + 8192 : d0) : d0;
+      const int64_t r0 = cols == 1 ? t * budget : 0, r1 = cols == 1 ? (r0 + budget < d0 ? r0 + budget : d0) : d0;
       for (int64_t c = c0; c < c1; ++c) {
         const double* col = base + c * d0;
         int64_t m = 0;
-#pragma unroll 4
+#pragma unroll 8
         for (int64_t r = r0 + lane; r < r1; r += 32)
           if (col[r] != 0.0) m = r + 1;
         if (__any_sync(0xffffffffu, m > 0)) {
@@ -722,7 +725,8 @@ __global__ void k_block_extents(const double* __restrict__ src, const int64_t* _
       }
     } else {
       // one lane per column; the warp's 32 columns are one contiguous run
-      const int64_t c0 = t * 2048, c1 = c0 + 2048 < cols ? c0 + 2048 : cols;
+      const int64_t per = ext_task_cols(d0, cols, budget);
+      const int64_t c0 = t * per, c1 = c0 + per < cols ? c0 + per : cols;
       for (int64_t c = c0 + lane; c < c1; c += 32) {
         const double* col = base + c * d0;
         int64_t m = 0;
@@ -750,16 +754,20 @@ __global__ void k_block_extents(const double* __restrict__ src, const int64_t* _
   }
 }
 
-int64_t block_extent_tasks(int64_t d0, int64_t cols) { return ext_tasks(d0, cols); }
+int64_t block_extent_budget(int64_t elems) {
+  const int64_t b = elems / (148LL * 48);
+  return b < 512 ? 512 : b > 8192 ? 8192 : b;
+}
+int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget) { return ext_tasks(d0, cols, budget); }
 
 cudaError_t launch_block_extents(const double* src, const int64_t* d_off, const int64_t* d_dims,
-                                 const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2, int* d_ext,
-                                 cudaStream_t s) {
+                                 const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2,
+                                 int64_t budget, int* d_ext, cudaStream_t s) {
   if (ntasks <= 0 || nblocks <= 0) return cudaSuccess;
   if (n2 < 1 || n2 > kMaxRank) return cudaErrorInvalidValue;
   const int64_t ctas = std::min<int64_t>((ntasks + 7) / 8, 148LL * 8);
   k_block_extents<<<static_cast<unsigned>(ctas), kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, n2,
-                                                                    d_ext);
+                                                                    budget, d_ext);
   return cudaGetLastError();
 }
 

@@ -321,6 +321,7 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
     const int64_t n = A.nkeys;
     if (n == 0 || A.n2 == 0) continue;
     std::vector<int64_t> off(n), dims(n * A.n2), tb(n + 1, 0);
+    const int64_t budget = block_extent_budget(A.payload_len());
     for (int64_t i = 0; i < n; ++i) {
       off[i] = A.block_off(i);
       int64_t cols = 1;
@@ -328,14 +329,15 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
         dims[i * A.n2 + t] = A.block_dim(i, t);
         if (t > 0) cols *= dims[i * A.n2 + t];
       }
-      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols);
+      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols, budget);
     }
     keep.push_back(upload(ctx, off));
     keep.push_back(upload(ctx, dims));
     keep.push_back(upload(ctx, tb));
     const size_t m = keep.size();
     SB_CK(launch_block_extents(A.payload(), keep[m - 3].as<int64_t>(), keep[m - 2].as<int64_t>(),
-                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, dext.as<int>() + base[k], ctx->stream));
+                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, budget,
+                               dext.as<int>() + base[k], ctx->stream));
     ctx->note_launch();
   }
   const auto e = download<int>(ctx, dext.raw(), base.back());

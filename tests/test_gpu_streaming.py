@@ -47,3 +47,26 @@ def test_coo_times_blocks_bit_exact(length, first):
     assert C.keys == W.keys
     got, want = C.blocks_by_key(), W.blocks_by_key()
     assert all(np.array_equal(got[k], np.ravel(want[k], order="F")) for k in want)
+
+
+@pytest.mark.parametrize("tail", [(1, 1), (31, 70), (32, 5), (33, 600), (600, 33), (5000, 1), (9, 40, 21), (515, 515)])
+@pytest.mark.parametrize("nblocks", [1, 6])
+def test_zero_padding_scan_extents(tail, nblocks):
+    """Extents found by the scan, for every form of its tasks (rows of one
+    column, runs of columns, a lane per column), with one nonzero entry on each
+    block's true corner and none at all in the last block."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(sum(tail) + nblocks))
+    keys = [(i + 1,) for i in range(nblocks)]
+    blocks, want = [], []
+    for i in range(nblocks):
+        b = np.zeros(tail)
+        e = (1,) * len(tail)
+        if i + 1 < nblocks or nblocks == 1:
+            e = tuple(int(rng.integers(1, t + 1)) for t in tail)
+            b[tuple(x - 1 for x in e)] = 1e-300
+            b[tuple(int(rng.integers(0, x)) for x in e)] = 2.0
+        blocks.append(b.reshape(-1, order="F"))
+        want.append(e)
+    A = sb.NewBlockSparseSorted((nblocks,) + tail, len(tail), keys, None, np.concatenate(blocks))
+    assert sb.crop_padding(A).block_dims == want
