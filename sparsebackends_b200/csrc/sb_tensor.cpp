@@ -241,6 +241,34 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
     }
   }
   rows = rows && elems >= 16 * nrows;
+  // otherwise tiles, when no item pads or crops; else the per-element gather,
+  // which is also the quicker one on a few thousand elements, where a tile's
+  // two dependent phases cost more than they save (11 000 elements: 6.6 to 8.0
+  // us against 7.7 to 8.8; 215 000: 11.5 to 11.9 against 8.8 to 10.3)
+  std::vector<PermTileItem> pt;
+  std::vector<int64_t> tb;
+  int64_t tiles = 0;
+  const uint32_t cap = perm_tile_cap(static_cast<int64_t>(bytes / 16));
+  if (!rows && bytes >= 16.0 * (1 << 15)) {
+    pt.resize(items.size());
+    for (auto& it : items) {
+      int64_t t = 0;
+      if (!perm_tile_item(it, cap, &pt[tb.size()], &t)) {
+        tb.clear();
+        break;
+      }
+      tb.push_back(tiles);
+      tiles += t;
+    }
+  }
+  if (!tb.empty()) {
+    DevBuf d = upload(ctx, pt), dtb = upload(ctx, tb);
+    ProfScope ps(ctx, PROF_PERMUTE, 0.0, bytes);
+    SB_CK(launch_perm_block_tiles(src, dst, d.as<PermTileItem>(), dtb.as<int64_t>(),
+                                  static_cast<int64_t>(items.size()), tiles, cap, ctx->stream));
+    ctx->note_launch();
+    return;
+  }
   DevBuf d = upload(ctx, items);
   ProfScope ps(ctx, PROF_PERMUTE, 0.0, bytes);
   if (rows)
