@@ -387,8 +387,7 @@ constexpr int kPermTileElems = 64 * 65;
 constexpr int kPermTileRows = 1024;  // largest tv
 __global__ void __launch_bounds__(256, 6)
     k_perm_block_tiles(const double* __restrict__ src, double* __restrict__ dst,
-                       const PermTileItem* __restrict__ items, const int64_t* __restrict__ tile_begin, int64_t n,
-                       int64_t total) {
+                       const PermTileItem* __restrict__ items, int64_t n, int64_t total) {
   extern __shared__ double ptile[];
   __shared__ int32_t row_off[kPermTileRows];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -397,13 +396,13 @@ __global__ void __launch_bounds__(256, 6)
     int64_t lo = 0, hi = n - 1;
     while (lo < hi) {
       const int64_t step = (hi - lo + 32) / 32, idx = lo + (lane + 1) * step;
-      const int k = __popc(__ballot_sync(0xffffffffu, idx <= hi && tile_begin[idx] <= task));
+      const int k = __popc(__ballot_sync(0xffffffffu, idx <= hi && items[idx].tile_begin <= task));
       lo += k * step;
       hi = hi < lo + step - 1 ? hi : lo + step - 1;
     }
     const PermTileItem& it = items[lo];
     const uint32_t du = it.du, dv = it.dv, tu = it.tu, tv = it.tv;
-    uint32_t t = static_cast<uint32_t>(task - tile_begin[lo]);
+    uint32_t t = static_cast<uint32_t>(task - it.tile_begin);
     const uint32_t u0 = (t % it.tiles_u) * tu;
     t /= it.tiles_u;
     const uint32_t v0 = (t % it.tiles_v) * tv;
@@ -749,6 +748,9 @@ bool perm_tile_item(const BlockPerm& b, uint32_t cap, PermTileItem* out, int64_t
     if (b.in_strides[r] == 1 && b.out_dims[r] > 1) p.q = r;
   }
   if (b.out_dims[p.q] > 1 && b.in_strides[p.q] != 1) return false;
+  // output axis 0 contiguous in the source too (crops, outer-axis reorders):
+  // a tile would hold one row of axis 0, so only long rows qualify
+  if (p.q == 0 && p.dims[0] < 256 && b.len > p.dims[0]) return false;
   int64_t nbatch = 1;
   p.dv = 1;
   for (int r = 0; r < p.q; ++r) p.dv *= p.dims[r];
@@ -775,14 +777,13 @@ bool perm_tile_item(const BlockPerm& b, uint32_t cap, PermTileItem* out, int64_t
   return true;
 }
 
-cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items,
-                                    const int64_t* d_tile_begin, int64_t n, int64_t total, uint32_t cap,
-                                    cudaStream_t s) {
+cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items, int64_t n,
+                                    int64_t total, uint32_t cap, cudaStream_t s) {
   if (n <= 0 || total <= 0) return cudaSuccess;
   if (cap > kPermTileElems) return cudaErrorInvalidValue;
   const int smem = static_cast<int>(cap) * static_cast<int>(sizeof(double));
   const unsigned g = static_cast<unsigned>(std::min<int64_t>(total, 148LL * 6));
-  k_perm_block_tiles<<<g, 256, smem, s>>>(src, dst, d_items, d_tile_begin, n, total);
+  k_perm_block_tiles<<<g, 256, smem, s>>>(src, dst, d_items, n, total);
   return cudaGetLastError();
 }
 

@@ -220,18 +220,18 @@ cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* 
 // false when it does not qualify (limits below the output extents, 2^31
 // elements or more); cap = elements of shared memory per tile (perm_tile_cap:
 // 1056 to 4160 by the elements moved, so that small operands make enough tiles
-// for the chip); d_tile_begin[i] = tiles before item i; total = all tiles.
+// for the chip).  The caller sets tile_begin = tiles before the item; total =
+// all tiles.
 struct PermTileItem {
-  int64_t src_off, dst_off;
+  int64_t src_off, dst_off, tile_begin;
   int32_t rank, q;  // q: the output axis that is contiguous in the source
   uint32_t dv, du, tv, tu, tiles_u, tiles_v;
   uint32_t dims[kMaxRank], strides[kMaxRank];
 };
 uint32_t perm_tile_cap(int64_t elems);
 bool perm_tile_item(const BlockPerm& it, uint32_t cap, PermTileItem* out, int64_t* tiles);
-cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items,
-                                    const int64_t* d_tile_begin, int64_t n, int64_t total, uint32_t cap,
-                                    cudaStream_t s);
+cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items, int64_t n,
+                                    int64_t total, uint32_t cap, cudaStream_t s);
 // The same for items whose out_dims[0] has in_strides[0] == 1 (one warp per
 // row of out_dims[0]); max_rows = the largest len / out_dims[0].
 cudaError_t launch_perm_block_rows(const double* src, double* dst, const BlockPerm* d_items, int64_t n,

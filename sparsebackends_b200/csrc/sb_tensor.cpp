@@ -246,26 +246,25 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
   // two dependent phases cost more than they save (11 000 elements: 6.6 to 8.0
   // us against 7.7 to 8.8; 215 000: 11.5 to 11.9 against 8.8 to 10.3)
   std::vector<PermTileItem> pt;
-  std::vector<int64_t> tb;
   int64_t tiles = 0;
   const uint32_t cap = perm_tile_cap(static_cast<int64_t>(bytes / 16));
   if (!rows && bytes >= 16.0 * (1 << 15)) {
     pt.resize(items.size());
-    for (auto& it : items) {
+    for (size_t i = 0; i < items.size(); ++i) {
       int64_t t = 0;
-      if (!perm_tile_item(it, cap, &pt[tb.size()], &t)) {
-        tb.clear();
+      if (!perm_tile_item(items[i], cap, &pt[i], &t)) {
+        pt.clear();
         break;
       }
-      tb.push_back(tiles);
+      pt[i].tile_begin = tiles;
       tiles += t;
     }
   }
-  if (!tb.empty()) {
-    DevBuf d = upload(ctx, pt), dtb = upload(ctx, tb);
+  if (!pt.empty()) {
+    DevBuf d = upload(ctx, pt);
     ProfScope ps(ctx, PROF_PERMUTE, 0.0, bytes);
-    SB_CK(launch_perm_block_tiles(src, dst, d.as<PermTileItem>(), dtb.as<int64_t>(),
-                                  static_cast<int64_t>(items.size()), tiles, cap, ctx->stream));
+    SB_CK(launch_perm_block_tiles(src, dst, d.as<PermTileItem>(), static_cast<int64_t>(pt.size()), tiles, cap,
+                                  ctx->stream));
     ctx->note_launch();
     return;
   }

@@ -88,3 +88,19 @@ def test_ragged_permute_tiles(tperm, top):
     want = {(1, i + 1): np.transpose(b, [t - 1 for t in tperm]).reshape(-1, order="F") for i, b in enumerate(blocks)}
     got = P.blocks_by_key()
     assert set(got) == set(want) and all(np.array_equal(got[k], want[k]) for k in want)
+
+
+def test_crop_of_short_rows_stays_off_the_tiles():
+    """Cropping blocks whose first axis is short (axis 0 contiguous on both
+    sides): one row of it would be a whole tile, so the gather keeps them."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(5))
+    tail, ext = (14, 60, 90), (11, 51, 77)
+    b = np.zeros((3,) + tail)
+    b[(slice(None),) + tuple(slice(0, e) for e in ext)] = rng.standard_normal((3,) + ext)
+    A = sb.NewBlockSparseSorted((3,) + tail, 3, [(1,), (2,), (3,)], None,
+                                np.concatenate([x.reshape(-1, order="F") for x in b]))
+    R = sb.to_ragged(A, [ext] * 3)
+    got = R.blocks_by_key()
+    for i in range(3):
+        assert np.array_equal(got[(i + 1,)], b[i][tuple(slice(0, e) for e in ext)].reshape(-1, order="F"))
