@@ -80,7 +80,11 @@ SB_API int64_t sb_ctx_launch_count(const sb_ctx* ctx);
  * ta/contract_bs_bs.jl:716-723 and ta/contract_bs_dense.jl:576-611, which the
  * reference runs in FP64).  Tensors stay FP64 unless created with
  * sb_tensor_create_bs_f32.
- *   SB_PRECISION_F64    FP64 tensor-core (DMMA) GEMMs, the drop-in (default);
+ *   SB_PRECISION_F64    FP64, the drop-in (default): DMMA tensor cores, and for
+ *                       large launches exact 8-bit integer products on the
+ *                       tcgen05 tensor cores (operands to 55 bits of each
+ *                       row's and column's largest magnitude; rows beyond
+ *                       2^+-400, infinities and NaN go to DMMA);
  *   SB_PRECISION_TF32X3 tcgen05 tensor cores: every operand value rounded
  *                       to FP32 and split into TF32 hi + lo, the three
  *                       significant products accumulated in FP32 chunks of
@@ -111,7 +115,8 @@ SB_API sb_status sb_ctx_set_profiling(sb_ctx* ctx, int enable);
  * 2 = outer-product accumulation, 3 = segmented axpy, 4 = other (QR/SVD,
  * gathers), 5 = vector-space operations, 6 = thin block GEMM (K <= 16),
  * 7 = tensor-core (tcgen05) block GEMM, 8 = packing of its operands (TF32
- * hi/lo split into the tensor core's shared-memory image layout).
+ * hi/lo split, or 8-bit digits of FP64, in the tensor core's shared-memory
+ * image layout).
  * Synchronises the context stream.                                           */
 SB_API sb_status sb_ctx_profile_summary(sb_ctx* ctx, int kind, int64_t* launches, double* total_ms,
                                         double* flops, double* bytes);

@@ -124,6 +124,7 @@ sb_status sb_ctx_create(int device, unsigned flags, sb_ctx** out) {
     }
     if (const char* th = std::getenv("SPARSEB_GEMM_THIN")) c->impl.gemm_thin = std::atoi(th);
     if (const char* ge = std::getenv("SPARSEB_GEMM_EDGES")) c->impl.gemm_edges = std::atoi(ge);
+    if (const char* i8 = std::getenv("SPARSEB_GEMM_I8")) c->impl.gemm_i8 = std::atoi(i8) != 0 ? 1 : 0;
     if (const char* pc = std::getenv("SPARSEB_PLAN_CACHE")) c->impl.plan_cache_on = std::atoi(pc) != 0;
     if (const char* ac = std::getenv("SPARSEB_AUTO_CROP")) c->impl.auto_crop = std::atoi(ac);
     if (const char* sk = std::getenv("SPARSEB_GEMM_SPLITK")) c->impl.gemm_splitk = std::max(0, std::atoi(sk));

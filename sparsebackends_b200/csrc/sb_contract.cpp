@@ -21,12 +21,14 @@
 //                              contract_aliased_shared.jl
 //   bs_bs_to_dense()           contract_bs_bs.jl:736-754
 #include <algorithm>
+#include <array>
 #include <climits>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <tuple>
 #include <numeric>
+#include <queue>
 #include <unordered_map>
 
 #include "sb_internal.hpp"
@@ -271,8 +273,8 @@ void reset_output(Ctx* ctx, Tensor& C, int64_t nkeys, int64_t payload) {
 // parameters, so that a contraction with an unchanged block structure can be
 // launched again without planning or uploads (the plan cache of shared_bb).
 struct GemmLaunch {
-  enum Kind { NONE, THIN, TILED, EDGES, TC } kind = NONE;
-  DevBuf dc, dp, dt, dsplit;
+  enum Kind { NONE, THIN, TILED, EDGES, TC, I8 } kind = NONE;
+  DevBuf dc, dp, dt, dsplit, dfirst;
   int32_t ncb = 0;
   int64_t n = 0;  // strips (thin) or tiles
   bool xT = false, yT = false, small_rows = false, persistent = false;
@@ -295,8 +297,54 @@ struct GemmLaunch {
   mutable const void* pk_a_src = nullptr;
   mutable const void* pk_b_src = nullptr;
   mutable uint64_t pk_a_ver = 0, pk_b_ver = 0;
+  // integer tensor-core launches (launch_gemm_i8): tiles, splits, packs and
+  // images as above, nscale operand rows; nf = 64x64 tiles of the DMMA launch
+  // behind the flag
+  int64_t nscale = 0, nf = 0;
+  int32_t nctas = 0;
   double flops = 0.0, bytes = 0.0;
   char desc[sizeof(Ctx::gemm_desc)] = "";
+  // Integer tensor-core launch.  One stream-ordered scratch buffer per call
+  // (packed planes, scales and flag, partial tiles); nothing is kept from one
+  // call to the next.  Without memory for it the DMMA launch runs instead.
+  void run_i8(Ctx* ctx, const double* X, const double* Y, double* C) const {
+    std::memcpy(ctx->gemm_desc, desc, sizeof(desc));
+    auto up = [](int64_t v) { return (v + 1023) / 1024 * 1024; };
+    const int64_t sc_off = up(pack_a_bytes + pack_b_bytes), sc_bytes = up((nscale + 1) * 4),
+                  part_off = sc_off + sc_bytes, total = part_off + nparts * kI8PartElems * 8;
+    DevBuf scratch;
+    try {
+      scratch = DevBuf(ctx, total);
+    } catch (const Error& e) {
+      if (e.code != SB_ERR_OOM) throw;
+    }
+    if (!scratch.raw()) {
+      ProfScope ps(ctx, PROF_GEMM, flops, bytes);
+      SB_CK(launch_gemm_f64_fallback(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), nf, xT, yT, nullptr,
+                                     ctx->stream));
+      ctx->note_launch();
+      return;
+    }
+    unsigned char* const b = scratch.as<unsigned char>();
+    uint32_t* const rowhi = reinterpret_cast<uint32_t*>(b + sc_off);
+    int* const flag = reinterpret_cast<int*>(rowhi + nscale);
+    SB_CK(cudaMemsetAsync(rowhi, 0, (nscale + 1) * 4, ctx->stream));
+    {
+      ProfScope ps(ctx, PROF_TC_PACK, 0.0,
+                   16.0 * (pack_a_elems + pack_b_elems) + static_cast<double>(pack_a_bytes + pack_b_bytes));
+      SB_CK(launch_i8_pack(X, dimg_a.as<I8Image>(), nimg_a, rowhi, b, flag, ctx->stream));
+      SB_CK(launch_i8_pack(Y, dimg_b.as<I8Image>(), nimg_b, rowhi, b, flag, ctx->stream));
+    }
+    {
+      ProfScope ps(ctx, PROF_GEMM, flops, bytes);
+      SB_CK(launch_gemm_i8(b, C, dc.as<GemmCBlock>(), dpk.as<I8Pack>(), rowhi, dt.as<TcTile>(),
+                           dfirst.as<int32_t>(), nctas, static_cast<int32_t>(n), nz_begin, reinterpret_cast<double*>(b + part_off),
+                           dsplit.as<TcSplit>(), nsplits, flag, ctx->stream));
+      SB_CK(launch_gemm_f64_fallback(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), nf, xT, yT, flag,
+                                     ctx->stream));
+    }
+    ctx->note_launch((nimg_a > 0 ? 2 : 0) + (nimg_b > 0 ? 2 : 0) + (nsplits > 0 ? 3 : 2));
+  }
   // Tensor-core launch: X and Y FP64 or FP32 arrays (versions 0 = unknown,
   // packed every call), C FP64 or FP32.
   void run_tc(Ctx* ctx, const void* X, bool x64, uint64_t xver, const void* Y, bool y64, uint64_t yver, void* C,
@@ -371,6 +419,10 @@ struct GemmLaunch {
     if (kind == NONE) return;
     if (kind == TC) {
       run_tc(ctx, X, true, 0, Y, true, 0, C, true);  // no tensors: packed every call
+      return;
+    }
+    if (kind == I8) {
+      run_i8(ctx, X, Y, C);
       return;
     }
     std::memcpy(ctx->gemm_desc, desc, sizeof(desc));
@@ -490,6 +542,7 @@ struct GemmPlan {
       prepare_tc(ctx, g, flops, bytes);
       return g;
     }
+    if (f32mask == 0 && prepare_i8(ctx, g, flops, bytes)) return g;
     // Tile shape from the FLOP-weighted block shape (ragged launches mix
     // large and small blocks; the heavy ones decide).
     double wm = 0.0, wn = 0.0, wsum = 0.0;
@@ -713,6 +766,186 @@ struct GemmPlan {
     std::snprintf(g.desc, sizeof(g.desc), "tcgen05 %s 128xN%s items:%lld split:%d chunk:%d%s",
                   g.passes == 3 ? "3xtf32" : "tf32", swap ? " swapped" : "", static_cast<long long>(g.n), g.nsplits,
                   g.kc, g.fold ? " fold" : "");
+  }
+
+  // FP64 launch on the integer tensor cores (launch_gemm_i8).  Tiles of 128 rows
+  // of X by nbs columns of Y (as few tiles of at most 128 columns as cover the
+  // block, of equal width rounded up to 16); each distinct operand block is
+  // packed once.  Returns false, leaving the launch to DMMA, unless the
+  // estimated time is below DMMA's.  The estimate: clocks per k-tile and per
+  // drained chunk over the SMs, the packing's bytes and 30 us of launches,
+  // against 27 TFLOP/s.  Measured (H_eff steps, us, with
+  // packing): psi*L at chi = 2048 1030 against 1831 with DMMA, R*T3 1280
+  // against 1911; chi = 1024 psi*L 247 against 284, R*T3 346 against 333;
+  // chi = 700 139 against 109: small blocks pad to 128-row tiles and 64-deep
+  // k-tiles, and every chunk pays its drain.
+  bool prepare_i8(Ctx* ctx, GemmLaunch& g, double flops, double bytes) {
+    if (ctx->gemm_i8 == 0 || ctx->gemm_tile >= 0 || ctx->autotune) return false;
+    if (ctx->gemm_i8 < 0 && flops < 2e8) return false;
+    auto up = [](int64_t v, int64_t m) { return (v + m - 1) / m * m; };
+    auto width = [&](int64_t n) {
+      const int64_t t = (n + kI8MaxN - 1) / kI8MaxN;
+      return up((n + t - 1) / t, 16);
+    };
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    struct Geo { int32_t c, a0, b0, nb; };
+    std::vector<Geo> geo, zero;
+    std::vector<int64_t> kt_of(cbs.size(), 0), chunks_of(cbs.size(), 0);
+    int64_t total_kt = 0, nf = 0;
+    double cycles = 0.0;
+    // clocks of one k-tile (operand reads of its 68 MMAs and the copies, at 128
+    // bytes per clock of shared memory) and of draining one chunk's accumulators
+    auto mma_cycles = [](int64_t nb) { return 2880.0 + 22.5 * static_cast<double>(nb); };
+    auto drain_cycles = [](int64_t nb) { return 2000.0 + 66.0 * static_cast<double>(nb); };
+    for (size_t c = 0; c < cbs.size(); ++c) {
+      for (int p = cbs[c].pair_begin; p < cbs[c].pair_end; ++p) {
+        const int64_t kt = (pairs[p].K + 63) / 64;
+        kt_of[c] += kt;
+        chunks_of[c] += (kt + kI8Chunk - 1) / kI8Chunk;
+      }
+      const int64_t nbs = width(cbs[c].N);
+      for (int64_t a0 = 0; a0 < cbs[c].M; a0 += 128)
+        for (int64_t b0 = 0; b0 < cbs[c].N; b0 += nbs) {
+          const Geo t{static_cast<int32_t>(c), static_cast<int32_t>(a0), static_cast<int32_t>(b0),
+                      static_cast<int32_t>(std::min(nbs, up(cbs[c].N - b0, 16)))};
+          (kt_of[c] > 0 ? geo : zero).push_back(t);
+          total_kt += kt_of[c];
+          cycles += kt_of[c] * mma_cycles(t.nb) + drain_cycles(t.nb) * chunks_of[c];
+        }
+      nf += ((cbs[c].M + 63) / 64) * ((cbs[c].N + 63) / 64);
+    }
+    if (nf >= (1LL << 31) || geo.size() >= (1ULL << 30)) return false;
+    // packed images: every distinct operand block once
+    const bool akc = g.xT, bkc = !g.yT;
+    std::vector<I8Pack> pk(pairs.size(), I8Pack{});
+    std::vector<I8Image> ia, ib;
+    struct Seen { int64_t base, scale; };
+    std::map<std::array<int64_t, 4>, Seen> sa, sb;  // (offset, ld, K, rows)
+    int64_t total = 0, nscale = 0, elems_a = 0, elems_b = 0;
+    auto add = [&](std::map<std::array<int64_t, 4>, Seen>& seen, std::vector<I8Image>& out, int64_t& elems, int64_t off,
+                   int64_t ld, int64_t K, int64_t rows, int64_t tile, bool kc) -> Seen {
+      auto it = seen.find({off, ld, K, rows});
+      if (it != seen.end()) return it->second;
+      const Seen s{total, nscale};
+      for (int64_t r0 = 0; r0 < rows; r0 += tile)
+        for (int64_t k0 = 0; k0 < K; k0 += 64) {
+          out.push_back(I8Image{off + (kc ? r0 * ld + k0 : r0 + k0 * ld), ld, total,
+                                static_cast<int32_t>(nscale + r0), static_cast<int32_t>(std::min(tile, rows - r0)),
+                                static_cast<int32_t>(tile), static_cast<int32_t>(std::min<int64_t>(64, K - k0)),
+                                kc ? 1 : 0, 0});
+          total += 7 * tile * 64;
+        }
+      elems += rows * K;
+      nscale += rows;
+      seen.emplace(std::array<int64_t, 4>{off, ld, K, rows}, s);
+      return s;
+    };
+    for (size_t c = 0; c < cbs.size(); ++c)
+      for (int p = cbs[c].pair_begin; p < cbs[c].pair_end; ++p) {
+        const GemmPair& q = pairs[p];
+        const int64_t nbs = width(cbs[c].N);
+        const Seen a = add(sa, ia, elems_a, q.x_off, q.ldx, q.K, cbs[c].M, 128, akc);
+        const Seen b = add(sb, ib, elems_b, q.y_off, q.ldy, q.K, cbs[c].N, nbs, bkc);
+        if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
+        pk[p] = I8Pack{a.base, b.base, static_cast<int32_t>(a.scale), static_cast<int32_t>(b.scale),
+                       static_cast<int32_t>((q.K + 63) / 64), static_cast<int32_t>(nbs)};
+      }
+    const double t_i8 = cycles / sms / 1.85e9 + (16.0 * (elems_a + elems_b) + total) / 4.5e12 + 30e-6;
+    const double t_f64 = flops / 27e12 + 5e-6;
+    if (ctx->gemm_i8 < 0 && t_i8 > 0.95 * t_f64) return false;
+    // k-segments when the tiles are fewer than four per SM, as in prepare_tc
+    const int64_t target = 4LL * sms;
+    int64_t seg = 0;
+    if (static_cast<int64_t>(geo.size()) < target && total_kt > 0)
+      seg = std::max<int64_t>(12, (total_kt + target - 1) / target);
+    struct W { TcTile t; double work; int64_t group; };
+    std::vector<W> items;
+    std::vector<TcSplit> splits;
+    int32_t nparts = 0;
+    for (const Geo& t : geo) {
+      const int64_t kt = kt_of[t.c];
+      const int64_t nseg = (seg > 0 && 4 * kt > 5 * seg) ? (kt + seg - 1) / seg : 1;
+      int p = cbs[t.c].pair_begin, k0 = 0;
+      if (nseg > 1) splits.push_back(TcSplit{t.c, t.a0, t.b0, t.nb, nparts, static_cast<int32_t>(nseg), 0, 0});
+      for (int64_t q = 0; q < nseg; ++q) {
+        const int64_t kb = kt * q / nseg, ke = kt * (q + 1) / nseg;
+        items.push_back(W{TcTile{t.c, t.a0, t.b0, t.nb, p, k0, static_cast<int32_t>(ke - kb),
+                                 nseg > 1 ? nparts + static_cast<int32_t>(q) : -1},
+                          (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q});
+        for (int64_t i = kb; i < ke; ++i) {
+          k0 += 64;
+          if (k0 >= pairs[p].K) {
+            ++p;
+            k0 = 0;
+          }
+        }
+      }
+      if (nseg > 1) nparts += static_cast<int32_t>(nseg);
+    }
+    // heaviest groups (C block, k-segment) first, a group's items together:
+    // they read the same images
+    std::unordered_map<int64_t, double> gwork;
+    for (const W& w : items) gwork[w.group] += w.work;
+    std::stable_sort(items.begin(), items.end(), [&](const W& a, const W& b) {
+      const double wa = gwork[a.group], wb = gwork[b.group];
+      return wa != wb ? wa > wb : a.group < b.group;
+    });
+    // each item to the CTA with the least work so far: in this order neighbours
+    // still run at about the same time, and the sums even out (the stride walk
+    // left R*T3 at chi = 2048 with 51% to 77% busy tensor cores)
+    const int32_t nctas = static_cast<int32_t>(std::max<size_t>(1, std::min<size_t>(sms, items.size())));
+    std::vector<std::vector<TcTile>> mine(nctas);
+    std::priority_queue<std::pair<double, int32_t>, std::vector<std::pair<double, int32_t>>, std::greater<>> least;
+    for (int32_t i = 0; i < nctas; ++i) least.emplace(0.0, i);
+    for (auto& w : items) {
+      auto [load, i] = least.top();
+      least.pop();
+      mine[i].push_back(w.t);
+      least.emplace(load + w.work, i);
+    }
+    std::vector<TcTile> tiles;
+    std::vector<int32_t> first(nctas + 1, 0);
+    tiles.reserve(items.size() + zero.size());
+    for (int32_t i = 0; i < nctas; ++i) {
+      tiles.insert(tiles.end(), mine[i].begin(), mine[i].end());
+      first[i + 1] = static_cast<int32_t>(tiles.size());
+    }
+    for (auto& t : zero) tiles.push_back(TcTile{t.c, t.a0, t.b0, t.nb, 0, 0, 0, -1});
+    require(tiles.size() < (1ULL << 31), SB_ERR_INVALID_ARG, "too many GEMM tiles in one launch");
+    int64_t f = 0;
+    for (auto& c : cbs) {  // 64x64 tiles of the DMMA launch behind the flag
+      c.tile_begin = static_cast<int32_t>(f);
+      c.mtiles = static_cast<int32_t>((c.M + 63) / 64);
+      f += static_cast<int64_t>(c.mtiles) * ((c.N + 63) / 64);
+    }
+    g.kind = GemmLaunch::I8;
+    g.dfirst = upload(ctx, first);
+    g.nctas = nctas;
+    g.dc = upload(ctx, cbs);
+    g.dp = upload(ctx, pairs);
+    g.dt = upload(ctx, tiles);
+    g.dsplit = upload(ctx, splits);
+    g.dpk = upload(ctx, pk);
+    g.dimg_a = upload(ctx, ia);
+    g.dimg_b = upload(ctx, ib);
+    g.nimg_a = static_cast<int64_t>(ia.size());
+    g.nimg_b = static_cast<int64_t>(ib.size());
+    g.pack_a_bytes = total;
+    g.pack_a_elems = elems_a;
+    g.pack_b_elems = elems_b;
+    g.nscale = nscale;
+    g.nf = f;
+    g.nsplits = static_cast<int32_t>(splits.size());
+    g.nparts = nparts;
+    g.ncb = static_cast<int32_t>(cbs.size());
+    g.n = static_cast<int64_t>(tiles.size());
+    g.nz_begin = static_cast<int32_t>(items.size());
+    g.flops = flops;
+    g.bytes = bytes;
+    std::snprintf(g.desc, sizeof(g.desc), "i8 128xN items:%lld split:%d est %.0f us (f64 %.0f)",
+                  static_cast<long long>(g.n), g.nsplits, t_i8 * 1e6, t_f64 * 1e6);
+    return true;
   }
 
   // Thin launches (K <= 16): output blocks whose pairs read the same block of

@@ -415,6 +415,43 @@ cudaError_t dispatch_t(bool xT, bool yT, const double* X, const double* Y, doubl
   return launch_t<BM, BN, WM, WN, true, true, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, part, s);
 }
 
+// 64x64 tiles walked by a resident grid, for a launch that another kernel has
+// usually made unnecessary: without the flag every CTA returns after one load,
+// where a grid of one CTA per tile would pay for launching them all.
+template <bool XT, bool YT>
+__global__ void __launch_bounds__(128, 4)
+    k_gemm_f64_fallback(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ C,
+                        const GemmCBlock* __restrict__ cblocks, int32_t ncb, const GemmPair* __restrict__ pairs,
+                        int32_t ntiles, const int* __restrict__ flag) {
+  extern __shared__ double smem[];
+  if (flag && *flag == 0) return;
+  for (int bid = static_cast<int>(blockIdx.x); bid < ntiles; bid += static_cast<int>(gridDim.x)) {
+    const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
+    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, bid - cb.tile_begin, 0, 1, nullptr, smem);
+    __syncthreads();  // the operand buffers are refilled by the next tile
+  }
+}
+
+template <bool XT, bool YT>
+cudaError_t launch_fallback_t(const double* X, const double* Y, double* C, const GemmCBlock* cb, int32_t ncb,
+                              const GemmPair* pr, int64_t ntiles, const int* flag, cudaStream_t s) {
+  constexpr int smem = TileLayout<64, 64, XT, YT>::bytes();
+  auto kern = k_gemm_f64_fallback<XT, YT>;
+  static std::atomic<unsigned long long> configured{0};  // one bit per device ordinal (host threads may race)
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const unsigned long long bit = 1ull << (dev & 63);
+  if (!(configured & bit)) {
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    configured.fetch_or(bit);
+  }
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>(ntiles, 148LL * 3));
+  kern<<<g, 128, smem, s>>>(X, Y, C, cb, ncb, pr, static_cast<int32_t>(ntiles), flag);
+  return cudaGetLastError();
+}
+
 // ── thin GEMM (K <= 16, one of M/N <= 16, the other long) ─────────────────
 // One CTA covers kThinBig elements of the long dimension of one C block; the
 // long operand tile (kThinBig x 16) and the small one (16 x 16) of each pair
@@ -919,6 +956,17 @@ cudaError_t launch_gemm_f64_edges(const double* X, const double* Y, double* C, c
   if (!xT && yT) return launch_edges_t<false, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
   if (xT && !yT) return launch_edges_t<true, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
   return launch_edges_t<true, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
+}
+
+cudaError_t launch_gemm_f64_fallback(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,
+                                     int32_t ncb, const GemmPair* d_pairs, int64_t ntiles, bool xT, bool yT,
+                                     const int* d_flag, cudaStream_t s) {
+  if (ntiles <= 0) return cudaSuccess;
+  if (ntiles > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (!xT && !yT) return launch_fallback_t<false, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, d_flag, s);
+  if (!xT && yT) return launch_fallback_t<false, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, d_flag, s);
+  if (xT && !yT) return launch_fallback_t<true, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, d_flag, s);
+  return launch_fallback_t<true, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, d_flag, s);
 }
 
 cudaError_t launch_gemm_f64(const double* X, const double* Y, double* C,

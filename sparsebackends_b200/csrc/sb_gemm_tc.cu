@@ -51,6 +51,7 @@
 #include <cstdio>
 
 #include "sb_kernels.hpp"
+#include "sb_tcgen05.cuh"
 
 namespace sb {
 namespace {
@@ -65,69 +66,6 @@ constexpr int kTcEpiBytes = kTcDrainWarps * 32 * 32 * 4;  // per-warp 32 x 32 FP
 constexpr int kTcSmemBytes = kTcStages * kTcStageBytes + kTcEpiBytes + 1024 /*alignment*/ + 256 /*barriers*/;
 constexpr int kTcTmemCols = 512;                   // two accumulators of up to 256 columns
 constexpr int kTcReduceSlices = kTcMaxN / 32;      // 32-column slices of a split tile
-constexpr unsigned long long kWaitNs = 2000000000ull;  // bound of every mbarrier wait
-
-__device__ __forceinline__ uint32_t smem_u32(const void* p) {
-  return static_cast<uint32_t>(__cvta_generic_to_shared(p));
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
-}
-
-__device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
-  asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
-}
-
-__device__ __forceinline__ bool mbar_try(uint32_t bar, uint32_t parity) {
-  uint32_t ok;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok)
-      : "r"(bar), "r"(parity)
-      : "memory");
-  return ok != 0;
-}
-
-// Bounded wait for the completion of phase `parity` of the mbarrier.  Returns
-// false (and records the failure) when the bound runs out.
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, int* status) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  while (true) {
-    if (mbar_try(bar, parity)) return true;
-    if (global_ns() - t0 > kWaitNs) {
-      atomicExch(status, 1);
-      return false;
-    }
-  }
-}
-
-// The same wait for roles that sit out most of a k-tile (the drain warps):
-// between polls the warp sleeps, leaving its issue slots to the producers.
-__device__ __forceinline__ bool mbar_wait_idle(uint32_t bar, uint32_t parity, int* status) {
-  if (mbar_try(bar, parity)) return true;
-  const unsigned long long t0 = global_ns();
-  while (true) {
-    __nanosleep(256);
-    if (mbar_try(bar, parity)) return true;
-    if (global_ns() - t0 > kWaitNs) {
-      atomicExch(status, 1);
-      return false;
-    }
-  }
-}
-
-__device__ __forceinline__ void mbar_arrive(uint32_t bar) {
-  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory");
-}
-
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
 // Shared-memory matrix descriptor of a K-major SWIZZLE_128B operand image:
 // start address >> 4, leading-byte offset 16 (unused by swizzled K-major
@@ -151,10 +89,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t d_tmem, uint64_t a, uint64_t b
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate ? 1u : 0u));
-}
-
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
 }
 
 __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
@@ -191,9 +125,6 @@ __device__ __forceinline__ void tmem_st32(uint32_t taddr, const float (&v)[32]) 
   tmem_st16(taddr + 16, *reinterpret_cast<const float(*)[16]>(&v[16]));
 }
 
-__device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_wait_st() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
-
 // x = hi + lo with both parts exactly representable in TF32 (low 13 mantissa
 // bits zero).
 __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) {
@@ -208,25 +139,6 @@ __device__ __forceinline__ void split_tf32(float x, uint32_t& hi, uint32_t& lo) 
 // SWIZZLE_128B image.
 __device__ __forceinline__ uint32_t img_off(int r, int c) {
   return static_cast<uint32_t>((r >> 3) * 1024 + (r & 7) * 128 + ((c ^ (r & 7)) << 4));
-}
-
-// 16-byte global store (packed images).
-__device__ __forceinline__ void st_global_v4(void* p, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.global.v4.b32 [%0], {%1, %2, %3, %4};" ::"l"(p), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
-}
-
-__device__ __forceinline__ void mbar_expect_tx(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
-}
-
-// Bulk asynchronous copy global -> this CTA's shared memory, completing
-// `bytes` of transaction count on the mbarrier (16-byte aligned addresses,
-// size a multiple of 16).
-__device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile(
-      "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst),
-      "l"(src), "r"(bytes), "r"(bar)
-      : "memory");
 }
 
 // One packed k-tile image: rows [0, rows) x k [0, kv) of the operand tile at

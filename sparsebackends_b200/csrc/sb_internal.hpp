@@ -93,6 +93,10 @@ struct Ctx {
   // SPARSEB_GEMM_EDGES=0 keeps 64x64-tile launches in one tile shape (tuning);
   // -1 = auto: column / row edges of <= 32 go to 64x32 / 32x64 tiles.
   int gemm_edges = -1;
+  // SPARSEB_GEMM_I8=0 keeps FP64 launches on DMMA, =1 takes the integer
+  // tensor-core path for every launch it can serve (tests); -1 = by the
+  // estimated times (prepare_i8).
+  int gemm_i8 = -1;
   // SPARSEB_AUTOTUNE=1: the first FP64 tiled block GEMM of a block-shape
   // histogram times the candidate tile shapes on its own operands and keeps the
   // fastest; later launches with the same histogram take it without timing

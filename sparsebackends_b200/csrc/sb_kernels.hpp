@@ -147,6 +147,49 @@ struct TcImage {
 cudaError_t launch_tc_pack(const void* src, bool src_f64, const TcImage* d_imgs, int64_t nimg, void* dst, int passes,
                            cudaStream_t s);
 
+// ── the same grouped GEMM in FP64 through 8-bit integer products ───────────
+// (sb_gemm_i8.cu: tcgen05 kind::i8).  X is the 128-row side, Y the other.
+// Scratch holds the packed digit planes, one scale word per operand row
+// (zeroed before the packs) and a flag (zeroed too): the kernels set it when
+// an operand row's magnitude is outside 2^+-400 (or not finite), or when a
+// bounded wait ran out; C is then what launch_gemm_f64_fallback, which must
+// follow on the stream, computes.
+//
+// One 128-row (X) or rows_img-row (Y) x 64 k-tile image: element (r, k) at src
+// + r*ld + k when kc, else src + r + k*ld; rows < 128 and kv <= 64 valid, zeros
+// elsewhere; seven planes of rows_img * 64 bytes at byte dst; row r's scale at
+// index scale + r.
+struct I8Image {
+  int64_t src, ld, dst;
+  int32_t scale, rows, rows_img, kv, kc, pad;
+};
+cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, uint32_t* d_rowhi, void* dst,
+                           int* d_flag, cudaStream_t s);
+// Per pair: byte offsets of the images of its X block (row tiles of 128, nkt
+// k-tiles each) and Y block (column tiles of nbs), and the scale indices of
+// their first row and column.
+struct I8Pack {
+  int64_t a_base, b_base;
+  int32_t a_sc, b_sc, nkt, nbs;
+};
+constexpr int kI8MaxN = 128;
+constexpr int64_t kI8PartElems = 128 * kI8MaxN;  // doubles of one partial tile
+// k-tiles per INT32 accumulation chunk: 24 * 64 = 1536 terms keep the four
+// diagonals that are combined (5 * 1536 * 2^14 * 2^24 + ...) below 2^51.
+constexpr int kI8Chunk = 24;
+// Items, splits and pair-less items as for launch_gemm_tc, with 64-deep
+// k-tiles, tiles of 128 x nb (nb <= 128) and column-major 128 x 128 partials.
+// CTA i of the nctas (one per SM at most) runs items [first[i], first[i + 1]).
+cudaError_t launch_gemm_i8(const void* pack, double* C, const GemmCBlock* d_cblocks, const I8Pack* d_packs,
+                           const uint32_t* d_rowhi, const TcTile* d_tiles, const int32_t* d_first, int32_t nctas,
+                           int32_t ntiles, int32_t nz_begin, double* d_partial, const TcSplit* d_splits,
+                           int32_t nsplits, int* d_flag, cudaStream_t s);
+// The DMMA kernel over the same C blocks (64x64 tiles numbered by tile_begin),
+// on a grid that returns at once unless *d_flag is set (NULL: it always runs).
+cudaError_t launch_gemm_f64_fallback(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,
+                                     int32_t ncblocks, const GemmPair* d_pairs, int64_t ntiles, bool xT, bool yT,
+                                     const int* d_flag, cudaStream_t s);
+
 // ── outer-product accumulation (K = 1 pairs) on CUDA cores ─────────────────
 //
 // For every C block c: C_c[i + j*M] = sum_p a_p[i] * b_p[j] in pair order, with
