@@ -435,19 +435,16 @@ struct GemmLaunch {
       ctx->note_launch();
       return;
     }
-    DevBuf part;
-    const int64_t tile = kind == EDGES ? 64 * 64 : static_cast<int64_t>(bm) * bn;
-    if (splitk > 1) part = DevBuf(ctx, static_cast<size_t>(splitk) * n * tile * sizeof(double));
     {
       ProfScope ps(ctx, PROF_GEMM, flops, bytes);
       if (kind == EDGES)
         SB_CK(launch_gemm_f64_edges(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), n, xT, yT, ctx->stream,
-                                    splitk, part.d()));
+                                    splitk));
       else
         SB_CK(launch_gemm_f64(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), n, xT, yT, shape, ctx->stream,
-                              splitk, part.d()));
+                              splitk));
     }
-    ctx->note_launch(splitk > 1 ? 2 : 1);
+    ctx->note_launch();
   }
 };
 
@@ -585,14 +582,15 @@ struct GemmPlan {
     }
     // Split-K when the tiles fill few waves of the 148 SMs and each tile has a
     // long K loop (choose_splitk).
-    int64_t kt_avg = 0;
+    int64_t kt_avg = 0, kt_max = 0;
     for (auto& c : cbs) {
       int64_t kt = 0;
       for (int p = c.pair_begin; p < c.pair_end; ++p) kt += (pairs[p].K + 15) / 16;
       kt_avg += kt * ((c.M + bm - 1) / bm) * ((c.N + bn - 1) / bn);
+      kt_max = std::max(kt_max, kt);
     }
     kt_avg = ntiles ? kt_avg / ntiles : 0;
-    const int splitk = choose_splitk(ctx, ntiles, kt_avg);
+    const int splitk = choose_splitk(ctx, ntiles, kt_avg, kt_max);
     std::snprintf(g.desc, sizeof(g.desc), "tiled %dx%d sk%d", bm, bn, splitk);
     g.kind = GemmLaunch::TILED;
     g.dc = upload(ctx, cbs);
@@ -1013,15 +1011,22 @@ struct GemmPlan {
     return any;
   }
 
-  // Split-K factor for ntiles tiles averaging kt_avg k-tiles: split while the
-  // tiles fill less than ~6 waves of 148 SMs x 4 CTAs and every segment keeps
-  // >= 32 k-tiles (6 waves against 3: R*T3 at chi=2048 2.02 -> 1.98 ms ragged,
-  // 8.04 -> 7.89 ms zero-padded; the shorter CTAs balance the uneven K loops).
-  static int choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg) {
+  // Split-K factor for ntiles tiles with kt_avg k-tiles on average and kt_max
+  // at most (a power of two up to the cluster size): split while the tiles
+  // fill less than ~6 waves of 148 SMs x 4 CTAs and every segment keeps >= 32
+  // k-tiles (the shorter CTAs balance the uneven K loops), and, when there are
+  // fewer CTAs than 4 per SM, as long as the longest K loop keeps >= 4 k-tiles
+  // per segment: one SM takes 0.5 us per 64x64x16 k-tile, so a few long
+  // tiles leave the chip idle (R*T3 of H_eff, us, before and after: chi = 256,
+  // 42 tiles of up to 130 k-tiles, 121 and 27; chi = 400 122 and 50; chi = 512
+  // 99 and 71; chi = 700 165 and 131; chi = 1024 332 and 318).
+  static int choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg, int64_t kt_max) {
     int splitk = 1;
     const int64_t wave = 148 * 4;
-    while (splitk < 16 && ntiles * splitk < 6 * wave && kt_avg / (2 * splitk) >= 32) splitk *= 2;
-    if (ctx->gemm_splitk > 0) splitk = ctx->gemm_splitk;
+    while (splitk < kMaxSplitK && ((ntiles * splitk < 6 * wave && kt_avg / (2 * splitk) >= 32) ||
+                                   (ntiles * splitk < wave && kt_max / (2 * splitk) >= 4)))
+      splitk *= 2;
+    if (ctx->gemm_splitk > 0) splitk = std::min(ctx->gemm_splitk, kMaxSplitK);
     return splitk;
   }
   // 64x64 tiles with the edges cut off: a column remainder N mod 64 of <= 32
@@ -1055,10 +1060,11 @@ struct GemmPlan {
     std::vector<GemmCBlock> sc;
     std::vector<GemmPair> ep(pairs);
     sc.reserve(cbs.size() * 3);
-    int64_t ntiles = 0, kts = 0;
+    int64_t ntiles = 0, kts = 0, kt_max = 0;
     for (auto& c : cbs) {
       int64_t kt = 0;
       for (int p = c.pair_begin; p < c.pair_end; ++p) kt += (pairs[p].K + 15) / 16;
+      kt_max = std::max(kt_max, kt);
       const int32_t mm = static_cast<int32_t>(body64(c.M)), nm = static_cast<int32_t>(body64(c.N));
       auto sub = [&](int32_t shape, int32_t r0, int32_t c0, int32_t rows, int32_t cols) {
         const int bm = edge_rows(shape), bn = edge_cols(shape);
@@ -1102,7 +1108,7 @@ struct GemmPlan {
         ntiles += static_cast<int64_t>(b.mtiles) * ((b.N + bn - 1) / bn);
       }
     }
-    const int splitk = choose_splitk(ctx, ntiles, kt_avg);
+    const int splitk = choose_splitk(ctx, ntiles, kt_avg, kt_max);
     long long nshape[5] = {0, 0, 0, 0, 0};
     for (auto& b : sc) nshape[b.tshape] += static_cast<long long>(b.mtiles) * ((b.N + edge_cols(b.tshape) - 1) /
                                                                                 edge_cols(b.tshape));

@@ -118,8 +118,8 @@ def test_error_not_above_dmma(kind):
 
 @pytest.mark.parametrize("what", ["inf", "nan", "huge", "tiny", "subnormal", "zero_rows", "zero_block"])
 def test_values_outside_the_scale_range(what):
-    """Rows that the integer path does not take are recomputed with DMMA: the
-    same values, infinities and NaN as without it."""
+    """Rows that the integer path does not take are recomputed with DMMA in one
+    K loop per tile: the values, infinities and NaN of the DMMA path unsplit."""
     import sparsebackends_b200 as sb
     rng = np.random.Generator(np.random.PCG64(3))
     A, B = _blocks(rng, 140, 150, (90, 70))
@@ -140,7 +140,7 @@ def test_values_outside_the_scale_range(what):
     else:
         A[1, 1][:] = 0.0
     x = _run(sb, _ctx(sb, SPARSEB_GEMM_I8=1), A, B, "AB")[1, 1]
-    y = _run(sb, _ctx(sb, SPARSEB_GEMM_I8=0), A, B, "AB")[1, 1]
+    y = _run(sb, _ctx(sb, SPARSEB_GEMM_I8=0, SPARSEB_GEMM_SPLITK=1), A, B, "AB")[1, 1]
     assert np.array_equal(np.isnan(x), np.isnan(y)) and np.array_equal(np.isinf(x), np.isinf(y))
     f = np.isfinite(y)
     if what in ("zero_rows", "zero_block"):
