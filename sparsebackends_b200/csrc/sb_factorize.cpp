@@ -72,7 +72,7 @@ QrResult blocksparse_left_qr(Ctx* ctx, const Tensor& A) {
     ln.push_back(ds);
   }
   copy_blocks(ctx, A.data.d(), M.d(), so, dof, ln);
-  DevBuf tau(ctx, std::max<int64_t>(k, 1) * sizeof(double));
+  DevBuf tau(ctx, std::max<int64_t>(householder_scalars(m, n), 1) * sizeof(double));
   DevBuf Q(ctx, std::max<int64_t>(m * k, 1) * sizeof(double));
   if (k > 0) {
     ProfScope ps(ctx, PROF_OTHER, 4.0 * m * n * k, 8.0 * m * n);

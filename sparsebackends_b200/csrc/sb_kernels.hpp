@@ -355,7 +355,10 @@ cudaError_t launch_add_blocks(const double* A, const double* B, double* C, const
 // ── block factorisations (QR, SVD truncation) ──────────────────────────────
 // In-place Householder QR of the column-major m x n matrix M (LAPACK dlarfg
 // convention): R in the upper triangle, reflector j below the diagonal of
-// column j with scale tau[j]; *launches counts the kernels issued.
+// column j; tau (householder_scalars(m, n) doubles) receives the reflectors'
+// scales: the panels' T matrices up to 1024 rows, else one per reflector;
+// *launches counts the kernels issued.
+int64_t householder_scalars(int64_t m, int64_t n);
 cudaError_t launch_householder_qr(double* M, int64_t m, int64_t n, double* tau, cudaStream_t s, int64_t* launches);
 // Thin Q (m x k, column-major) from the reflectors in M.
 cudaError_t launch_householder_form_q(const double* M, int64_t m, int64_t k, const double* tau, double* Q,
