@@ -18,7 +18,6 @@
 // values and the keep counts) is host work, as in the reference; every value
 // is computed on the device.
 #include <algorithm>
-#include <map>
 #include <numeric>
 
 #include "sb_internal.hpp"
@@ -38,6 +37,33 @@ void gather(Ctx* ctx, const double* src, double* dst, const double* scale, const
   ctx->note_launch();
 }
 
+// The sorted distinct values of one prefix axis and the position of each:
+// by a table over the axis when it is not much longer than the key list
+// (two passes over the keys), else by sorting.
+struct Ranks {
+  std::vector<int64_t> vals, table;  // table[x] = position of value x, when used
+  Ranks(const Tensor& A, int axis) {
+    const int64_t d = A.dims[axis];
+    if (d <= 4 * A.nkeys + 1024) {
+      table.assign(d + 1, -1);
+      for (int64_t i = 0; i < A.nkeys; ++i) table[A.key(i)[axis]] = 0;
+      for (int64_t x = 1; x <= d; ++x)
+        if (table[x] == 0) {
+          table[x] = static_cast<int64_t>(vals.size());
+          vals.push_back(x);
+        }
+      return;
+    }
+    for (int64_t i = 0; i < A.nkeys; ++i) vals.push_back(A.key(i)[axis]);
+    std::sort(vals.begin(), vals.end());
+    vals.erase(std::unique(vals.begin(), vals.end()), vals.end());
+  }
+  int64_t of(int64_t x) const {
+    if (!table.empty()) return table[x];
+    return static_cast<int64_t>(std::lower_bound(vals.begin(), vals.end(), x) - vals.begin());
+  }
+};
+
 }  // namespace
 
 QrResult blocksparse_left_qr(Ctx* ctx, const Tensor& A) {
@@ -47,29 +73,19 @@ QrResult blocksparse_left_qr(Ctx* ctx, const Tensor& A) {
   require_uniform(A, "blocksparse_left_qr");
   require(A.nkeys > 0, SB_ERR_INVALID_ARG, "blocksparse_left_qr: tensor has no blocks");
   QrResult out;
-  for (int64_t i = 0; i < A.nkeys; ++i) {
-    out.l_vals.push_back(A.key(i)[0]);
-    out.r_vals.push_back(A.key(i)[1]);
-  }
-  for (auto* v : {&out.l_vals, &out.r_vals}) {
-    std::sort(v->begin(), v->end());
-    v->erase(std::unique(v->begin(), v->end()), v->end());
-  }
+  Ranks lr(A, 0), rr(A, 1);
+  out.l_vals = lr.vals;
+  out.r_vals = rr.vals;
   const int64_t ds = A.dims[2];
   const int64_t nl = static_cast<int64_t>(out.l_vals.size()), nr = static_cast<int64_t>(out.r_vals.size());
   const int64_t m = nl * ds, n = nr, k = std::min(m, n);
-  auto pos = [](const std::vector<int64_t>& v, int64_t x) {
-    return static_cast<int64_t>(std::lower_bound(v.begin(), v.end(), x) - v.begin());
-  };
   // dense M (column-major m x n)
   DevBuf M(ctx, std::max<int64_t>(m * n, 1) * sizeof(double));
   if (m * n) SB_CK(cudaMemsetAsync(M.raw(), 0, m * n * sizeof(double), ctx->stream));
-  std::vector<int64_t> so, dof, ln;
+  std::vector<int64_t> so(A.nkeys), dof(A.nkeys), ln(A.nkeys, ds);
   for (int64_t i = 0; i < A.nkeys; ++i) {
-    const int64_t li = pos(out.l_vals, A.key(i)[0]), ri = pos(out.r_vals, A.key(i)[1]);
-    so.push_back(A.block_off(i));
-    dof.push_back(li * ds + ri * m);
-    ln.push_back(ds);
+    so[i] = A.block_off(i);
+    dof[i] = lr.of(A.key(i)[0]) * ds + rr.of(A.key(i)[1]) * m;
   }
   copy_blocks(ctx, A.data.d(), M.d(), so, dof, ln);
   DevBuf tau(ctx, std::max<int64_t>(householder_scalars(m, n), 1) * sizeof(double));
@@ -113,29 +129,29 @@ SvdResult blocksparse_svd(Ctx* ctx, const Tensor& A, bool ortho_right, int64_t m
   require(maxdim >= 1 && mindim >= 0 && cutoff >= 0.0, SB_ERR_INVALID_ARG,
           "blocksparse_svd: maxdim >= 1, mindim >= 0, cutoff >= 0 required");
   // group keys by L (keys are sorted by L + nL*R, so R ascends within a group)
-  std::map<int64_t, std::vector<std::pair<int64_t, int64_t>>> groups;  // L -> [(R, key index)]
-  for (int64_t i = 0; i < A.nkeys; ++i) groups[A.key(i)[0]].push_back({A.key(i)[1], i});
+  const Ranks lr(A, 0);
   struct G {
     int64_t L, n, a_off, u_off, s_off, k;
-    std::vector<int64_t> rlist;
   };
-  std::vector<G> gs;
+  std::vector<G> gs(lr.vals.size());
+  std::vector<int64_t> gof(A.nkeys), col(A.nkeys);  // group of key i, its place in the group
+  for (int64_t i = 0; i < A.nkeys; ++i) {
+    gof[i] = lr.of(A.key(i)[0]);
+    col[i] = gs[gof[i]].n++;
+  }
   int64_t aw = 0, uw = 0, sw = 0;
-  std::vector<Gather2D> items;
-  for (auto& [L, lst] : groups) {
-    std::sort(lst.begin(), lst.end());
-    G g{L, static_cast<int64_t>(lst.size()) * d2, aw, uw, sw, 0, {}};
-    g.k = std::min(d1, g.n);
-    for (size_t j = 0; j < lst.size(); ++j) {
-      g.rlist.push_back(lst[j].first);
-      // M_L[s1, j*d2 + s2] (row-major, row length n) = A block [s1 + s2*d1]
-      items.push_back(Gather2D{A.block_off(lst[j].second), g.a_off + static_cast<int64_t>(j) * d2, d1, d2, 1, d1,
-                               g.n, 1, -1});
-    }
-    aw += d1 * g.n;
+  for (size_t gi = 0; gi < gs.size(); ++gi) {
+    const int64_t n = gs[gi].n * d2;
+    gs[gi] = G{lr.vals[gi], n, aw, uw, sw, std::min(d1, n)};
+    aw += d1 * n;
     uw += d1 * d1;
     sw += d1;
-    gs.push_back(std::move(g));
+  }
+  // M_L[s1, j*d2 + s2] (row-major, row length n) = A block [s1 + s2*d1]
+  std::vector<Gather2D> items(A.nkeys);
+  for (int64_t i = 0; i < A.nkeys; ++i) {
+    const G& g = gs[gof[i]];
+    items[i] = Gather2D{A.block_off(i), g.a_off + col[i] * d2, d1, d2, 1, d1, g.n, 1, -1};
   }
   SvdResult out;
   DevBuf W(ctx, std::max<int64_t>(aw, 1) * sizeof(double)), Vt(ctx, std::max<int64_t>(aw, 1) * sizeof(double));
@@ -183,40 +199,38 @@ SvdResult blocksparse_svd(Ctx* ctx, const Tensor& A, bool ortho_right, int64_t m
   // U: dims (nL, nb, d1), prefix (L, b), dense s1; keys in nb order are sorted
   out.U = make_tensor(ctx, BS, {nL, nb, d1}, 1);
   out.SV = make_tensor(ctx, BS, {nb, nR, d2}, 1);
-  std::vector<Gather2D> ui;
-  struct SvItem {
-    int64_t lin, b, r;
-    Gather2D g;
-  };
-  std::vector<SvItem> vi;
+  std::vector<Gather2D> ui, vg(A.nkeys);
+  out.U->keys.reserve(2 * nb);
   for (size_t gi = 0; gi < gs.size(); ++gi) {
     const G& g = gs[gi];
     for (int64_t c = 0; c < kk[gi]; ++c) {
-      const int64_t b = off[gi] + c;
-      out.svs[b] = sv[g.s_off + c];
+      out.svs[off[gi] + c] = sv[g.s_off + c];
       out.U->keys.push_back(g.L);
-      out.U->keys.push_back(b + 1);
-      ui.push_back(Gather2D{g.u_off + c * d1, b * d1, d1, 1, 1, 0, 1, 0, ortho_right ? g.s_off + c : -1});
-      for (size_t j = 0; j < g.rlist.size(); ++j)
-        vi.push_back(SvItem{b + nb * (g.rlist[j] - 1), b + 1, g.rlist[j],
-                            Gather2D{g.a_off + c * g.n + static_cast<int64_t>(j) * d2, 0, d2, 1, 1, 0, 1, 0,
-                                     ortho_right ? -1 : g.s_off + c}});
+      out.U->keys.push_back(off[gi] + c + 1);
     }
+    if (kk[gi] > 0)  // column c of U_L, times its singular value when ortho = right
+      ui.push_back(Gather2D{g.u_off, off[gi] * d1, d1, kk[gi], 1, d1, 1, d1, ortho_right ? g.s_off : -1});
   }
   out.U->nkeys = nb;
   out.U->data = DevBuf(ctx, std::max<int64_t>(nb * d1, 1) * sizeof(double));
   gather(ctx, U.d(), out.U->data.d(), S.d(), ui);
-  std::stable_sort(vi.begin(), vi.end(), [](const SvItem& a, const SvItem& b) { return a.lin < b.lin; });
-  std::vector<Gather2D> vg;
-  for (size_t i = 0; i < vi.size(); ++i) {
-    out.SV->keys.push_back(vi[i].b);
-    out.SV->keys.push_back(vi[i].r);
-    Gather2D g = vi[i].g;
-    g.dst_off = static_cast<int64_t>(i) * d2;
-    vg.push_back(g);
+  // SV's keys (b, R) column-major: A's keys run through R, and for one R
+  // through L, whose bond values b ascend with it
+  int64_t nsv = 0;
+  for (int64_t i = 0; i < A.nkeys; ++i) nsv += kk[gof[i]];
+  out.SV->keys.resize(2 * nsv);
+  int64_t at = 0;
+  for (int64_t i = 0; i < A.nkeys; ++i) {
+    const int64_t gi = gof[i], R = A.key(i)[1];
+    const G& g = gs[gi];
+    vg[i] = Gather2D{g.a_off + col[i] * d2, at * d2, d2, kk[gi], 1, g.n, 1, d2, ortho_right ? -1 : g.s_off};
+    for (int64_t c = 0; c < kk[gi]; ++c, ++at) {
+      out.SV->keys[2 * at] = off[gi] + c + 1;
+      out.SV->keys[2 * at + 1] = R;
+    }
   }
-  out.SV->nkeys = static_cast<int64_t>(vi.size());
-  out.SV->data = DevBuf(ctx, std::max<int64_t>(out.SV->nkeys * d2, 1) * sizeof(double));
+  out.SV->nkeys = nsv;
+  out.SV->data = DevBuf(ctx, std::max<int64_t>(nsv * d2, 1) * sizeof(double));
   gather(ctx, Vt.d(), out.SV->data.d(), S.d(), vg);
   return out;
 }

@@ -307,7 +307,7 @@ __global__ void k_gather_2d(const double* __restrict__ src, double* __restrict__
        e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
     const int64_t r = e % it.rows, c = e / it.rows;
     const double v = src[it.src_off + r * it.src_rs + c * it.src_cs];
-    dst[it.dst_off + r * it.dst_rs + c * it.dst_cs] = it.s_idx >= 0 ? __dmul_rn(v, scale[it.s_idx]) : v;
+    dst[it.dst_off + r * it.dst_rs + c * it.dst_cs] = it.s_idx >= 0 ? __dmul_rn(v, scale[it.s_idx + c]) : v;
   }
 }
 

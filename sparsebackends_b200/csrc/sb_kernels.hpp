@@ -366,7 +366,7 @@ cudaError_t launch_householder_form_q(const double* M, int64_t m, int64_t k, con
 // R (k x n, column-major) = upper triangle of the first k rows of M.
 cudaError_t launch_upper(const double* M, int64_t m, int64_t k, int64_t n, double* R, cudaStream_t s);
 // Strided 2-D copies: dst[dst_off + r*dst_rs + c*dst_cs] = src[src_off + r*src_rs + c*src_cs]
-// (times scale[s_idx] when s_idx >= 0) for r < rows, c < cols.
+// (times scale[s_idx + c] when s_idx >= 0) for r < rows, c < cols.
 struct Gather2D {
   int64_t src_off, dst_off, rows, cols, src_rs, src_cs, dst_rs, dst_cs, s_idx;
 };
