@@ -299,12 +299,17 @@ __global__ void k_upper(const double* __restrict__ M, int64_t m, int64_t k, int6
   }
 }
 
+// WARP: a warp per item (items of a few elements, the blocks of a sparse
+// prefix); otherwise a row of CTAs per item.
+template <bool WARP>
 __global__ void k_gather_2d(const double* __restrict__ src, double* __restrict__ dst, const double* __restrict__ scale,
-                            const Gather2D* __restrict__ items) {
-  const Gather2D it = items[blockIdx.y];
-  const int64_t n = it.rows * it.cols;
-  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
-       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+                            const Gather2D* __restrict__ items, int64_t nitems) {
+  const int64_t i = WARP ? static_cast<int64_t>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5) : blockIdx.y;
+  if (i >= nitems) return;
+  const Gather2D it = items[i];
+  const int64_t n = it.rows * it.cols, step = WARP ? 32 : static_cast<int64_t>(gridDim.x) * blockDim.x;
+  for (int64_t e = WARP ? threadIdx.x & 31 : static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+       e += step) {
     const int64_t r = e % it.rows, c = e / it.rows;
     const double v = src[it.src_off + r * it.src_rs + c * it.src_cs];
     dst[it.dst_off + r * it.dst_rs + c * it.dst_cs] = it.s_idx >= 0 ? __dmul_rn(v, scale[it.s_idx + c]) : v;
@@ -491,10 +496,14 @@ cudaError_t launch_upper(const double* M, int64_t m, int64_t k, int64_t n, doubl
 cudaError_t launch_gather_2d(const double* src, double* dst, const double* scale, const Gather2D* d_items, int64_t n,
                              int64_t max_elems, cudaStream_t s) {
   if (n <= 0 || max_elems <= 0) return cudaSuccess;
+  if (max_elems <= 64 && (n + 7) / 8 <= 0x7fffffffLL) {
+    k_gather_2d<true><<<static_cast<unsigned>((n + 7) / 8), 256, 0, s>>>(src, dst, scale, d_items, n);
+    return cudaGetLastError();
+  }
   for (int64_t b = 0; b < n; b += 65535) {
     const unsigned gy = static_cast<unsigned>(std::min<int64_t>(65535, n - b));
     const unsigned gx = static_cast<unsigned>(std::min<int64_t>((max_elems + 255) / 256, 64));
-    k_gather_2d<<<dim3(gx, gy), 256, 0, s>>>(src, dst, scale, d_items + b);
+    k_gather_2d<false><<<dim3(gx, gy), 256, 0, s>>>(src, dst, scale, d_items + b, gy);
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
   }
