@@ -64,7 +64,9 @@ void destroy_ctx_now(sb_ctx* ctx) {
   ctx->impl.plan_cache.reset();  // its device buffers are released on the stream
   ctx->impl.crop_scratch.reset();
   ctx->impl.tc_status.reset();
+  ctx->impl.dot_scratch.reset();
   cudaStreamSynchronize(ctx->impl.stream);
+  if (ctx->impl.host_scalar) cudaFreeHost(ctx->impl.host_scalar);
   ctx->impl.release_staging();
   if (ctx->impl.own_stream) cudaStreamDestroy(ctx->impl.stream);
   delete ctx;

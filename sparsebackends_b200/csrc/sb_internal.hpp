@@ -119,6 +119,12 @@ struct Ctx {
   // bounded waits ran out); allocated when a tensor-core precision is chosen
   // and read by sb_ctx_synchronize.
   DevBuf tc_status;
+  // Dot products: arrival counter (first 16 bytes, zero between calls) and
+  // partial sums on the device, and the mapped host word the kernel writes the
+  // result to.  Every call ends with a synchronisation, so one of each serves
+  // the context's calls in turn.
+  DevBuf dot_scratch;
+  double* host_scalar = nullptr;
   bool tc_launched = false;  // a tensor-core GEMM ran since the status was last read
   // Plan cache of the BS x BS contract_shared! path (sb_contract.cpp): the
   // output block structure and the prepared block GEMM of recent

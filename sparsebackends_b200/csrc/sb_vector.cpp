@@ -46,24 +46,38 @@ double run_dot(Ctx* ctx, const double* X, const double* Y, const double* S, std:
     }
     merged.push_back(s);
   }
+  if (merged.empty()) return 0.0;
   std::vector<DotChunk> chunks;
-  int64_t total = 0;
+  int64_t total = 0, nchunks = 0;
+  const bool contiguous = merged.size() == 1 && merged[0].s_idx < 0;
   for (const Seg& s : merged) {
     total += s.len;
+    nchunks += (s.len + kDotChunk - 1) / kDotChunk;
+    if (contiguous) continue;
     for (int64_t b = 0; b < s.len; b += kDotChunk)
       chunks.push_back(DotChunk{s.x_off + b, s.y_off + b, s.s_idx,
                                 static_cast<int32_t>(std::min<int64_t>(kDotChunk, s.len - b)), 0});
   }
   DevBuf dc = upload(ctx, chunks);
-  DevBuf part(ctx, std::max<size_t>(chunks.size(), 1) * sizeof(double));
-  DevBuf out(ctx, sizeof(double));
+  // partials and the arrival counter: kept by the context, grown to the
+  // longest vector (8 bytes per 1024 elements)
+  const size_t need = static_cast<size_t>(nchunks) * sizeof(double) + 16;
+  if (ctx->dot_scratch.bytes() < need) {
+    ctx->dot_scratch = DevBuf(ctx, std::max<size_t>(need, 2 * ctx->dot_scratch.bytes()));
+    SB_CK(cudaMemsetAsync(ctx->dot_scratch.raw(), 0, 16, ctx->stream));
+  }
+  if (!ctx->host_scalar) SB_CK(cudaHostAlloc(&ctx->host_scalar, sizeof(double), cudaHostAllocMapped));
+  double* out = nullptr;
+  SB_CK(cudaHostGetDevicePointer(&out, ctx->host_scalar, 0));
   {
     ProfScope ps(ctx, PROF_VECTOR, 2.0 * total, 16.0 * total);
-    SB_CK(launch_dot_chunks(X, Y, S, dc.as<DotChunk>(), static_cast<int64_t>(chunks.size()), part.d(), out.d(),
-                            ctx->stream));
+    SB_CK(launch_dot(X + (contiguous ? merged[0].x_off : 0), Y + (contiguous ? merged[0].y_off : 0), S,
+                     contiguous ? nullptr : dc.as<DotChunk>(), nchunks, total, ctx->dot_scratch.d() + 2,
+                     ctx->dot_scratch.as<unsigned>(), out, ctx->stream));
   }
-  ctx->note_launch(chunks.empty() ? 0 : 2);
-  return download<double>(ctx, out.raw(), 1)[0];
+  ctx->note_launch();
+  ctx->sync();
+  return *static_cast<volatile double*>(ctx->host_scalar);
 }
 
 void map_values(Ctx* ctx, double* R, const double* A, int64_t n, int op, double alpha, double beta) {

@@ -104,3 +104,21 @@ def test_crop_of_short_rows_stays_off_the_tiles():
     got = R.blocks_by_key()
     for i in range(3):
         assert np.array_equal(got[(i + 1,)], b[i][tuple(slice(0, e) for e in ext)].reshape(-1, order="F"))
+
+
+@pytest.mark.parametrize("n", [1, 1023, 1024, 1025, 262144, 1048577, 3000000])
+def test_dot_and_norm_lengths(n):
+    """One launch per scalar: chunk edges, more partials than the final sum's
+    1024 strands, and repeated calls on growing and shrinking vectors.  The
+    pairwise-like sum is compared with numpy's extended precision at n eps."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(n))
+    x, y = rng.standard_normal(n), rng.standard_normal(n)
+    X, Y = sb.DenseTensor(x), sb.DenseTensor(y)
+    want = float(np.sum(x.astype(np.longdouble) * y))
+    tol = n * np.finfo(float).eps * float(np.sum(np.abs(x * y))) / np.sqrt(n)
+    first = sb.dot(X, Y)
+    assert abs(first - want) <= tol
+    assert abs(sb.norm(X) - float(np.sqrt(np.sum(x.astype(np.longdouble) ** 2)))) <= n * np.finfo(float).eps * np.sqrt(n)
+    assert sb.dot(sb.DenseTensor(x[:1]), sb.DenseTensor(y[:1])) == x[0] * y[0]
+    assert sb.dot(X, Y) == first
