@@ -315,21 +315,32 @@ __global__ void k_perm_blocks(const double* __restrict__ src, double* __restrict
   for (int64_t b = blockIdx.y; b < n; b += gridDim.y) {
     const BlockPerm& it = items[b];
     if (it.len < (int64_t{1} << 31)) {
-      // a block below 2^31 elements: 32-bit index arithmetic (every extent and
-      // coordinate of it fits), several times cheaper than 64-bit division
-      for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e0 < it.len;
-           e0 += (int64_t)gridDim.x * blockDim.x) {
-        uint32_t e = static_cast<uint32_t>(e0);
-        int64_t so = 0;
-        bool in = true;
-        for (int r = 0; r < it.rank; ++r) {
-          const uint32_t d = static_cast<uint32_t>(it.out_dims[r]);
-          const uint32_t c = e % d;
-          e /= d;
-          in = in && c < it.in_lim[r];
-          so += static_cast<int64_t>(c) * it.in_strides[r];
+      // a block below 2^31 elements: 32-bit indices, divided by multiplication;
+      // four elements per thread, their loads in flight together.  With the
+      // divisions in hardware the index work bound it: cropping the zero-padded
+      // T3 of a chi = 1023 H_eff (rows of 12 to 14) took 181 us, now 107.
+      constexpr int kPer = 4;
+      const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
+      for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e0 < it.len; e0 += kPer * stride) {
+        double v[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) {
+          const int64_t e1 = e0 + q * stride;
+          uint32_t e = static_cast<uint32_t>(e1 < it.len ? e1 : 0);
+          int64_t so = it.src_off;
+          bool in = e1 < it.len;
+          for (int r = 0; r < it.rank; ++r) {
+            const uint32_t d = static_cast<uint32_t>(it.out_dims[r]);
+            const uint32_t next = (__umulhi(e, it.div_mul[r]) + e) >> it.div_shift[r], c = e - next * d;
+            e = next;
+            in = in && c < it.in_lim[r];
+            so += static_cast<int64_t>(c) * it.in_strides[r];
+          }
+          v[q] = in ? src[so] : 0.0;
         }
-        dst[it.dst_off + e0] = in ? src[it.src_off + so] : 0.0;
+#pragma unroll
+        for (int q = 0; q < kPer; ++q)
+          if (e0 + q * stride < it.len) dst[it.dst_off + e0 + q * stride] = v[q];
       }
       continue;
     }
@@ -363,19 +374,37 @@ __global__ void k_perm_block_rows(const double* __restrict__ src, double* __rest
     const int64_t lim0 = it.in_lim[0] < d0 ? it.in_lim[0] : d0;
     for (int64_t row = static_cast<int64_t>(blockIdx.x) * wpc + (threadIdx.x >> 5); row < rows;
          row += static_cast<int64_t>(gridDim.x) * wpc) {
-      int64_t rr = row, so = 0;
+      int64_t so = 0;
       bool in = true;
-      for (int r = 1; r < it.rank; ++r) {
-        const int64_t c = rr % it.out_dims[r];
-        rr /= it.out_dims[r];
-        in = in && c < it.in_lim[r];
-        so += c * it.in_strides[r];
+      if (it.len < (int64_t{1} << 31)) {
+        uint32_t rr = static_cast<uint32_t>(row);
+        for (int r = 1; r < it.rank; ++r) {
+          const uint32_t d = static_cast<uint32_t>(it.out_dims[r]);
+          const uint32_t next = (__umulhi(rr, it.div_mul[r]) + rr) >> it.div_shift[r], c = rr - next * d;
+          rr = next;
+          in = in && c < it.in_lim[r];
+          so += static_cast<int64_t>(c) * it.in_strides[r];
+        }
+      } else {
+        int64_t rr = row;
+        for (int r = 1; r < it.rank; ++r) {
+          const int64_t c = rr % it.out_dims[r];
+          rr /= it.out_dims[r];
+          in = in && c < it.in_lim[r];
+          so += c * it.in_strides[r];
+        }
       }
       const double* sp = src + it.src_off + so;
       double* o = dst + it.dst_off + row * d0;
       const int64_t lim = in ? lim0 : 0;
-#pragma unroll 4
-      for (int64_t e = lane; e < d0; e += 32) o[e] = e < lim ? sp[e] : 0.0;
+      for (int64_t e = lane; e < d0; e += 256) {  // eight loads in flight per lane
+        double v[8];
+#pragma unroll
+        for (int q = 0; q < 8; ++q) v[q] = e + 32 * q < lim ? sp[e + 32 * q] : 0.0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q)
+          if (e + 32 * q < d0) o[e + 32 * q] = v[q];
+      }
     }
   }
 }
@@ -911,18 +940,89 @@ __global__ void k_block_extents(const double* __restrict__ src, const int64_t* _
   }
 }
 
+// The scan of tails of up to four axes (blocks below 2^31 elements): a warp
+// task is a contiguous run of `budget` elements, read coalesced with eight
+// loads in flight per lane whatever the axes' extents; the coordinates of a
+// nonzero element come from multiplications.  HBM-bound on large operands:
+// L and T3 of a chi = 1023 zero-padded H_eff (147 and 580 MB) took 85 and 172
+// us by columns, with a 64-bit division per axis and column; 40 and 116 (5.0
+// TB/s).
+template <int N2>
+__global__ void __launch_bounds__(kThreads)
+    k_block_extents_linear(const double* __restrict__ src, const int64_t* __restrict__ off,
+                           const int64_t* __restrict__ dims, const int64_t* __restrict__ task_begin, int64_t nblocks,
+                           int64_t budget, int* __restrict__ ext) {
+  const int lane = threadIdx.x & 31;
+  const int64_t ntasks = task_begin[nblocks];
+  const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
+  for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < ntasks; w += warps) {
+    int64_t lo = 0, hi = nblocks - 1;  // the last block with task_begin <= w, 32 candidates per round
+    while (lo < hi) {
+      const int64_t step = (hi - lo + 32) / 32, idx = lo + (lane + 1) * step;
+      const int k = __popc(__ballot_sync(0xffffffffu, idx <= hi && task_begin[idx] <= w));
+      lo += k * step;
+      hi = hi < lo + step - 1 ? hi : lo + step - 1;
+    }
+    uint32_t d[N2], mul[N2], sh[N2], m[N2];
+    uint32_t len = 1;
+#pragma unroll
+    for (int r = 0; r < N2; ++r) {
+      d[r] = static_cast<uint32_t>(dims[lo * N2 + r]);
+      len *= d[r];
+      m[r] = 0;
+      sh[r] = d[r] <= 1 ? 0 : 32 - __clz(d[r] - 1);  // as set_divisors
+      mul[r] = static_cast<uint32_t>((((uint64_t{1} << sh[r]) - d[r]) << 32) / d[r] + 1);
+    }
+    const uint32_t e0 = static_cast<uint32_t>((w - task_begin[lo]) * budget);
+    const uint32_t e1 = len - e0 < budget ? len : e0 + static_cast<uint32_t>(budget);
+    const double* p = src + off[lo];
+    for (uint32_t e = e0 + lane; e < e1; e += 256) {
+      double v[8];
+#pragma unroll
+      for (int q = 0; q < 8; ++q) v[q] = e + 32 * q < e1 ? p[e + 32 * q] : 0.0;
+#pragma unroll
+      for (int q = 0; q < 8; ++q)
+        if (v[q] != 0.0) {
+          uint32_t x = e + 32 * q;
+#pragma unroll
+          for (int r = 0; r < N2; ++r) {
+            const uint32_t next = r + 1 < N2 ? (__umulhi(x, mul[r]) + x) >> sh[r] : 0;
+            const uint32_t c = x - next * (r + 1 < N2 ? d[r] : 0) + 1;
+            x = next;
+            m[r] = c > m[r] ? c : m[r];
+          }
+        }
+    }
+#pragma unroll
+    for (int r = 0; r < N2; ++r) m[r] = __reduce_max_sync(0xffffffffu, m[r]);
+    if (lane == 0 && m[0] > 0)
+#pragma unroll
+      for (int r = 0; r < N2; ++r) atomicMax(&ext[lo * N2 + r], static_cast<int>(m[r]));
+  }
+}
+
 int64_t block_extent_budget(int64_t elems) {
   const int64_t b = elems / (148LL * 48);
   return b < 512 ? 512 : b > 8192 ? 8192 : b;
 }
-int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget) { return ext_tasks(d0, cols, budget); }
+int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget, bool linear) {
+  return linear ? (d0 * cols + budget - 1) / budget : ext_tasks(d0, cols, budget);
+}
 
 cudaError_t launch_block_extents(const double* src, const int64_t* d_off, const int64_t* d_dims,
                                  const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2,
-                                 int64_t budget, int* d_ext, cudaStream_t s) {
+                                 int64_t budget, bool linear, int* d_ext, cudaStream_t s) {
   if (ntasks <= 0 || nblocks <= 0) return cudaSuccess;
-  if (n2 < 1 || n2 > kMaxRank) return cudaErrorInvalidValue;
+  if (n2 < 1 || n2 > kMaxRank || (linear && n2 > 4)) return cudaErrorInvalidValue;
   const int64_t ctas = std::min<int64_t>((ntasks + 7) / 8, 148LL * 8);
+  const unsigned g = static_cast<unsigned>(ctas);
+  if (linear) {
+    if (n2 == 1) k_block_extents_linear<1><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
+    else if (n2 == 2) k_block_extents_linear<2><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
+    else if (n2 == 3) k_block_extents_linear<3><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
+    else k_block_extents_linear<4><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
+    return cudaGetLastError();
+  }
   k_block_extents<<<static_cast<unsigned>(ctas), kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, n2,
                                                                     budget, d_ext);
   return cudaGetLastError();

@@ -256,7 +256,21 @@ struct BlockPerm {
   int64_t out_dims[kMaxRank];
   int64_t in_strides[kMaxRank];
   int64_t in_lim[kMaxRank];
+  // division by out_dims[r] (blocks below 2^31 elements) as a multiply and a
+  // shift: q = (mulhi(n, div_mul) + n) >> div_shift, exact for n < 2^31
+  // (Granlund and Montgomery 1994); set by set_divisors
+  uint32_t div_mul[kMaxRank], div_shift[kMaxRank];
 };
+inline void set_divisors(BlockPerm& b) {
+  for (int r = 0; r < b.rank; ++r) {
+    const uint64_t d = static_cast<uint64_t>(b.out_dims[r]);
+    uint32_t s = 0;
+    while (s < 32 && (uint64_t{1} << s) < d) ++s;
+    b.div_shift[r] = s;
+    b.div_mul[r] = d < 1 || d >= (uint64_t{1} << 31) ? 0
+                   : static_cast<uint32_t>((uint64_t{1} << 32) * ((uint64_t{1} << s) - d) / d + 1);
+  }
+}
 cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* d_items, int64_t n,
                                int64_t max_len, cudaStream_t s);
 // The same through shared-memory tiles, for items that neither pad nor crop.
@@ -283,16 +297,17 @@ cudaError_t launch_perm_block_rows(const double* src, double* dst, const BlockPe
 // ext[b*n2 + r] = smallest axis-r extent of block b (payload at d_off[b],
 // extents d_dims[b*n2 ..]) that keeps all its nonzero entries (>= 1; d_ext
 // holds 1s on entry).  The scan runs in warp tasks: block b has
-// block_extent_tasks(d0, cols, budget) of them (d0 = its first extent, cols =
+// block_extent_tasks(d0, cols, ...) of them (d0 = its first extent, cols =
 // the product of the others), starting at d_task_begin[b]; d_task_begin has
 // nblocks + 1 entries, the last = ntasks.  budget: elements per task, 512 to
 // 8192 by the number of elements scanned (block_extent_budget), the same
-// value for every call of one launch.
+// value for every call of one launch; linear (likewise): tails of at most four
+// axes and blocks below 2^31 elements, whose tasks are runs of elements.
 int64_t block_extent_budget(int64_t elems);
-int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget);
+int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget, bool linear);
 cudaError_t launch_block_extents(const double* src, const int64_t* d_off, const int64_t* d_dims,
                                  const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2,
-                                 int64_t budget, int* d_ext, cudaStream_t s);
+                                 int64_t budget, bool linear, int* d_ext, cudaStream_t s);
 // flags[i] = 1 if block i of src holds a nonzero outside its box in_lim
 // (used to check that cropping a padded block loses nothing).
 cudaError_t launch_outside_nonzero(const double* src, const BlockPerm* d_items, int64_t n, int64_t max_len,

@@ -242,13 +242,14 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
   }
   rows = rows && elems >= 16 * nrows;
   // otherwise tiles, when no item pads or crops; else the per-element gather,
-  // which is also the quicker one on a few thousand elements, where a tile's
-  // two dependent phases cost more than they save (11 000 elements: 6.6 to 8.0
-  // us against 7.7 to 8.8; 215 000: 11.5 to 11.9 against 8.8 to 10.3)
+  // which is also the quicker one on small operands, where a tile's two
+  // dependent phases cost more than they save (11 000 elements: 6.6 to 8.0 us
+  // against 7.7 to 8.8; 215 000: 11.5 to 11.9 against 8.8 to 10.3; 89 000: the
+  // whole call 19.9 us against 20.6)
   std::vector<PermTileItem> pt;
   int64_t tiles = 0;
   const uint32_t cap = perm_tile_cap(static_cast<int64_t>(bytes / 16));
-  if (!rows && bytes >= 16.0 * (1 << 15)) {
+  if (!rows && bytes >= 16.0 * (1 << 17)) {
     pt.resize(items.size());
     for (size_t i = 0; i < items.size(); ++i) {
       int64_t t = 0;
@@ -292,6 +293,7 @@ static BlockPerm make_block_perm(int64_t src_off, int64_t dst_off, const std::ve
     b.in_lim[r] = in_lim[r];
     b.len *= out_dims[r];
   }
+  set_divisors(b);
   return b;
 }
 
@@ -349,6 +351,8 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
     if (n == 0 || A.n2 == 0) continue;
     std::vector<int64_t> off(n), dims(n * A.n2), tb(n + 1, 0);
     const int64_t budget = block_extent_budget(A.payload_len());
+    bool linear = A.n2 <= 4;
+    for (int64_t i = 0; i < n; ++i) linear = linear && A.block_len(i) < (int64_t{1} << 31);
     for (int64_t i = 0; i < n; ++i) {
       off[i] = A.block_off(i);
       int64_t cols = 1;
@@ -356,14 +360,14 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
         dims[i * A.n2 + t] = A.block_dim(i, t);
         if (t > 0) cols *= dims[i * A.n2 + t];
       }
-      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols, budget);
+      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols, budget, linear);
     }
     keep.push_back(upload(ctx, off));
     keep.push_back(upload(ctx, dims));
     keep.push_back(upload(ctx, tb));
     const size_t m = keep.size();
     SB_CK(launch_block_extents(A.payload(), keep[m - 3].as<int64_t>(), keep[m - 2].as<int64_t>(),
-                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, budget,
+                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, budget, linear,
                                dext.as<int>() + base[k], ctx->stream));
     ctx->note_launch();
   }

@@ -49,7 +49,7 @@ def test_coo_times_blocks_bit_exact(length, first):
     assert all(np.array_equal(got[k], np.ravel(want[k], order="F")) for k in want)
 
 
-@pytest.mark.parametrize("tail", [(1, 1), (31, 70), (32, 5), (33, 600), (600, 33), (5000, 1), (9, 40, 21), (515, 515)])
+@pytest.mark.parametrize("tail", [(7,), (9000,), (3, 2, 5, 4, 6), (5, 7, 6, 11), (1, 1), (31, 70), (32, 5), (33, 600), (600, 33), (5000, 1), (9, 40, 21), (515, 515)])
 @pytest.mark.parametrize("nblocks", [1, 6])
 def test_zero_padding_scan_extents(tail, nblocks):
     """Extents found by the scan, for every form of its tasks (rows of one
@@ -73,7 +73,7 @@ def test_zero_padding_scan_extents(tail, nblocks):
 
 
 @pytest.mark.parametrize("tperm", [(2, 1, 3), (2, 3, 1), (3, 1, 2), (3, 2, 1), (1, 3, 2)])
-@pytest.mark.parametrize("top", [(1, 1, 1), (2, 3, 2), (64, 64, 1), (65, 130, 3), (33, 1, 200), (7, 150, 90)])
+@pytest.mark.parametrize("top", [(1, 1, 1), (2, 3, 2), (64, 64, 1), (64, 64, 9), (65, 130, 3), (33, 1, 200), (33, 1, 900), (7, 150, 90)])
 def test_ragged_permute_tiles(tperm, top):
     """Ragged tail permutes through tiles: partial tiles on either side, blocks
     with extents of one, a short contiguous axis; bit-exact against numpy."""
