@@ -274,7 +274,7 @@ void reset_output(Ctx* ctx, Tensor& C, int64_t nkeys, int64_t payload) {
 // launched again without planning or uploads (the plan cache of shared_bb).
 struct GemmLaunch {
   enum Kind { NONE, THIN, TILED, EDGES, TC, I8 } kind = NONE;
-  DevBuf dc, dp, dt, dsplit, dfirst;
+  DevBuf dc, dp, dt, dsplit, dfirst, dgroup, drow_off, drow_ld;
   int32_t ncb = 0;
   int64_t n = 0;  // strips (thin) or tiles
   bool xT = false, yT = false, small_rows = false, persistent = false;
@@ -337,8 +337,8 @@ struct GemmLaunch {
     }
     {
       ProfScope ps(ctx, PROF_GEMM, flops, bytes);
-      SB_CK(launch_gemm_i8(b, C, dc.as<GemmCBlock>(), dpk.as<I8Pack>(), rowhi, dt.as<TcTile>(),
-                           dfirst.as<int32_t>(), nctas, static_cast<int32_t>(n), nz_begin, reinterpret_cast<double*>(b + part_off),
+      SB_CK(launch_gemm_i8(b, C, dgroup.as<I8Group>(), drow_off.as<int64_t>(), drow_ld.as<int32_t>(),
+                           dpk.as<I8Pack>(), rowhi, dt.as<TcTile>(), dfirst.as<int32_t>(), nctas, static_cast<int32_t>(n), nz_begin, reinterpret_cast<double*>(b + part_off),
                            dsplit.as<TcSplit>(), nsplits, flag, ctx->stream));
       SB_CK(launch_gemm_f64_fallback(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), nf, xT, yT, flag,
                                      ctx->stream));
@@ -766,17 +766,19 @@ struct GemmPlan {
                   g.kc, g.fold ? " fold" : "");
   }
 
-  // FP64 launch on the integer tensor cores (launch_gemm_i8).  Tiles of 128 rows
-  // of X by nbs columns of Y (as few tiles of at most 128 columns as cover the
-  // block, of equal width rounded up to 16); each distinct operand block is
-  // packed once.  Returns false, leaving the launch to DMMA, unless the
+  // FP64 launch on the integer tensor cores (launch_gemm_i8).  C blocks that read
+  // the same Y blocks stack their rows (psi*L and R*T3 of H_eff: the four spin
+  // pairs of a link pair), so that rows pad to 128 once per stack: 14 to 20%
+  // fewer clocks at chi = 2048 and 700.  Tiles of 128 rows by nbs columns of Y
+  // (as few tiles of at most 128 columns as cover the block, of equal width
+  // rounded up to 16).  Returns false, leaving the launch to DMMA, unless the
   // estimated time is below DMMA's.  The estimate: clocks per k-tile and per
   // drained chunk over the SMs, the packing's bytes and 30 us of launches,
   // against 27 TFLOP/s.  Measured (H_eff steps, us, with
-  // packing): psi*L at chi = 2048 1030 against 1831 with DMMA, R*T3 1280
-  // against 1911; chi = 1024 psi*L 247 against 284, R*T3 346 against 333;
-  // chi = 700 139 against 109: small blocks pad to 128-row tiles and 64-deep
-  // k-tiles, and every chunk pays its drain.
+  // packing): psi*L at chi = 2048 946 against 1831 with DMMA, R*T3 1215 against
+  // 1911; chi = 1024 psi*L 225 against 284, R*T3 366 against 318; chi = 700
+  // 122 against 109: small blocks pad to 64-deep k-tiles and 16-wide columns,
+  // every chunk pays its drain.
   bool prepare_i8(Ctx* ctx, GemmLaunch& g, double flops, double bytes) {
     if (ctx->gemm_i8 == 0 || ctx->gemm_tile >= 0 || ctx->autotune) return false;
     if (ctx->gemm_i8 < 0 && flops < 2e8) return false;
@@ -787,67 +789,148 @@ struct GemmPlan {
     };
     int sms = 148;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    // groups of C blocks that read the same Y blocks (planning many thousands
+    // of tiny pairs would cost more than DMMA takes)
+    if (pairs.size() > 20000) return false;
+    struct Grp {
+      std::vector<int> members;
+      int64_t rows = 0, kt = 0, chunks = 0;
+      int32_t row0 = 0, p0 = 0, npairs = 0;
+    };
+    std::vector<Grp> grp;
+    {
+      std::map<std::vector<int64_t>, size_t> by;
+      std::vector<int64_t> key;
+      for (size_t c = 0; c < cbs.size(); ++c) {
+        key.assign(1, cbs[c].N);
+        for (int p = cbs[c].pair_begin; p < cbs[c].pair_end; ++p) {
+          key.push_back(pairs[p].y_off);
+          key.push_back(pairs[p].ldy);
+          key.push_back(pairs[p].K);
+        }
+        const auto it = by.emplace(key, grp.size());
+        if (it.second) grp.emplace_back();
+        Grp& gr = grp[it.first->second];
+        if (gr.rows + cbs[c].M >= (1LL << 31)) return false;
+        gr.members.push_back(static_cast<int>(c));
+        gr.rows += cbs[c].M;
+      }
+    }
     struct Geo { int32_t c, a0, b0, nb; };
     std::vector<Geo> geo, zero;
-    std::vector<int64_t> kt_of(cbs.size(), 0), chunks_of(cbs.size(), 0);
-    int64_t total_kt = 0, nf = 0;
+    int64_t total_kt = 0, nf = 0, nrows = 0, npairs = 0;
     double cycles = 0.0;
     // clocks of one k-tile (operand reads of its 68 MMAs and the copies, at 128
     // bytes per clock of shared memory) and of draining one chunk's accumulators
     auto mma_cycles = [](int64_t nb) { return 2880.0 + 22.5 * static_cast<double>(nb); };
     auto drain_cycles = [](int64_t nb) { return 2000.0 + 66.0 * static_cast<double>(nb); };
-    for (size_t c = 0; c < cbs.size(); ++c) {
-      for (int p = cbs[c].pair_begin; p < cbs[c].pair_end; ++p) {
-        const int64_t kt = (pairs[p].K + 63) / 64;
-        kt_of[c] += kt;
-        chunks_of[c] += (kt + kI8Chunk - 1) / kI8Chunk;
+    for (size_t i = 0; i < grp.size(); ++i) {
+      Grp& gr = grp[i];
+      const GemmCBlock& c0 = cbs[gr.members[0]];
+      for (int p = c0.pair_begin; p < c0.pair_end; ++p) {
+        const int64_t kt = (static_cast<int64_t>(pairs[p].K) + 63) / 64;
+        gr.kt += kt;
+        gr.chunks += (kt + kI8Chunk - 1) / kI8Chunk;
       }
-      const int64_t nbs = width(cbs[c].N);
-      for (int64_t a0 = 0; a0 < cbs[c].M; a0 += 128)
-        for (int64_t b0 = 0; b0 < cbs[c].N; b0 += nbs) {
-          const Geo t{static_cast<int32_t>(c), static_cast<int32_t>(a0), static_cast<int32_t>(b0),
-                      static_cast<int32_t>(std::min(nbs, up(cbs[c].N - b0, 16)))};
-          (kt_of[c] > 0 ? geo : zero).push_back(t);
-          total_kt += kt_of[c];
-          cycles += kt_of[c] * mma_cycles(t.nb) + drain_cycles(t.nb) * chunks_of[c];
+      gr.row0 = static_cast<int32_t>(nrows);
+      gr.p0 = static_cast<int32_t>(npairs);
+      gr.npairs = c0.pair_end - c0.pair_begin;
+      nrows += gr.rows;
+      npairs += gr.npairs;
+      if (nrows >= (1LL << 31)) return false;
+      const int64_t nbs = width(c0.N);
+      for (int64_t a0 = 0; a0 < gr.rows; a0 += 128)
+        for (int64_t b0 = 0; b0 < c0.N; b0 += nbs) {
+          const Geo t{static_cast<int32_t>(i), static_cast<int32_t>(a0), static_cast<int32_t>(b0),
+                      static_cast<int32_t>(std::min(nbs, up(c0.N - b0, 16)))};
+          (gr.kt > 0 ? geo : zero).push_back(t);
+          total_kt += gr.kt;
+          cycles += gr.kt * mma_cycles(t.nb) + drain_cycles(t.nb) * gr.chunks;
         }
-      nf += ((cbs[c].M + 63) / 64) * ((cbs[c].N + 63) / 64);
     }
+    for (auto& c : cbs) nf += ((static_cast<int64_t>(c.M) + 63) / 64) * ((static_cast<int64_t>(c.N) + 63) / 64);
     if (nf >= (1LL << 31) || geo.size() >= (1ULL << 30)) return false;
-    // packed images: every distinct operand block once
+    // packed images: every distinct Y block and every distinct stack of X blocks
+    // once (finding the scales and packing 40 or 160 MB at a time, so that the
+    // second read hits L2, was slower: 565 and 474 us against 402 for R*T3)
     const bool akc = g.xT, bkc = !g.yT;
-    std::vector<I8Pack> pk(pairs.size(), I8Pack{});
+    std::vector<I8Pack> pk(npairs, I8Pack{});
     std::vector<I8Image> ia, ib;
     struct Seen { int64_t base, scale; };
-    std::map<std::array<int64_t, 4>, Seen> sa, sb;  // (offset, ld, K, rows)
+    struct Seg { int64_t off, ld, rows; };  // a block of the stack
+    std::map<std::vector<int64_t>, Seen> sa, sb;
     int64_t total = 0, nscale = 0, elems_a = 0, elems_b = 0;
-    auto add = [&](std::map<std::array<int64_t, 4>, Seen>& seen, std::vector<I8Image>& out, int64_t& elems, int64_t off,
-                   int64_t ld, int64_t K, int64_t rows, int64_t tile, bool kc) -> Seen {
-      auto it = seen.find({off, ld, K, rows});
+    std::vector<int64_t> key;
+    auto add = [&](std::map<std::vector<int64_t>, Seen>& seen, std::vector<I8Image>& out, int64_t& elems,
+                   const std::vector<Seg>& segs, int64_t K, int64_t tile, bool kc) -> Seen {
+      key.assign(1, K);
+      for (const Seg& q : segs) {
+        key.push_back(q.off);
+        key.push_back(q.ld);
+        key.push_back(q.rows);
+      }
+      auto it = seen.find(key);
       if (it != seen.end()) return it->second;
       const Seen s{total, nscale};
-      for (int64_t r0 = 0; r0 < rows; r0 += tile)
+      int64_t rows = 0;
+      for (const Seg& q : segs) rows += q.rows;
+      size_t si = 0;
+      int64_t sr = 0;  // block and row in it that the tile starts with
+      for (int64_t r0 = 0; r0 < rows; r0 += tile) {
+        const int64_t r1 = std::min(rows, r0 + tile);
         for (int64_t k0 = 0; k0 < K; k0 += 64) {
-          out.push_back(I8Image{off + (kc ? r0 * ld + k0 : r0 + k0 * ld), ld, total,
-                                static_cast<int32_t>(nscale + r0), static_cast<int32_t>(std::min(tile, rows - r0)),
-                                static_cast<int32_t>(tile), static_cast<int32_t>(std::min<int64_t>(64, K - k0)),
-                                kc ? 1 : 0, 0});
+          size_t i = si;
+          int64_t at = sr;
+          for (int64_t r = r0; r < r1;) {
+            const Seg& q = segs[i];
+            const int64_t n = std::min(q.rows - at, r1 - r);
+            out.push_back(I8Image{q.off + (kc ? at * q.ld + k0 : at + k0 * q.ld), q.ld, total,
+                                  static_cast<int32_t>(nscale + r), static_cast<int32_t>(r - r0),
+                                  static_cast<int32_t>(n), static_cast<int32_t>(r + n == rows ? tile : r - r0 + n),
+                                  static_cast<int32_t>(tile), static_cast<int32_t>(std::min<int64_t>(64, K - k0)),
+                                  kc ? 1 : 0, 0});
+            r += n;
+            at += n;
+            if (at == q.rows) {
+              ++i;
+              at = 0;
+            }
+          }
           total += 7 * tile * 64;
+          if (k0 + 64 >= K) {
+            si = i;
+            sr = at;
+          }
         }
+      }
       elems += rows * K;
       nscale += rows;
-      seen.emplace(std::array<int64_t, 4>{off, ld, K, rows}, s);
+      seen.emplace(key, s);
       return s;
     };
-    for (size_t c = 0; c < cbs.size(); ++c)
-      for (int p = cbs[c].pair_begin; p < cbs[c].pair_end; ++p) {
-        const GemmPair& q = pairs[p];
-        const int64_t nbs = width(cbs[c].N);
-        const Seen a = add(sa, ia, elems_a, q.x_off, q.ldx, q.K, cbs[c].M, 128, akc);
-        const Seen b = add(sb, ib, elems_b, q.y_off, q.ldy, q.K, cbs[c].N, nbs, bkc);
+    std::vector<Seg> segs;
+    for (const Grp& gr : grp)
+      for (int j = 0; j < gr.npairs; ++j) {
+        segs.clear();
+        for (int m : gr.members) {
+          const GemmPair& q = pairs[cbs[m].pair_begin + j];
+          segs.push_back(Seg{q.x_off, q.ldx, cbs[m].M});
+        }
+        const int64_t K = pairs[cbs[gr.members[0]].pair_begin + j].K;
+        const Seen a = add(sa, ia, elems_a, segs, K, 128, akc);
+        pk[gr.p0 + j] = I8Pack{a.base, 0, static_cast<int32_t>(a.scale), 0, static_cast<int32_t>((K + 63) / 64),
+                               static_cast<int32_t>(width(cbs[gr.members[0]].N))};
         if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
-        pk[p] = I8Pack{a.base, b.base, static_cast<int32_t>(a.scale), static_cast<int32_t>(b.scale),
-                       static_cast<int32_t>((q.K + 63) / 64), static_cast<int32_t>(nbs)};
+      }
+    for (const Grp& gr : grp)
+      for (int j = 0; j < gr.npairs; ++j) {
+        const GemmCBlock& c0 = cbs[gr.members[0]];
+        const GemmPair& q = pairs[c0.pair_begin + j];
+        segs.assign(1, Seg{q.y_off, q.ldy, c0.N});
+        const Seen b = add(sb, ib, elems_b, segs, q.K, width(c0.N), bkc);
+        pk[gr.p0 + j].b_base = b.base;
+        pk[gr.p0 + j].b_sc = static_cast<int32_t>(b.scale);
+        if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
       }
     const double t_i8 = cycles / sms / 1.85e9 + (16.0 * (elems_a + elems_b) + total) / 4.5e12 + 30e-6;
     const double t_f64 = flops / 27e12 + 5e-6;
@@ -862,9 +945,9 @@ struct GemmPlan {
     std::vector<TcSplit> splits;
     int32_t nparts = 0;
     for (const Geo& t : geo) {
-      const int64_t kt = kt_of[t.c];
+      const int64_t kt = grp[t.c].kt;
       const int64_t nseg = (seg > 0 && 4 * kt > 5 * seg) ? (kt + seg - 1) / seg : 1;
-      int p = cbs[t.c].pair_begin, k0 = 0;
+      int p = grp[t.c].p0, k0 = 0, kp = 0;  // pair, offset in it, k-tile in it
       if (nseg > 1) splits.push_back(TcSplit{t.c, t.a0, t.b0, t.nb, nparts, static_cast<int32_t>(nseg), 0, 0});
       for (int64_t q = 0; q < nseg; ++q) {
         const int64_t kb = kt * q / nseg, ke = kt * (q + 1) / nseg;
@@ -873,9 +956,9 @@ struct GemmPlan {
                           (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q});
         for (int64_t i = kb; i < ke; ++i) {
           k0 += 64;
-          if (k0 >= pairs[p].K) {
+          if (++kp >= pk[p].nkt) {
             ++p;
-            k0 = 0;
+            k0 = kp = 0;
           }
         }
       }
@@ -920,6 +1003,22 @@ struct GemmPlan {
     g.kind = GemmLaunch::I8;
     g.dfirst = upload(ctx, first);
     g.nctas = nctas;
+    std::vector<I8Group> dg;
+    std::vector<int64_t> row_off;
+    std::vector<int32_t> row_ld;
+    row_off.reserve(nrows);
+    row_ld.reserve(nrows);
+    for (const Grp& gr : grp) {
+      dg.push_back(I8Group{static_cast<int32_t>(gr.rows), cbs[gr.members[0]].N, gr.row0, 0});
+      for (int m : gr.members)
+        for (int32_t r = 0; r < cbs[m].M; ++r) {
+          row_off.push_back(cbs[m].c_off + r);
+          row_ld.push_back(cbs[m].ldc);
+        }
+    }
+    g.dgroup = upload(ctx, dg);
+    g.drow_off = upload(ctx, row_off);
+    g.drow_ld = upload(ctx, row_ld);
     g.dc = upload(ctx, cbs);
     g.dp = upload(ctx, pairs);
     g.dt = upload(ctx, tiles);

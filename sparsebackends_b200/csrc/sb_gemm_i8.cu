@@ -26,6 +26,7 @@
 // k-tile, of the high words), k_i8_pack writes the seven digit planes of each
 // 64-deep k-tile of each 128-row tile of X and nbs-column tile of Y in the
 // layout the tensor core reads from shared memory (K-major, 64-byte swizzle),
+// (rows of several C blocks that read the same Y blocks are stacked, I8Group);
 // k_gemm_i8 is persistent, one CTA per SM: warp 0 moves images with bulk
 // copies, warp 1 issues the MMAs, warps 4-11 drain.  A tile is 128 x nb (nb <=
 // 128, a multiple of 16).  INT32 accumulators of 128 columns for four diagonals
@@ -41,7 +42,8 @@
 // the drain 0.38 M (reading the accumulators back runs at about 64 bytes per
 // clock and SM; overlapping it with the next pass, diagonal by diagonal, made
 // both slower: 1231 against 913 us), waits for copies 0.10 M.  Measured against
-// DMMA: psi*L 1831 -> 913 us + 119 packing, R*T3 1911 -> 870 + 414.
+// DMMA: psi*L 1831 -> 913 us + 119 packing, R*T3 1911 -> 870 + 414; with the
+// rows of C blocks that share Y stacked, 827 + 119 and 808 + 402.
 #include <algorithm>
 #include <atomic>
 
@@ -136,20 +138,21 @@ __global__ void __launch_bounds__(256)
   const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
   const int plane = im.rows_img * kI8BK;
   unsigned char* const d = dst + im.dst;
-  for (int g = warp; g < im.rows_img / 8; g += 8) {
-    const int rl = lane >> 2, c = lane & 3, r = 8 * g + rl;
+  for (int g = im.row0 / 8 + warp; 8 * g < im.row_end; g += 8) {
+    const int rl = lane >> 2, c = lane & 3;
+    const int ri = 8 * g + rl, r = ri - im.row0;  // row of the image, of the block
     const double* s = src + im.src;
     double x[16];
     if (im.kc) {
       double* st = stage[warp];
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
-        const int rr = 8 * g + q;
+        const int rr = 8 * g + q - im.row0;
         const double* p = s + static_cast<int64_t>(rr) * im.ld;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
           const int k = lane + 32 * h;
-          st[68 * q + 17 * (k >> 4) + (k & 15)] = rr < im.rows && k < im.kv ? p[k] : 0.0;
+          st[68 * q + 17 * (k >> 4) + (k & 15)] = rr >= 0 && rr < im.rows && k < im.kv ? p[k] : 0.0;
         }
       }
       __syncwarp();
@@ -160,9 +163,9 @@ __global__ void __launch_bounds__(256)
       const double* p = s + r + static_cast<int64_t>(16 * c) * im.ld;
 #pragma unroll
       for (int j = 0; j < 16; ++j)
-        x[j] = r < im.rows && 16 * c + j < im.kv ? p[static_cast<int64_t>(j) * im.ld] : 0.0;
+        x[j] = r >= 0 && r < im.rows && 16 * c + j < im.kv ? p[static_cast<int64_t>(j) * im.ld] : 0.0;
     }
-    const uint32_t hi = r < im.rows ? rowhi[im.scale + r] : 0u;
+    const uint32_t hi = r >= 0 && r < im.rows ? rowhi[im.scale + r] : 0u;
     double f = 0.0;
     if (hi != 0) {
       const int e = scale_exp(hi);
@@ -201,9 +204,10 @@ __global__ void __launch_bounds__(256)
       w[0][q] = __byte_perm(c1, d1, 0x5410);
     }
     // K-major 64-byte swizzle: row r at (r/8)*512 + (r%8)*64, chunk c at c ^ ((r/2) % 4)
-    unsigned char* o = d + (r >> 3) * 512 + (r & 7) * 64 + ((c ^ ((r >> 1) & 3)) << 4);
+    unsigned char* o = d + (ri >> 3) * 512 + (ri & 7) * 64 + ((c ^ ((ri >> 1) & 3)) << 4);
+    if (r >= 0 && ri < im.row_end)
 #pragma unroll
-    for (int q = 0; q < kI8Planes; ++q) st_global_v4(o + q * plane, w[q][0], w[q][1], w[q][2], w[q][3]);
+      for (int q = 0; q < kI8Planes; ++q) st_global_v4(o + q * plane, w[q][0], w[q][1], w[q][2], w[q][3]);
   }
 }
 
@@ -273,8 +277,8 @@ __device__ __forceinline__ void issue_ktile(uint32_t tmem, uint32_t sa, uint32_t
 }
 
 __global__ void __launch_bounds__(kI8Threads, 1)
-    k_gemm_i8(const unsigned char* __restrict__ pack, double* __restrict__ C, const GemmCBlock* __restrict__ cblocks,
-              const I8Pack* __restrict__ packs, const uint32_t* __restrict__ rowhi, const TcTile* __restrict__ tiles,
+    k_gemm_i8(const unsigned char* __restrict__ pack, double* __restrict__ C, const I8Group* __restrict__ groups,
+              const int64_t* __restrict__ row_off, const int32_t* __restrict__ row_ld, const I8Pack* __restrict__ packs, const uint32_t* __restrict__ rowhi, const TcTile* __restrict__ tiles,
               const int32_t* __restrict__ first, int32_t ntiles, int32_t nz_begin, double* __restrict__ partial,
               int* __restrict__ flag) {
   extern __shared__ unsigned char smem_raw[];
@@ -393,10 +397,12 @@ __global__ void __launch_bounds__(kI8Threads, 1)
     uint32_t np = 0;
     for (int t = t0; t < t1; ++t) {
       const TcTile tl = tiles[t];
-      const GemmCBlock cb = cblocks[tl.cb];
+      const I8Group gr = groups[tl.cb];
       const int row = tl.a0 + 32 * q + lane;
-      const int cols = min(tl.nb, cb.N - tl.b0) - 64 * h;  // valid columns of this warp (may be <= 0)
-      const bool row_ok = row < cb.M;
+      const int cols = min(tl.nb, gr.N - tl.b0) - 64 * h;  // valid columns of this warp (may be <= 0)
+      const bool row_ok = row < gr.rows;
+      const int64_t c_off = row_ok ? row_off[gr.row0 + row] : 0;
+      const int c_ld = row_ok ? row_ld[gr.row0 + row] : 0;
       double acc[64];
 #pragma unroll
       for (int j = 0; j < 64; ++j) acc[j] = 0.0;
@@ -448,21 +454,23 @@ __global__ void __launch_bounds__(kI8Threads, 1)
         for (int j = 0; j < 64; ++j)
           if (j < cols) pt[j * 128] = acc[j];
       } else {
-        double* c = C + cb.c_off + row + static_cast<int64_t>(tl.b0 + 64 * h) * cb.ldc;
+        double* c = C + c_off + static_cast<int64_t>(tl.b0 + 64 * h) * c_ld;
 #pragma unroll
         for (int j = 0; j < 64; ++j) {
           if (j < cols) *c = acc[j];
-          c += cb.ldc;
+          c += c_ld;
         }
       }
     }
     // C blocks without pairs (items [nz_begin, ntiles)): zeros
     for (int t = nz_begin + static_cast<int>(blockIdx.x); t < ntiles; t += grid) {
       const TcTile tl = tiles[t];
-      const GemmCBlock cb = cblocks[tl.cb];
-      const int rows = min(128, cb.M - tl.a0), cols = min(tl.nb, cb.N - tl.b0);
-      for (int e = tid - 128; e < rows * cols; e += 32 * kI8DrainWarps)
-        C[cb.c_off + tl.a0 + e % rows + static_cast<int64_t>(tl.b0 + e / rows) * cb.ldc] = 0.0;
+      const I8Group gr = groups[tl.cb];
+      const int rows = min(128, gr.rows - tl.a0), cols = min(tl.nb, gr.N - tl.b0);
+      for (int e = tid - 128; e < rows * cols; e += 32 * kI8DrainWarps) {
+        const int r = gr.row0 + tl.a0 + e % rows;
+        C[row_off[r] + static_cast<int64_t>(tl.b0 + e / rows) * row_ld[r]] = 0.0;
+      }
     }
   }
 
@@ -477,19 +485,23 @@ __global__ void __launch_bounds__(kI8Threads, 1)
 // Sum of the k-segment partial tiles of split tiles, in segment order.  One
 // CTA per (split tile, 32 columns), reads and writes coalesced along the rows.
 __global__ void __launch_bounds__(256) k_i8_reduce(const double* __restrict__ partial, double* __restrict__ C,
-                                                   const GemmCBlock* __restrict__ cblocks,
+                                                   const I8Group* __restrict__ groups,
+                                                   const int64_t* __restrict__ row_off,
+                                                   const int32_t* __restrict__ row_ld,
                                                    const TcSplit* __restrict__ splits) {
   const TcSplit sp = splits[blockIdx.x >> 2];
   const int c0 = 32 * static_cast<int>(blockIdx.x & 3);
-  const GemmCBlock cb = cblocks[sp.cb];
+  const I8Group gr = groups[sp.cb];
   const int r = static_cast<int>(threadIdx.x) & 127, row = sp.a0 + r;
-  const int cols = min(min(sp.nb, cb.N - sp.b0) - c0, 32);
-  if (row >= cb.M) return;
+  const int cols = min(min(sp.nb, gr.N - sp.b0) - c0, 32);
+  if (row >= gr.rows) return;
+  const int64_t c_off = row_off[gr.row0 + row];
+  const int c_ld = row_ld[gr.row0 + row];
   for (int c = static_cast<int>(threadIdx.x) >> 7; c < cols; c += 2) {
     const double* p = partial + static_cast<int64_t>(sp.part0) * kI8PartElems + r + (c0 + c) * 128;
     double acc = 0.0;
     for (int q = 0; q < sp.nparts; ++q) acc = __dadd_rn(acc, p[q * kI8PartElems]);
-    C[cb.c_off + row + static_cast<int64_t>(sp.b0 + c0 + c) * cb.ldc] = acc;
+    C[c_off + static_cast<int64_t>(sp.b0 + c0 + c) * c_ld] = acc;
   }
 }
 
@@ -507,10 +519,11 @@ cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nim
   return cudaGetLastError();
 }
 
-cudaError_t launch_gemm_i8(const void* pack, double* C, const GemmCBlock* d_cblocks, const I8Pack* d_packs,
-                           const uint32_t* d_rowhi, const TcTile* d_tiles, const int32_t* d_first, int32_t nctas,
-                           int32_t ntiles, int32_t nz_begin, double* d_partial, const TcSplit* d_splits,
-                           int32_t nsplits, int* d_flag, cudaStream_t s) {
+cudaError_t launch_gemm_i8(const void* pack, double* C, const I8Group* d_groups, const int64_t* d_row_off,
+                           const int32_t* d_row_ld, const I8Pack* d_packs, const uint32_t* d_rowhi,
+                           const TcTile* d_tiles, const int32_t* d_first, int32_t nctas, int32_t ntiles,
+                           int32_t nz_begin, double* d_partial, const TcSplit* d_splits, int32_t nsplits, int* d_flag,
+                           cudaStream_t s) {
   if (ntiles <= 0) return cudaSuccess;
   if (nctas < 1 || (nsplits > 0 && (!d_partial || !d_splits))) return cudaErrorInvalidValue;
   static std::atomic<unsigned long long> configured{0};  // one bit per device ordinal (host threads may race)
@@ -524,11 +537,12 @@ cudaError_t launch_gemm_i8(const void* pack, double* C, const GemmCBlock* d_cblo
     configured.fetch_or(bit);
   }
   const unsigned g = static_cast<unsigned>(nctas);
-  k_gemm_i8<<<g, kI8Threads, kI8SmemBytes, s>>>(static_cast<const unsigned char*>(pack), C, d_cblocks, d_packs,
-                                                d_rowhi, d_tiles, d_first, ntiles, nz_begin, d_partial, d_flag);
+  k_gemm_i8<<<g, kI8Threads, kI8SmemBytes, s>>>(static_cast<const unsigned char*>(pack), C, d_groups, d_row_off,
+                                                d_row_ld, d_packs, d_rowhi, d_tiles, d_first, ntiles, nz_begin, d_partial, d_flag);
   e = cudaGetLastError();
   if (e != cudaSuccess || nsplits <= 0) return e;
-  k_i8_reduce<<<static_cast<unsigned>(nsplits) * 4, 256, 0, s>>>(d_partial, C, d_cblocks, d_splits);
+  k_i8_reduce<<<static_cast<unsigned>(nsplits) * 4, 256, 0, s>>>(d_partial, C, d_groups, d_row_off,
+                                                                   d_row_ld, d_splits);
   return cudaGetLastError();
 }
 

@@ -156,13 +156,21 @@ cudaError_t launch_tc_pack(const void* src, bool src_f64, const TcImage* d_imgs,
 // bounded wait ran out; C is then what launch_gemm_f64_fallback, which must
 // follow on the stream, computes.
 //
-// One 128-row (X) or rows_img-row (Y) x 64 k-tile image: element (r, k) at src
-// + r*ld + k when kc, else src + r + k*ld; rows < 128 and kv <= 64 valid, zeros
-// elsewhere; seven planes of rows_img * 64 bytes at byte dst; row r's scale at
-// index scale + r.
+// C blocks whose pairs read the same Y blocks (the same offsets, leading
+// dimensions and K in the same order) form one group and share row tiles: their
+// rows are numbered through, and row_off / row_ld give each row's C offset and
+// column stride.
+struct I8Group {
+  int32_t rows, N, row0, pad;  // row0: the group's first entry in the row tables
+};
+// A piece of a 128-row (X) or rows_img-row (Y) x 64 k-tile image: image rows
+// [row0, row0 + rows) are an operand block's, element (r, k) at src + r*ld + k
+// when kc, else src + r + k*ld, kv <= 64 of them along k; rows up to row_end and
+// the rest of k are zeros.  Seven planes of rows_img * 64 bytes at byte dst; the
+// scale of row row0 at index scale.
 struct I8Image {
   int64_t src, ld, dst;
-  int32_t scale, rows, rows_img, kv, kc, pad;
+  int32_t scale, row0, rows, row_end, rows_img, kv, kc, pad;
 };
 cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, uint32_t* d_rowhi, void* dst,
                            int* d_flag, cudaStream_t s);
@@ -180,11 +188,13 @@ constexpr int64_t kI8PartElems = 128 * kI8MaxN;  // doubles of one partial tile
 constexpr int kI8Chunk = 24;
 // Items, splits and pair-less items as for launch_gemm_tc, with 64-deep
 // k-tiles, tiles of 128 x nb (nb <= 128) and column-major 128 x 128 partials.
-// CTA i of the nctas (one per SM at most) runs items [first[i], first[i + 1]).
-cudaError_t launch_gemm_i8(const void* pack, double* C, const GemmCBlock* d_cblocks, const I8Pack* d_packs,
-                           const uint32_t* d_rowhi, const TcTile* d_tiles, const int32_t* d_first, int32_t nctas,
-                           int32_t ntiles, int32_t nz_begin, double* d_partial, const TcSplit* d_splits,
-                           int32_t nsplits, int* d_flag, cudaStream_t s);
+// A tile's cb is its group's index.  CTA i of the nctas (one per SM at most)
+// runs items [first[i], first[i + 1]).
+cudaError_t launch_gemm_i8(const void* pack, double* C, const I8Group* d_groups, const int64_t* d_row_off,
+                           const int32_t* d_row_ld, const I8Pack* d_packs, const uint32_t* d_rowhi,
+                           const TcTile* d_tiles, const int32_t* d_first, int32_t nctas, int32_t ntiles,
+                           int32_t nz_begin, double* d_partial, const TcSplit* d_splits, int32_t nsplits, int* d_flag,
+                           cudaStream_t s);
 // The DMMA kernel over the same C blocks (64x64 tiles numbered by tile_begin),
 // on a grid that returns at once unless *d_flag is set (NULL: it always runs).
 cudaError_t launch_gemm_f64_fallback(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,

@@ -167,3 +167,26 @@ def test_split_tiles_and_many_blocks():
         want = (a.astype(np.longdouble) @ b.astype(np.longdouble)).astype(float)
         scale = np.outer(np.sqrt((a ** 2).sum(1)), np.sqrt((b ** 2).sum(0)))
         assert np.max(np.abs(c - want) / scale) <= 8 * 2.0 ** -55, (i, j)
+
+
+@pytest.mark.parametrize("ms", [(1, 1, 1), (127, 2, 130), (64, 64, 128), (5, 251, 17)])
+@pytest.mark.parametrize("order", ["AB", "BA"])
+def test_rows_stacked_over_output_blocks(ms, order):
+    """Output blocks that read the same Y blocks share row tiles: stacks whose
+    joints fall anywhere in a tile, beside a block with another list of pairs
+    and an extent of its own, either operand order."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(sum(ms)))
+    ks = (70, 130)
+    A = {(i + 1, q + 1): rng.standard_normal((m, k)) for i, m in enumerate(ms) for q, k in enumerate(ks)}
+    A[4, 2] = rng.standard_normal((77, 130))
+    B = {(q + 1, j): rng.standard_normal((k, n)) for j, n in ((1, 90), (2, 150)) for q, k in enumerate(ks)}
+    got = _run(sb, _ctx(sb, SPARSEB_GEMM_I8=1, SPARSEB_POISON_OUTPUT=1), A, B, order)
+    assert set(got) == {(i, j) for i in (1, 2, 3, 4) for j in (1, 2)}
+    for (i, j), c in got.items():
+        qs = [q for q in (1, 2) if (i, q) in A]
+        a = np.concatenate([A[i, q] for q in qs], 1)
+        b = np.concatenate([B[q, j] for q in qs], 0)
+        want = (a.astype(np.longdouble) @ b.astype(np.longdouble)).astype(float)
+        scale = np.outer(np.sqrt((a ** 2).sum(1)), np.sqrt((b ** 2).sum(0)))
+        assert np.max(np.abs(c - want) / scale) <= 8 * 2.0 ** -55, (i, j)
