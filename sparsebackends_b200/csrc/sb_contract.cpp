@@ -1240,7 +1240,9 @@ struct OuterPlan {
   }
   void launch(Ctx* ctx, const double* A, const double* B, double* C, bool kahan) {
     if (cbs.empty()) return;
-    DevBuf dc = upload(ctx, cbs), dp = upload(ctx, pairs);
+    size_t po = 0;
+    DevBuf dc = upload2(ctx, cbs, pairs, &po);
+    const auto* dp = reinterpret_cast<const OuterPair*>(dc.as<unsigned char>() + po);
     double flops = 0.0, bytes = 0.0;
     for (auto& c : cbs) {
       const double np = c.pair_end - c.pair_begin;
@@ -1249,7 +1251,7 @@ struct OuterPlan {
     }
     {
       ProfScope ps(ctx, PROF_OUTER, flops, bytes);
-      SB_CK(launch_outer_acc(A, B, C, dc.as<OuterCBlock>(), static_cast<int64_t>(cbs.size()), dp.as<OuterPair>(),
+      SB_CK(launch_outer_acc(A, B, C, dc.as<OuterCBlock>(), static_cast<int64_t>(cbs.size()), dp,
                              max_elems, kahan, ctx->stream));
     }
     ctx->note_launch();
@@ -1270,7 +1272,9 @@ struct AxpyPlan {
   }
   void launch(Ctx* ctx, const double* src, const double* alpha, double* C) {
     if (segs.empty()) return;
-    DevBuf ds = upload(ctx, segs), de = upload(ctx, ents);
+    size_t eo = 0;
+    DevBuf ds = upload2(ctx, segs, ents, &eo);
+    const auto* de = reinterpret_cast<const AxpyEntry*>(ds.as<unsigned char>() + eo);
     double flops = 0.0, bytes = 0.0;
     for (auto& g : segs) {
       const double ne = g.e_end - g.e_begin;
@@ -1279,7 +1283,7 @@ struct AxpyPlan {
     }
     {
       ProfScope ps(ctx, PROF_AXPY, flops, bytes);
-      SB_CK(launch_axpy_seg(src, alpha, C, ds.as<AxpySeg>(), static_cast<int64_t>(segs.size()), de.as<AxpyEntry>(),
+      SB_CK(launch_axpy_seg(src, alpha, C, ds.as<AxpySeg>(), static_cast<int64_t>(segs.size()), de,
                             max_len, ctx->stream));
     }
     ctx->note_launch();

@@ -201,6 +201,16 @@ DevBuf upload(Ctx* ctx, const std::vector<T>& v) {
   if (!v.empty()) ctx->stage_copy(b.raw(), v.data(), v.size() * sizeof(T));
   return b;
 }
+// Two plan arrays in one buffer and one copy: second starts at byte off2.
+template <class T, class U>
+DevBuf upload2(Ctx* ctx, const std::vector<T>& a, const std::vector<U>& b, size_t* off2) {
+  const size_t na = a.size() * sizeof(T);
+  *off2 = (na + 15) / 16 * 16;
+  std::vector<unsigned char> h(*off2 + b.size() * sizeof(U));
+  std::copy_n(reinterpret_cast<const unsigned char*>(a.data()), na, h.data());
+  std::copy_n(reinterpret_cast<const unsigned char*>(b.data()), b.size() * sizeof(U), h.data() + *off2);
+  return upload(ctx, h);
+}
 template <class T>
 std::vector<T> download(Ctx* ctx, const void* dptr, size_t n) {
   std::vector<T> v(n);

@@ -949,33 +949,32 @@ __global__ void k_block_extents(const double* __restrict__ src, const int64_t* _
 // TB/s).
 template <int N2>
 __global__ void __launch_bounds__(kThreads)
-    k_block_extents_linear(const double* __restrict__ src, const int64_t* __restrict__ off,
-                           const int64_t* __restrict__ dims, const int64_t* __restrict__ task_begin, int64_t nblocks,
-                           int64_t budget, int* __restrict__ ext) {
+    k_block_extents_linear(const ExtBlock* __restrict__ blocks, int64_t nblocks, int64_t ntasks, int64_t budget,
+                           int* __restrict__ ext) {
   const int lane = threadIdx.x & 31;
-  const int64_t ntasks = task_begin[nblocks];
   const int64_t warps = static_cast<int64_t>(gridDim.x) * (blockDim.x >> 5);
   for (int64_t w = (static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5; w < ntasks; w += warps) {
     int64_t lo = 0, hi = nblocks - 1;  // the last block with task_begin <= w, 32 candidates per round
     while (lo < hi) {
       const int64_t step = (hi - lo + 32) / 32, idx = lo + (lane + 1) * step;
-      const int k = __popc(__ballot_sync(0xffffffffu, idx <= hi && task_begin[idx] <= w));
+      const int k = __popc(__ballot_sync(0xffffffffu, idx <= hi && blocks[idx].task_begin <= w));
       lo += k * step;
       hi = hi < lo + step - 1 ? hi : lo + step - 1;
     }
+    const ExtBlock b = blocks[lo];
     uint32_t d[N2], mul[N2], sh[N2], m[N2];
     uint32_t len = 1;
 #pragma unroll
     for (int r = 0; r < N2; ++r) {
-      d[r] = static_cast<uint32_t>(dims[lo * N2 + r]);
+      d[r] = b.dims[r];
       len *= d[r];
       m[r] = 0;
       sh[r] = d[r] <= 1 ? 0 : 32 - __clz(d[r] - 1);  // as set_divisors
       mul[r] = static_cast<uint32_t>((((uint64_t{1} << sh[r]) - d[r]) << 32) / d[r] + 1);
     }
-    const uint32_t e0 = static_cast<uint32_t>((w - task_begin[lo]) * budget);
+    const uint32_t e0 = static_cast<uint32_t>((w - b.task_begin) * budget);
     const uint32_t e1 = len - e0 < budget ? len : e0 + static_cast<uint32_t>(budget);
-    const double* p = src + off[lo];
+    const double* p = b.p;
     for (uint32_t e = e0 + lane; e < e1; e += 256) {
       double v[8];
 #pragma unroll
@@ -986,8 +985,8 @@ __global__ void __launch_bounds__(kThreads)
           uint32_t x = e + 32 * q;
 #pragma unroll
           for (int r = 0; r < N2; ++r) {
-            const uint32_t next = r + 1 < N2 ? (__umulhi(x, mul[r]) + x) >> sh[r] : 0;
-            const uint32_t c = x - next * (r + 1 < N2 ? d[r] : 0) + 1;
+            const uint32_t next = (__umulhi(x, mul[r]) + x) >> sh[r];
+            const uint32_t c = x - next * d[r] + 1;
             x = next;
             m[r] = c > m[r] ? c : m[r];
           }
@@ -997,7 +996,8 @@ __global__ void __launch_bounds__(kThreads)
     for (int r = 0; r < N2; ++r) m[r] = __reduce_max_sync(0xffffffffu, m[r]);
     if (lane == 0 && m[0] > 0)
 #pragma unroll
-      for (int r = 0; r < N2; ++r) atomicMax(&ext[lo * N2 + r], static_cast<int>(m[r]));
+      for (int r = 0; r < N2; ++r)
+        if (r < b.n2) atomicMax(&ext[b.ext0 + r], static_cast<int>(m[r]));
   }
 }
 
@@ -1005,24 +1005,25 @@ int64_t block_extent_budget(int64_t elems) {
   const int64_t b = elems / (148LL * 48);
   return b < 512 ? 512 : b > 8192 ? 8192 : b;
 }
-int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget, bool linear) {
-  return linear ? (d0 * cols + budget - 1) / budget : ext_tasks(d0, cols, budget);
+int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget) { return ext_tasks(d0, cols, budget); }
+
+cudaError_t launch_block_extents_linear(const ExtBlock* d_blocks, int64_t nblocks, int64_t ntasks, int n2,
+                                        int64_t budget, int* d_ext, cudaStream_t s) {
+  if (ntasks <= 0 || nblocks <= 0) return cudaSuccess;
+  if (n2 < 1 || n2 > 4) return cudaErrorInvalidValue;
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>((ntasks + 7) / 8, 148LL * 8));
+  if (n2 <= 2) k_block_extents_linear<2><<<g, kThreads, 0, s>>>(d_blocks, nblocks, ntasks, budget, d_ext);
+  else if (n2 == 3) k_block_extents_linear<3><<<g, kThreads, 0, s>>>(d_blocks, nblocks, ntasks, budget, d_ext);
+  else k_block_extents_linear<4><<<g, kThreads, 0, s>>>(d_blocks, nblocks, ntasks, budget, d_ext);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_block_extents(const double* src, const int64_t* d_off, const int64_t* d_dims,
                                  const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2,
-                                 int64_t budget, bool linear, int* d_ext, cudaStream_t s) {
+                                 int64_t budget, int* d_ext, cudaStream_t s) {
   if (ntasks <= 0 || nblocks <= 0) return cudaSuccess;
-  if (n2 < 1 || n2 > kMaxRank || (linear && n2 > 4)) return cudaErrorInvalidValue;
+  if (n2 < 1 || n2 > kMaxRank) return cudaErrorInvalidValue;
   const int64_t ctas = std::min<int64_t>((ntasks + 7) / 8, 148LL * 8);
-  const unsigned g = static_cast<unsigned>(ctas);
-  if (linear) {
-    if (n2 == 1) k_block_extents_linear<1><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
-    else if (n2 == 2) k_block_extents_linear<2><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
-    else if (n2 == 3) k_block_extents_linear<3><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
-    else k_block_extents_linear<4><<<g, kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, budget, d_ext);
-    return cudaGetLastError();
-  }
   k_block_extents<<<static_cast<unsigned>(ctas), kThreads, 0, s>>>(src, d_off, d_dims, d_task_begin, nblocks, n2,
                                                                     budget, d_ext);
   return cudaGetLastError();

@@ -311,13 +311,24 @@ cudaError_t launch_perm_block_rows(const double* src, double* dst, const BlockPe
 // the product of the others), starting at d_task_begin[b]; d_task_begin has
 // nblocks + 1 entries, the last = ntasks.  budget: elements per task, 512 to
 // 8192 by the number of elements scanned (block_extent_budget), the same
-// value for every call of one launch; linear (likewise): tails of at most four
-// axes and blocks below 2^31 elements, whose tasks are runs of elements.
+// value for every call of one launch.
 int64_t block_extent_budget(int64_t elems);
-int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget, bool linear);
+int64_t block_extent_tasks(int64_t d0, int64_t cols, int64_t budget);
 cudaError_t launch_block_extents(const double* src, const int64_t* d_off, const int64_t* d_dims,
                                  const int64_t* d_task_begin, int64_t nblocks, int64_t ntasks, int n2,
-                                 int64_t budget, bool linear, int* d_ext, cudaStream_t s);
+                                 int64_t budget, int* d_ext, cudaStream_t s);
+// The same for blocks below 2^31 elements with tails of at most four axes
+// (n2 = the most any block has; dims beyond a block's own n2 are 1), of any
+// number of tensors in one launch: tasks are runs of `budget` elements, block
+// b's starting at task_begin, its results at ext[ext0 ..] (0 = all zero).
+struct ExtBlock {
+  const double* p;
+  int64_t task_begin;
+  uint32_t dims[4];
+  int32_t ext0, n2;
+};
+cudaError_t launch_block_extents_linear(const ExtBlock* d_blocks, int64_t nblocks, int64_t ntasks, int n2,
+                                        int64_t budget, int* d_ext, cudaStream_t s);
 // flags[i] = 1 if block i of src holds a nonzero outside its box in_lim
 // (used to check that cropping a padded block loses nothing).
 cudaError_t launch_outside_nonzero(const double* src, const BlockPerm* d_items, int64_t n, int64_t max_len,

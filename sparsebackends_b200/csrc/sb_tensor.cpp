@@ -343,16 +343,32 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
     for (size_t k = 0; k < ts.size(); ++k) out[k].assign(ts[k]->nkeys * ts[k]->n2, 1);
     return out;
   }
-  DevBuf dext = upload(ctx, std::vector<int>(base.back(), 1));
+  DevBuf dext(ctx, base.back() * sizeof(int));
+  SB_CK(cudaMemsetAsync(dext.raw(), 0, base.back() * sizeof(int), ctx->stream));
   std::vector<DevBuf> keep;
+  // tensors of up to four tail axes go into one launch (and one upload)
+  std::vector<ExtBlock> lin;
+  int64_t lin_tasks = 0, elems = 0;
+  int lin_n2 = 0;
+  for (const Tensor* t : ts) elems += t->payload_len();
+  const int64_t budget = block_extent_budget(elems);
   for (size_t k = 0; k < ts.size(); ++k) {
     const Tensor& A = *ts[k];
     const int64_t n = A.nkeys;
     if (n == 0 || A.n2 == 0) continue;
-    std::vector<int64_t> off(n), dims(n * A.n2), tb(n + 1, 0);
-    const int64_t budget = block_extent_budget(A.payload_len());
-    bool linear = A.n2 <= 4;
+    bool linear = A.n2 <= 4 && base.back() < (int64_t{1} << 31);
     for (int64_t i = 0; i < n; ++i) linear = linear && A.block_len(i) < (int64_t{1} << 31);
+    if (linear) {
+      lin_n2 = std::max(lin_n2, A.n2);
+      for (int64_t i = 0; i < n; ++i) {
+        ExtBlock b{A.payload() + A.block_off(i), lin_tasks, {1, 1, 1, 1}, static_cast<int32_t>(base[k] + i * A.n2), A.n2};
+        for (int t = 0; t < A.n2; ++t) b.dims[t] = static_cast<uint32_t>(A.block_dim(i, t));
+        lin.push_back(b);
+        lin_tasks += (A.block_len(i) + budget - 1) / budget;
+      }
+      continue;
+    }
+    std::vector<int64_t> off(n), dims(n * A.n2), tb(n + 1, 0);
     for (int64_t i = 0; i < n; ++i) {
       off[i] = A.block_off(i);
       int64_t cols = 1;
@@ -360,19 +376,28 @@ std::vector<std::vector<int64_t>> bs_nonzero_extents(Ctx* ctx, const std::vector
         dims[i * A.n2 + t] = A.block_dim(i, t);
         if (t > 0) cols *= dims[i * A.n2 + t];
       }
-      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols, budget, linear);
+      tb[i + 1] = tb[i] + block_extent_tasks(dims[i * A.n2], cols, budget);
     }
     keep.push_back(upload(ctx, off));
     keep.push_back(upload(ctx, dims));
     keep.push_back(upload(ctx, tb));
     const size_t m = keep.size();
     SB_CK(launch_block_extents(A.payload(), keep[m - 3].as<int64_t>(), keep[m - 2].as<int64_t>(),
-                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, budget, linear,
-                               dext.as<int>() + base[k], ctx->stream));
+                               keep[m - 1].as<int64_t>(), n, tb[n], A.n2, budget, dext.as<int>() + base[k],
+                               ctx->stream));
+    ctx->note_launch();
+  }
+  if (!lin.empty()) {
+    keep.push_back(upload(ctx, lin));
+    SB_CK(launch_block_extents_linear(keep.back().as<ExtBlock>(), static_cast<int64_t>(lin.size()), lin_tasks, lin_n2,
+                                      budget, dext.as<int>(), ctx->stream));
     ctx->note_launch();
   }
   const auto e = download<int>(ctx, dext.raw(), base.back());
-  for (size_t k = 0; k < ts.size(); ++k) out[k].assign(e.begin() + base[k], e.begin() + base[k + 1]);
+  for (size_t k = 0; k < ts.size(); ++k) {
+    out[k].resize(base[k + 1] - base[k]);
+    for (int64_t i = base[k]; i < base[k + 1]; ++i) out[k][i - base[k]] = std::max(e[i], 1);
+  }
   return out;
 }
 
