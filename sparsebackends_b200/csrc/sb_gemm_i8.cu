@@ -500,7 +500,14 @@ __global__ void __launch_bounds__(256) k_i8_reduce(const double* __restrict__ pa
   for (int c = static_cast<int>(threadIdx.x) >> 7; c < cols; c += 2) {
     const double* p = partial + static_cast<int64_t>(sp.part0) * kI8PartElems + r + (c0 + c) * 128;
     double acc = 0.0;
-    for (int q = 0; q < sp.nparts; ++q) acc = __dadd_rn(acc, p[q * kI8PartElems]);
+    for (int q = 0; q < sp.nparts; q += 4) {  // four loads in flight, added in segment order
+      double v[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) v[j] = q + j < sp.nparts ? p[(q + j) * kI8PartElems] : 0.0;
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (q + j < sp.nparts) acc = __dadd_rn(acc, v[j]);
+    }
     C[c_off + static_cast<int64_t>(sp.b0 + c0 + c) * c_ld] = acc;
   }
 }

@@ -146,21 +146,24 @@ __device__ __forceinline__ uint32_t img_off(int r, int c) {
 // zero; hi plane at dst, lo plane at dst + plane (plane = image rows x 128 B).
 template <bool F64>
 __global__ void __launch_bounds__(256)
-    k_tc_pack(const void* __restrict__ srcv, const TcImage* __restrict__ imgs, int64_t nimg,
+    k_tc_pack(const void* __restrict__ srcv, const TcImage* __restrict__ imgs, int64_t nimg, int slices,
               unsigned char* __restrict__ dst, int32_t passes) {
   const int tid = static_cast<int>(threadIdx.x);
-  for (int64_t i = blockIdx.x; i < nimg; i += gridDim.x) {
-    const TcImage im = imgs[i];
+  for (int64_t u = blockIdx.x; u < nimg * slices; u += gridDim.x) {
+    const TcImage im = imgs[u / slices];
     const int rows_img = im.plane >> 7;
     const int nchunks = rows_img * 8;
     unsigned char* const d = dst + im.dst;
-    for (int ch = tid; ch < nchunks; ch += 256) {
+    for (int ch = tid + 256 * static_cast<int>(u % slices); ch < nchunks; ch += 256 * slices) {
       // k-contiguous sources: a warp takes the 8 chunks of 4 rows;
-      // row-contiguous ones: 4 chunks of 8 rows, so that both the loads (8
-      // consecutive rows) and the stores (64 bytes of a row) fill their sectors
-      // (32 rows of one chunk, stored 128 bytes apart, packed L and R of the
-      // chi = 2048 H_eff at 2.2 TB/s: 600 us for its four packs, now 382)
-      const int r = im.kc ? ch >> 3 : (ch >> 6 << 3) + (ch >> 2 & 7), c = im.kc ? ch & 7 : (ch >> 5 & 1) * 4 + (ch & 3);
+      // row-contiguous FP64 ones: 2 chunks of 16 rows, so that both the loads
+      // (16 consecutive rows) and the stores (two chunks of a row are 32
+      // contiguous bytes under the swizzle) fill their sectors (with 32 rows of
+      // one chunk, stored 128 bytes apart, L and R of the chi = 2048 H_eff
+      // packed at 2.2 TB/s: 600 us for its four packs, now 388); FP32 ones: 32
+      // rows of one chunk, whose loads are half as wide
+      const int r = im.kc ? ch >> 3 : F64 ? (ch >> 7 << 4) + (ch >> 1 & 15) : ch % rows_img;
+      const int c = im.kc ? ch & 7 : F64 ? (ch >> 5 & 3) * 2 + (ch & 1) : ch / rows_img;
       uint32_t h[4], l[4];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -476,9 +479,17 @@ __global__ void __launch_bounds__(256) k_tc_reduce(const double* __restrict__ pa
   for (int e = tid; e < 128 * 32; e += 256) {
     const int r = e & 127, c = e >> 7;
     double acc = 0.0;
-    if (r < rows && c < cols)
-      for (int q = 0; q < sp.nparts; ++q)
-        acc += partial[static_cast<int64_t>(sp.part0 + q) * kTcPartElems + r + (c0 + c) * 128];
+    if (r < rows && c < cols) {
+      const double* p = partial + static_cast<int64_t>(sp.part0) * kTcPartElems + r + (c0 + c) * 128;
+      for (int q = 0; q < sp.nparts; q += 8) {  // eight loads in flight, added in segment order
+        double v[8];
+#pragma unroll
+        for (int j = 0; j < 8; ++j) v[j] = q + j < sp.nparts ? p[(q + j) * kTcPartElems] : 0.0;
+#pragma unroll
+        for (int j = 0; j < 8; ++j)
+          if (q + j < sp.nparts) acc += v[j];
+      }
+    }
     S[c][r] = acc;
   }
   __syncthreads();
@@ -503,11 +514,15 @@ cudaError_t launch_tc_pack(const void* src, bool src_f64, const TcImage* d_imgs,
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const unsigned g = static_cast<unsigned>(std::min<int64_t>(nimg, 8LL * sms));
+  // few images: several CTAs each, so that every SM has its share of loads in
+  // flight (the four packs of a chi = 762 H_eff, 110 to 476 images each: 56 us
+  // with one CTA per image, 41 now)
+  const int slices = 4 * nimg <= 8LL * sms ? 4 : 2 * nimg <= 8LL * sms ? 2 : 1;
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>(nimg * slices, 8LL * sms));
   if (src_f64)
-    k_tc_pack<true><<<g, 256, 0, s>>>(src, d_imgs, nimg, static_cast<unsigned char*>(dst), passes);
+    k_tc_pack<true><<<g, 256, 0, s>>>(src, d_imgs, nimg, slices, static_cast<unsigned char*>(dst), passes);
   else
-    k_tc_pack<false><<<g, 256, 0, s>>>(src, d_imgs, nimg, static_cast<unsigned char*>(dst), passes);
+    k_tc_pack<false><<<g, 256, 0, s>>>(src, d_imgs, nimg, slices, static_cast<unsigned char*>(dst), passes);
   return cudaGetLastError();
 }
 
