@@ -574,21 +574,24 @@ def contract_new(labelsC, n2C, A, labelsA, B, labelsB):
 # The three contract! calls of each environment update: (labels of the result,
 # its tail count, labels of the left operand, labels of the right operand).
 # make_L: E1 = L*A, E2 = E1*W, L' = E2*A;  make_R: F1 = R*B, F2 = F1*W, R' = F2*B.
+# E2 and F2 put the axis that the last step reduces at the end of their tails,
+# which is the order that step reads (with it in the middle, each update
+# permuted the whole intermediate: 30 of 297 us at chi = 1024, w = 26).
 MAKE_L_STEPS = (
     (["qlp", "qwl", "s1", "qr", "mr", "mlp", "mwl"], 3,
      ["qlp", "qwl", "ql", "mlp", "mwl", "ml"], ["ql", "s1", "qr", "ml", "mr"]),
-    (["qlp", "qr", "s1p", "qwm", "mr", "mlp", "mwm"], 3,
+    (["qlp", "qr", "s1p", "qwm", "mwm", "mr", "mlp"], 3,
      ["qlp", "qwl", "s1", "qr", "mr", "mlp", "mwl"], ["qwl", "s1p", "s1", "qwm", "mwl", "mwm"]),
     (["qrp", "qwm", "qr", "mrp", "mwm", "mr"], 3,
-     ["qlp", "qr", "s1p", "qwm", "mr", "mlp", "mwm"], ["qlp", "s1p", "qrp", "mlp", "mrp"]),
+     ["qlp", "qr", "s1p", "qwm", "mwm", "mr", "mlp"], ["qlp", "s1p", "qrp", "mlp", "mrp"]),
 )
 MAKE_R_STEPS = (
     (["qrp", "qwm", "ql", "s1", "ml", "mrp", "mwm"], 3,
      ["qrp", "qwm", "qr", "mrp", "mwm", "mr"], ["ql", "s1", "qr", "ml", "mr"]),
-    (["qrp", "ql", "s1p", "qwl", "ml", "mrp", "mwl"], 3,
+    (["qrp", "ql", "s1p", "qwl", "mwl", "ml", "mrp"], 3,
      ["qrp", "qwm", "ql", "s1", "ml", "mrp", "mwm"], ["qwl", "s1p", "s1", "qwm", "mwl", "mwm"]),
     (["qlp", "qwl", "ql", "mlp", "mwl", "ml"], 3,
-     ["qrp", "ql", "s1p", "qwl", "ml", "mrp", "mwl"], ["qlp", "s1p", "qrp", "mlp", "mrp"]),
+     ["qrp", "ql", "s1p", "qwl", "mwl", "ml", "mrp"], ["qlp", "s1p", "qrp", "mlp", "mrp"]),
 )
 
 
