@@ -3,6 +3,7 @@
 // Every launcher enqueues work on the given stream and returns immediately.
 // Offsets are in elements (doubles) relative to the base pointers passed.
 #pragma once
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -274,8 +275,7 @@ struct BlockPerm {
 inline void set_divisors(BlockPerm& b) {
   for (int r = 0; r < b.rank; ++r) {
     const uint64_t d = static_cast<uint64_t>(b.out_dims[r]);
-    uint32_t s = 0;
-    while (s < 32 && (uint64_t{1} << s) < d) ++s;
+    const uint32_t s = d <= 1 ? 0 : std::min(32u, 64u - static_cast<uint32_t>(__builtin_clzll(d - 1)));
     b.div_shift[r] = s;
     b.div_mul[r] = d < 1 || d >= (uint64_t{1} << 31) ? 0
                    : static_cast<uint32_t>((uint64_t{1} << 32) * ((uint64_t{1} << s) - d) / d + 1);

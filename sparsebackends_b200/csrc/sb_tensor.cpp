@@ -269,6 +269,7 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
     ctx->note_launch();
     return;
   }
+  for (auto& it : items) set_divisors(it);
   DevBuf d = upload(ctx, items);
   ProfScope ps(ctx, PROF_PERMUTE, 0.0, bytes);
   if (rows)
@@ -293,7 +294,6 @@ static BlockPerm make_block_perm(int64_t src_off, int64_t dst_off, const std::ve
     b.in_lim[r] = in_lim[r];
     b.len *= out_dims[r];
   }
-  set_divisors(b);
   return b;
 }
 
@@ -432,6 +432,7 @@ TensorPtr bs_to_ragged(Ctx* ctx, const Tensor& A, const std::vector<int64_t>& bd
   if (reuse && reuse->bytes() == need) out->data = std::move(*reuse);
   else out->data = DevBuf(ctx, need);
   std::vector<BlockPerm> items, checks;
+  items.reserve(A.nkeys);
   for (int64_t i = 0; i < A.nkeys; ++i) {
     std::vector<int64_t> od(A.n2), st(A.n2), full(A.n2);
     int64_t acc = 1;
@@ -503,6 +504,7 @@ TensorPtr bs_permute(Ctx* ctx, const Tensor& A, const std::vector<int>& perm) {
       copy_blocks(ctx, A.payload(), out->data.d(), so, dof, len);
     } else {
       std::vector<BlockPerm> items;
+      items.reserve(n);
       for (int64_t i = 0; i < n; ++i) {
         std::vector<int64_t> sst(A.n2), od(A.n2), is(A.n2);
         int64_t acc = 1;
