@@ -301,7 +301,7 @@ struct GemmLaunch {
   // images as above, nscale operand rows; nf = 64x64 tiles of the DMMA launch
   // behind the flag
   int64_t nscale = 0, nf = 0;
-  int32_t nctas = 0;
+  int32_t nctas = 0, strip = 0;  // longest K when images are strips, else 0
   double flops = 0.0, bytes = 0.0;
   char desc[sizeof(Ctx::gemm_desc)] = "";
   // Integer tensor-core launch.  One stream-ordered scratch buffer per call
@@ -331,9 +331,10 @@ struct GemmLaunch {
     SB_CK(cudaMemsetAsync(rowhi, 0, (nscale + 1) * 4, ctx->stream));
     {
       ProfScope ps(ctx, PROF_TC_PACK, 0.0,
-                   16.0 * (pack_a_elems + pack_b_elems) + static_cast<double>(pack_a_bytes + pack_b_bytes));
-      SB_CK(launch_i8_pack(X, dimg_a.as<I8Image>(), nimg_a, rowhi, b, flag, ctx->stream));
-      SB_CK(launch_i8_pack(Y, dimg_b.as<I8Image>(), nimg_b, rowhi, b, flag, ctx->stream));
+                   (strip > 0 ? 8.0 : 16.0) * (pack_a_elems + pack_b_elems) +
+                       static_cast<double>(pack_a_bytes + pack_b_bytes));
+      SB_CK(launch_i8_pack(X, dimg_a.as<I8Image>(), nimg_a, strip, rowhi, b, flag, ctx->stream));
+      SB_CK(launch_i8_pack(Y, dimg_b.as<I8Image>(), nimg_b, strip, rowhi, b, flag, ctx->stream));
     }
     {
       ProfScope ps(ctx, PROF_GEMM, flops, bytes);
@@ -343,7 +344,7 @@ struct GemmLaunch {
       SB_CK(launch_gemm_f64_fallback(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), nf, xT, yT, flag,
                                      ctx->stream));
     }
-    ctx->note_launch((nimg_a > 0 ? 2 : 0) + (nimg_b > 0 ? 2 : 0) + (nsplits > 0 ? 3 : 2));
+    ctx->note_launch(((nimg_a > 0) + (nimg_b > 0)) * (strip > 0 ? 1 : 2) + (nsplits > 0 ? 3 : 2));
   }
   // Tensor-core launch: X and Y FP64 or FP32 arrays (versions 0 = unknown,
   // packed every call), C FP64 or FP32.
@@ -858,6 +859,11 @@ struct GemmPlan {
     // second read hits L2, was slower: 565 and 474 us against 402 for R*T3)
     const bool akc = g.xT, bkc = !g.yT;
     std::vector<I8Pack> pk(npairs, I8Pack{});
+    // one pass over the operands while every K is short (strips of one launch
+    // next to k-tiles of two cost more than they save: R*T3 402 -> 423 us)
+    int32_t kmax = 0;
+    for (const GemmPair& q : pairs) kmax = std::max(kmax, q.K);
+    const int32_t strip = kmax <= kI8StripK ? kmax : 0;
     std::vector<I8Image> ia, ib;
     struct Seen { int64_t base, scale; };
     struct Seg { int64_t off, ld, rows; };  // a block of the stack
@@ -879,7 +885,24 @@ struct GemmPlan {
       for (const Seg& q : segs) rows += q.rows;
       size_t si = 0;
       int64_t sr = 0;  // block and row in it that the tile starts with
-      for (int64_t r0 = 0; r0 < rows; r0 += tile) {
+      if (strip > 0) {
+        const int64_t image = up(K, 64) * 7 * tile;  // bytes of a row tile
+        for (int64_t r = 0; r < rows;) {
+          const Seg& q = segs[si];
+          const int64_t at = r % tile, n = std::min({q.rows - sr, 16 - at % 16, tile - at});
+          out.push_back(I8Image{q.off + (kc ? sr * q.ld : sr), q.ld, total + r / tile * image,
+                                static_cast<int32_t>(nscale + r), static_cast<int32_t>(at), static_cast<int32_t>(n),
+                                static_cast<int32_t>(r + n == rows ? tile : at + n), static_cast<int32_t>(tile),
+                                static_cast<int32_t>(K), kc ? 1 : 0, 0});
+          r += n;
+          if ((sr += n) == q.rows) {
+            ++si;
+            sr = 0;
+          }
+        }
+        total += (rows + tile - 1) / tile * image;
+      }
+      for (int64_t r0 = 0; strip == 0 && r0 < rows; r0 += tile) {
         const int64_t r1 = std::min(rows, r0 + tile);
         for (int64_t k0 = 0; k0 < K; k0 += 64) {
           size_t i = si;
@@ -935,7 +958,8 @@ struct GemmPlan {
         pk[gr.p0 + j].b_sc = static_cast<int32_t>(b.scale);
         if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
       }
-    const double t_i8 = cycles / sms / 1.85e9 + (16.0 * (elems_a + elems_b) + total) / 4.5e12 + 30e-6;
+    const double pack = (strip > 0 ? 8.0 : 16.0) * (elems_a + elems_b) + total;
+    const double t_i8 = cycles / sms / 1.85e9 + pack / 4.5e12 + 30e-6;
     const double t_f64 = flops / 27e12 + 5e-6;
     if (ctx->gemm_i8 < 0 && t_i8 > 0.95 * t_f64) return false;
     // k-segments when the tiles are fewer than four per SM, as in prepare_tc
@@ -1004,6 +1028,7 @@ struct GemmPlan {
       f += static_cast<int64_t>(c.mtiles) * ((c.N + 63) / 64);
     }
     g.kind = GemmLaunch::I8;
+    g.strip = strip;
     g.dfirst = upload(ctx, first);
     g.nctas = nctas;
     std::vector<I8Group> dg;

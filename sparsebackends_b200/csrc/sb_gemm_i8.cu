@@ -26,7 +26,8 @@
 // k-tile, of the high words), k_i8_pack writes the seven digit planes of each
 // 64-deep k-tile of each 128-row tile of X and nbs-column tile of Y in the
 // layout the tensor core reads from shared memory (K-major, 64-byte swizzle),
-// (rows of several C blocks that read the same Y blocks are stacked, I8Group);
+// (rows of several C blocks that read the same Y blocks are stacked, I8Group); with
+// every K at most 768 k_i8_pack_strip does both in one pass;
 // k_gemm_i8 is persistent, one CTA per SM: warp 0 moves images with bulk
 // copies, warp 1 issues the MMAs, warps 4-11 drain.  A tile is 128 x nb (nb <=
 // 128, a multiple of 16).  INT32 accumulators of 128 columns for four diagonals
@@ -126,6 +127,57 @@ __global__ void __launch_bounds__(256)
   }
 }
 
+// K-major 64-byte swizzle: byte of image row ri, chunk c of 16 k in its plane.
+__device__ __forceinline__ int digit_at(int ri, int c) {
+  return (ri >> 3) * 512 + (ri & 7) * 64 + ((c ^ ((ri >> 1) & 3)) << 4);
+}
+
+// Seven digits of a row's 16 consecutive k (largest magnitude hi) into the
+// planes at o.
+__device__ __forceinline__ void put_digits(double (&x)[16], uint32_t hi, bool store, unsigned char* o, int plane,
+                                           int* flag) {
+      double f = 0.0;
+      if (hi != 0) {
+        const int e = scale_exp(hi);
+        if (e < -400 || e > 400) {
+          *flag = 1;  // the DMMA launch recomputes (also infinities and NaN)
+#pragma unroll
+          for (int j = 0; j < 16; ++j) x[j] = 0.0;
+        } else {
+          f = pow2(54 - e);
+        }
+      }
+      uint32_t w[kI8Planes][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        uint32_t lo[4], up[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          // balanced digits: add 128 to each of the seven bytes, then take 128 off
+          // again byte by byte (flip the top bit)
+          const uint64_t v = (static_cast<uint64_t>(__double2ll_rn(__dmul_rn(x[4 * q + j], f))) + 0x0080808080808080ull) ^
+                             0x0080808080808080ull;
+          lo[j] = static_cast<uint32_t>(v);
+          up[j] = static_cast<uint32_t>(v >> 32);
+        }
+        // 4 x 4 byte transposes: plane 6 holds the lowest byte of each value
+        const uint32_t a0 = __byte_perm(lo[0], lo[1], 0x5140), a1 = __byte_perm(lo[0], lo[1], 0x7362);
+        const uint32_t b0 = __byte_perm(lo[2], lo[3], 0x5140), b1 = __byte_perm(lo[2], lo[3], 0x7362);
+        w[6][q] = __byte_perm(a0, b0, 0x5410);
+        w[5][q] = __byte_perm(a0, b0, 0x7632);
+        w[4][q] = __byte_perm(a1, b1, 0x5410);
+        w[3][q] = __byte_perm(a1, b1, 0x7632);
+        const uint32_t c0 = __byte_perm(up[0], up[1], 0x5140), c1 = __byte_perm(up[0], up[1], 0x7362);
+        const uint32_t d0 = __byte_perm(up[2], up[3], 0x5140), d1 = __byte_perm(up[2], up[3], 0x7362);
+        w[2][q] = __byte_perm(c0, d0, 0x5410);
+        w[1][q] = __byte_perm(c0, d0, 0x7632);
+        w[0][q] = __byte_perm(c1, d1, 0x5410);
+      }
+  if (store)
+#pragma unroll
+    for (int q = 0; q < kI8Planes; ++q) st_global_v4(o + q * plane, w[q][0], w[q][1], w[q][2], w[q][3]);
+}
+
 // Digit planes of one k-tile image: a warp takes 8 rows, lane = 4*row + chunk
 // of 16 k, so that its 16-byte stores cover 512 contiguous bytes per plane.
 // k-contiguous rows go through a shared-memory copy (loads coalesced along k;
@@ -166,48 +218,81 @@ __global__ void __launch_bounds__(256)
         x[j] = r >= 0 && r < im.rows && 16 * c + j < im.kv ? p[static_cast<int64_t>(j) * im.ld] : 0.0;
     }
     const uint32_t hi = r >= 0 && r < im.rows ? rowhi[im.scale + r] : 0u;
-    double f = 0.0;
-    if (hi != 0) {
-      const int e = scale_exp(hi);
-      if (e < -400 || e > 400) {
-        *flag = 1;  // the DMMA launch recomputes (also infinities and NaN)
-#pragma unroll
-        for (int j = 0; j < 16; ++j) x[j] = 0.0;
-      } else {
-        f = pow2(54 - e);
-      }
+    put_digits(x, hi, r >= 0 && ri < im.row_end, d + digit_at(ri, c), plane, flag);
+  }
+}
+
+// Doubles from one row of a strip to the next in shared memory.
+__host__ __device__ constexpr int strip_stride(int k) {
+  const int n = (k + kI8BK - 1) / kI8BK;
+  return 68 * n + ((4 - 4 * n) & 15);
+}
+
+__device__ __forceinline__ void cp_async8(double* smem, const double* g) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(static_cast<uint32_t>(__cvta_generic_to_shared(smem))),
+               "l"(g)
+               : "memory");
+}
+
+// The same for strips: up to 16 image rows and all of their K, which is in
+// shared memory while the scales are found and the digits written, so that HBM
+// is read once and one launch does both.  Element (r, k) lies at r*ss + (r >> 2)
+// + k + (k >> 4), ss = 4 modulo 16: no bank conflicts for 16 rows of one k, for
+// a row's consecutive k, or for 4 rows x 4 chunks.  The issue of the conversion
+// and the phases' latencies bound it (a double-buffered persistent form was
+// slower, 163 us), not HBM: the packs of psi*L at chi = 2048 119 -> 103 us, 1400
+// 74 -> 57, 1024 51 -> 40.
+__global__ void __launch_bounds__(256)
+    k_i8_pack_strip(const double* __restrict__ src, const I8Image* __restrict__ imgs, uint32_t* __restrict__ rowhi,
+                    unsigned char* __restrict__ dst, int* __restrict__ flag) {
+  extern __shared__ double strip[];
+  __shared__ uint32_t top[8 * 16];
+  const I8Image im = imgs[blockIdx.x];
+  const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31;
+  const int nkt = (im.kv + kI8BK - 1) / kI8BK, ss = strip_stride(im.kv);
+  const int r16 = tid & 15;
+  const double* s = src + im.src;
+  if (im.kc) {
+    for (int r = warp; r < im.rows; r += 8) {
+      const double* p = s + static_cast<int64_t>(r) * im.ld;
+      double* q = strip + r * ss + (r >> 2);
+#pragma unroll 4
+      for (int k = lane; k < im.kv; k += 32) cp_async8(q + k + (k >> 4), p + k);
     }
-    uint32_t w[kI8Planes][4];
+  } else if (r16 < im.rows) {
+    double* q = strip + r16 * ss + (r16 >> 2);
+#pragma unroll 4
+    for (int k = tid >> 4; k < im.kv; k += 16) cp_async8(q + k + (k >> 4), s + r16 + static_cast<int64_t>(k) * im.ld);
+  }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  uint32_t m = 0;
+  if (r16 < im.rows) {
+    const double* q = strip + r16 * ss + (r16 >> 2);
+#pragma unroll 4
+    for (int k = tid >> 4; k < im.kv; k += 16) m = max(m, abs_hi(q[k + (k >> 4)]));
+  }
+  m = max(m, __shfl_xor_sync(0xffffffffu, m, 16));
+  if (lane < 16) top[16 * warp + lane] = m;
+  __syncthreads();
+  if (tid < 16) {
+    for (int j = 1; j < 8; ++j) m = max(m, top[16 * j + tid]);
+    top[tid] = m;
+    if (tid < im.rows) rowhi[im.scale + tid] = m;
+  }
+  __syncthreads();
+  const int plane = im.rows_img * kI8BK;
+  const int g0 = im.row0 / 8, ng = (im.row_end + 7) / 8 - g0;
+  for (int u = warp; u < ng * nkt; u += 8) {
+    const int kt = u / ng, rl = lane >> 2, c = lane & 3;
+    const int ri = 8 * (g0 + u - kt * ng) + rl, r = ri - im.row0, k0 = kt * kI8BK + 16 * c;
+    const bool own = r >= 0 && r < im.rows;
+    const double* p = strip + r * ss + (r >> 2) + k0 + (k0 >> 4);
+    double x[16];
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      uint32_t lo[4], up[4];
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        // balanced digits: add 128 to each of the seven bytes, then take 128 off
-        // again byte by byte (flip the top bit)
-        const uint64_t v = (static_cast<uint64_t>(__double2ll_rn(__dmul_rn(x[4 * q + j], f))) + 0x0080808080808080ull) ^
-                           0x0080808080808080ull;
-        lo[j] = static_cast<uint32_t>(v);
-        up[j] = static_cast<uint32_t>(v >> 32);
-      }
-      // 4 x 4 byte transposes: plane 6 holds the lowest byte of each value
-      const uint32_t a0 = __byte_perm(lo[0], lo[1], 0x5140), a1 = __byte_perm(lo[0], lo[1], 0x7362);
-      const uint32_t b0 = __byte_perm(lo[2], lo[3], 0x5140), b1 = __byte_perm(lo[2], lo[3], 0x7362);
-      w[6][q] = __byte_perm(a0, b0, 0x5410);
-      w[5][q] = __byte_perm(a0, b0, 0x7632);
-      w[4][q] = __byte_perm(a1, b1, 0x5410);
-      w[3][q] = __byte_perm(a1, b1, 0x7632);
-      const uint32_t c0 = __byte_perm(up[0], up[1], 0x5140), c1 = __byte_perm(up[0], up[1], 0x7362);
-      const uint32_t d0 = __byte_perm(up[2], up[3], 0x5140), d1 = __byte_perm(up[2], up[3], 0x7362);
-      w[2][q] = __byte_perm(c0, d0, 0x5410);
-      w[1][q] = __byte_perm(c0, d0, 0x7632);
-      w[0][q] = __byte_perm(c1, d1, 0x5410);
-    }
-    // K-major 64-byte swizzle: row r at (r/8)*512 + (r%8)*64, chunk c at c ^ ((r/2) % 4)
-    unsigned char* o = d + (ri >> 3) * 512 + (ri & 7) * 64 + ((c ^ ((ri >> 1) & 3)) << 4);
-    if (r >= 0 && ri < im.row_end)
-#pragma unroll
-      for (int q = 0; q < kI8Planes; ++q) st_global_v4(o + q * plane, w[q][0], w[q][1], w[q][2], w[q][3]);
+    for (int j = 0; j < 16; ++j) x[j] = own && k0 + j < im.kv ? p[j] : 0.0;
+    put_digits(x, own ? top[r] : 0u, r >= 0 && ri < im.row_end,
+               dst + im.dst + static_cast<int64_t>(kt) * kI8Planes * plane + digit_at(ri, c), plane, flag);
   }
 }
 
@@ -514,15 +599,32 @@ __global__ void __launch_bounds__(256) k_i8_reduce(const double* __restrict__ pa
 
 }  // namespace
 
-cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, uint32_t* d_rowhi, void* dst,
-                           int* d_flag, cudaStream_t s) {
+cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, int32_t strip_k, uint32_t* d_rowhi,
+                           void* dst, int* d_flag, cudaStream_t s) {
   if (nimg <= 0) return cudaSuccess;
-  if (nimg > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (nimg > 0x7fffffffLL || strip_k > kI8StripK) return cudaErrorInvalidValue;
   const unsigned g = static_cast<unsigned>(nimg);
+  unsigned char* const d = static_cast<unsigned char*>(dst);
+  if (strip_k > 0) {
+    auto smem = [](int k) { return static_cast<size_t>(16 * strip_stride(k) + 4) * sizeof(double); };
+    static std::atomic<unsigned long long> configured{0};  // as in launch_gemm_i8
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(configured & bit)) {
+      e = cudaFuncSetAttribute(k_i8_pack_strip, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                               static_cast<int>(smem(kI8StripK)));
+      if (e != cudaSuccess) return e;
+      configured.fetch_or(bit);
+    }
+    k_i8_pack_strip<<<g, 256, smem(strip_k), s>>>(src, d_imgs, d_rowhi, d, d_flag);
+    return cudaGetLastError();
+  }
   k_i8_rowmax<<<g, 256, 0, s>>>(src, d_imgs, d_rowhi);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  k_i8_pack<<<g, 256, 0, s>>>(src, d_imgs, d_rowhi, static_cast<unsigned char*>(dst), d_flag);
+  k_i8_pack<<<g, 256, 0, s>>>(src, d_imgs, d_rowhi, d, d_flag);
   return cudaGetLastError();
 }
 

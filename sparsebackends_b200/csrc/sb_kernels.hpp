@@ -168,13 +168,16 @@ struct I8Group {
 // [row0, row0 + rows) are an operand block's, element (r, k) at src + r*ld + k
 // when kc, else src + r + k*ld, kv <= 64 of them along k; rows up to row_end and
 // the rest of k are zeros.  Seven planes of rows_img * 64 bytes at byte dst; the
-// scale of row row0 at index scale.
+// scale of row row0 at index scale.  With strip_k > 0 an entry is a strip: rows
+// of an aligned range of 16 image rows and all of K (kv <= strip_k <=
+// kI8StripK), its k-tiles' images one after the other.
 struct I8Image {
   int64_t src, ld, dst;
   int32_t scale, row0, rows, row_end, rows_img, kv, kc, pad;
 };
-cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, uint32_t* d_rowhi, void* dst,
-                           int* d_flag, cudaStream_t s);
+constexpr int32_t kI8StripK = 768;  // 16 rows of 768: two CTAs per SM
+cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, int32_t strip_k, uint32_t* d_rowhi,
+                           void* dst, int* d_flag, cudaStream_t s);
 // Per pair: byte offsets of the images of its X block (row tiles of 128, nkt
 // k-tiles each) and Y block (column tiles of nbs), and the scale indices of
 // their first row and column.

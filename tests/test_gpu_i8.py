@@ -83,6 +83,13 @@ def test_edges_of_tiles_and_chunks(m, n, ks, order):
     assert _worst(got, A, B)[0] <= 8 * 2.0 ** -55
 
 
+@pytest.mark.parametrize("order", ["AB", "BA"])
+@pytest.mark.parametrize("m,n,ks", [(15, 16, (768, 1)), (17, 31, (767,)), (33, 129, (769, 5)), (145, 47, (64, 703))])
+def test_edges_of_strips(m, n, ks, order):
+    """Packing in strips of 16 rows while every K is at most 768."""
+    test_edges_of_tiles_and_chunks(m, n, ks, order)
+
+
 @pytest.mark.parametrize("kind", ["gaussian", "graded_k", "graded_rows", "one_large", "opposed", "positive"])
 def test_error_not_above_dmma(kind):
     """Root-mean-square error against |row| |column|, next to the DMMA path's,
