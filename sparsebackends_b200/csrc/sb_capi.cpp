@@ -65,6 +65,7 @@ void destroy_ctx_now(sb_ctx* ctx) {
   ctx->impl.crop_scratch.reset();
   ctx->impl.tc_status.reset();
   ctx->impl.dot_scratch.reset();
+  ctx->impl.i8_scratch.reset();
   cudaStreamSynchronize(ctx->impl.stream);
   if (ctx->impl.host_scalar) cudaFreeHost(ctx->impl.host_scalar);
   ctx->impl.release_staging();

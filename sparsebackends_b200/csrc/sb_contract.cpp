@@ -304,20 +304,24 @@ struct GemmLaunch {
   int32_t nctas = 0, strip = 0;  // longest K when images are strips, else 0
   double flops = 0.0, bytes = 0.0;
   char desc[sizeof(Ctx::gemm_desc)] = "";
-  // Integer tensor-core launch.  One stream-ordered scratch buffer per call
-  // (packed planes, scales and flag, partial tiles); nothing is kept from one
-  // call to the next.  Without memory for it the DMMA launch runs instead.
+  static constexpr int64_t kI8ScratchKeep = 2LL << 30;
+  // Integer tensor-core launch.  One scratch buffer (packed planes, scales and
+  // flag, partial tiles), written anew by every call.  Without memory for it the DMMA launch runs instead.
   void run_i8(Ctx* ctx, const double* X, const double* Y, double* C) const {
     std::memcpy(ctx->gemm_desc, desc, sizeof(desc));
     auto up = [](int64_t v) { return (v + 1023) / 1024 * 1024; };
     const int64_t sc_off = up(pack_a_bytes + pack_b_bytes), sc_bytes = up((nscale + 1) * 4),
                   part_off = sc_off + sc_bytes, total = part_off + nparts * kI8PartElems * 8;
-    DevBuf scratch;
-    try {
-      scratch = DevBuf(ctx, total);
-    } catch (const Error& e) {
-      if (e.code != SB_ERR_OOM) throw;
-    }
+    // Up to 2 GB it stays with the context: out of the stream-ordered pool it came
+    // back as the next call's tensors and the pool grew, 5 to 1000 ms at a time.
+    DevBuf own;
+    DevBuf& scratch = total > kI8ScratchKeep || ctx->capturing ? own : ctx->i8_scratch;
+    if (scratch.bytes() < static_cast<size_t>(total)) try {
+        scratch.reset();
+        scratch = DevBuf(ctx, total);
+      } catch (const Error& e) {
+        if (e.code != SB_ERR_OOM) throw;
+      }
     if (!scratch.raw()) {
       ProfScope ps(ctx, PROF_GEMM, flops, bytes);
       SB_CK(launch_gemm_f64_fallback(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), nf, xT, yT, nullptr,
@@ -864,13 +868,14 @@ struct GemmPlan {
     int32_t kmax = 0;
     for (const GemmPair& q : pairs) kmax = std::max(kmax, q.K);
     const int32_t strip = kmax <= kI8StripK ? kmax : 0;
-    std::vector<I8Image> ia, ib;
+    std::vector<I8Block> ia, ib;
+    int64_t na = 0, nb = 0;  // their image entries
     struct Seen { int64_t base, scale; };
     struct Seg { int64_t off, ld, rows; };  // a block of the stack
     std::map<std::vector<int64_t>, Seen> sa, sb;
     int64_t total = 0, nscale = 0, elems_a = 0, elems_b = 0;
     std::vector<int64_t> key;
-    auto add = [&](std::map<std::vector<int64_t>, Seen>& seen, std::vector<I8Image>& out, int64_t& elems,
+    auto add = [&](std::map<std::vector<int64_t>, Seen>& seen, std::vector<I8Block>& out, int64_t& n, int64_t& elems,
                    const std::vector<Seg>& segs, int64_t K, int64_t tile, bool kc) -> Seen {
       key.assign(1, K);
       for (const Seg& q : segs) {
@@ -881,54 +886,16 @@ struct GemmPlan {
       auto it = seen.find(key);
       if (it != seen.end()) return it->second;
       const Seen s{total, nscale};
-      int64_t rows = 0;
+      int64_t rows = 0, at = 0;
       for (const Seg& q : segs) rows += q.rows;
-      size_t si = 0;
-      int64_t sr = 0;  // block and row in it that the tile starts with
-      if (strip > 0) {
-        const int64_t image = up(K, 64) * 7 * tile;  // bytes of a row tile
-        for (int64_t r = 0; r < rows;) {
-          const Seg& q = segs[si];
-          const int64_t at = r % tile, n = std::min({q.rows - sr, 16 - at % 16, tile - at});
-          out.push_back(I8Image{q.off + (kc ? sr * q.ld : sr), q.ld, total + r / tile * image,
-                                static_cast<int32_t>(nscale + r), static_cast<int32_t>(at), static_cast<int32_t>(n),
-                                static_cast<int32_t>(r + n == rows ? tile : at + n), static_cast<int32_t>(tile),
-                                static_cast<int32_t>(K), kc ? 1 : 0, 0});
-          r += n;
-          if ((sr += n) == q.rows) {
-            ++si;
-            sr = 0;
-          }
-        }
-        total += (rows + tile - 1) / tile * image;
+      for (const Seg& q : segs) {
+        out.push_back(I8Block{q.off, q.ld, total, static_cast<int32_t>(nscale), static_cast<int32_t>(at),
+                              static_cast<int32_t>(q.rows), static_cast<int32_t>(rows), static_cast<int32_t>(tile),
+                              static_cast<int32_t>(K), kc ? 1 : 0, strip > 0 ? 1 : 0, static_cast<int32_t>(n), 0});
+        n += i8_entries(out.back());
+        at += q.rows;
       }
-      for (int64_t r0 = 0; strip == 0 && r0 < rows; r0 += tile) {
-        const int64_t r1 = std::min(rows, r0 + tile);
-        for (int64_t k0 = 0; k0 < K; k0 += 64) {
-          size_t i = si;
-          int64_t at = sr;
-          for (int64_t r = r0; r < r1;) {
-            const Seg& q = segs[i];
-            const int64_t n = std::min(q.rows - at, r1 - r);
-            out.push_back(I8Image{q.off + (kc ? at * q.ld + k0 : at + k0 * q.ld), q.ld, total,
-                                  static_cast<int32_t>(nscale + r), static_cast<int32_t>(r - r0),
-                                  static_cast<int32_t>(n), static_cast<int32_t>(r + n == rows ? tile : r - r0 + n),
-                                  static_cast<int32_t>(tile), static_cast<int32_t>(std::min<int64_t>(64, K - k0)),
-                                  kc ? 1 : 0, 0});
-            r += n;
-            at += n;
-            if (at == q.rows) {
-              ++i;
-              at = 0;
-            }
-          }
-          total += 7 * tile * 64;
-          if (k0 + 64 >= K) {
-            si = i;
-            sr = at;
-          }
-        }
-      }
+      total += (rows + tile - 1) / tile * up(K, 64) * 7 * tile;
       elems += rows * K;
       nscale += rows;
       seen.emplace(key, s);
@@ -943,20 +910,20 @@ struct GemmPlan {
           segs.push_back(Seg{q.x_off, q.ldx, cbs[m].M});
         }
         const int64_t K = pairs[cbs[gr.members[0]].pair_begin + j].K;
-        const Seen a = add(sa, ia, elems_a, segs, K, 128, akc);
+        const Seen a = add(sa, ia, na, elems_a, segs, K, 128, akc);
         pk[gr.p0 + j] = I8Pack{a.base, 0, static_cast<int32_t>(a.scale), 0, static_cast<int32_t>((K + 63) / 64),
                                static_cast<int32_t>(width(cbs[gr.members[0]].N))};
-        if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
+        if (nscale >= (1LL << 31) || total > (16LL << 30) || na + nb >= (1LL << 30)) return false;
       }
     for (const Grp& gr : grp)
       for (int j = 0; j < gr.npairs; ++j) {
         const GemmCBlock& c0 = cbs[gr.members[0]];
         const GemmPair& q = pairs[c0.pair_begin + j];
         segs.assign(1, Seg{q.y_off, q.ldy, c0.N});
-        const Seen b = add(sb, ib, elems_b, segs, q.K, width(c0.N), bkc);
+        const Seen b = add(sb, ib, nb, elems_b, segs, q.K, width(c0.N), bkc);
         pk[gr.p0 + j].b_base = b.base;
         pk[gr.p0 + j].b_sc = static_cast<int32_t>(b.scale);
-        if (nscale >= (1LL << 31) || total > (16LL << 30)) return false;
+        if (nscale >= (1LL << 31) || total > (16LL << 30) || na + nb >= (1LL << 30)) return false;
       }
     const double pack = (strip > 0 ? 8.0 : 16.0) * (elems_a + elems_b) + total;
     const double t_i8 = cycles / sms / 1.85e9 + pack / 4.5e12 + 30e-6;
@@ -967,7 +934,7 @@ struct GemmPlan {
     int64_t seg = 0;
     if (static_cast<int64_t>(geo.size()) < target && total_kt > 0)
       seg = std::max<int64_t>(12, (total_kt + target - 1) / target);
-    struct W { TcTile t; double work; int64_t group; };
+    struct W { TcTile t; double work; int64_t group; double sum; };
     std::vector<W> items;
     std::vector<TcSplit> splits;
     int32_t nparts = 0;
@@ -980,14 +947,18 @@ struct GemmPlan {
         const int64_t kb = kt * q / nseg, ke = kt * (q + 1) / nseg;
         items.push_back(W{TcTile{t.c, t.a0, t.b0, t.nb, p, k0, static_cast<int32_t>(ke - kb),
                                  nseg > 1 ? nparts + static_cast<int32_t>(q) : -1},
-                          (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q});
-        for (int64_t i = kb; i < ke; ++i) {
-          k0 += 64;
-          if (++kp >= pk[p].nkt) {
+                          (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q,
+                          0.0});
+        if (q + 1 == nseg) break;
+        for (int64_t left = ke - kb; left > 0;) {  // on to the next segment's first k-tile
+          const int n = static_cast<int>(std::min<int64_t>(left, pk[p].nkt - kp));
+          left -= n;
+          if ((kp += n) >= pk[p].nkt) {
             ++p;
-            k0 = kp = 0;
+            kp = 0;
           }
         }
+        k0 = 64 * kp;
       }
       if (nseg > 1) nparts += static_cast<int32_t>(nseg);
     }
@@ -995,9 +966,9 @@ struct GemmPlan {
     // they read the same images
     std::unordered_map<int64_t, double> gwork;
     for (const W& w : items) gwork[w.group] += w.work;
-    std::stable_sort(items.begin(), items.end(), [&](const W& a, const W& b) {
-      const double wa = gwork[a.group], wb = gwork[b.group];
-      return wa != wb ? wa > wb : a.group < b.group;
+    for (W& w : items) w.sum = gwork[w.group];
+    std::stable_sort(items.begin(), items.end(), [](const W& a, const W& b) {
+      return a.sum != b.sum ? a.sum > b.sum : a.group < b.group;
     });
     // each item to the CTA with the least work so far: in this order neighbours
     // still run at about the same time, and the sums even out (the stride walk
@@ -1032,30 +1003,53 @@ struct GemmPlan {
     g.dfirst = upload(ctx, first);
     g.nctas = nctas;
     std::vector<I8Group> dg;
-    std::vector<int64_t> row_off;
-    std::vector<int32_t> row_ld;
-    row_off.reserve(nrows);
-    row_ld.reserve(nrows);
+    std::vector<I8RowRun> runs;
     for (const Grp& gr : grp) {
       dg.push_back(I8Group{static_cast<int32_t>(gr.rows), cbs[gr.members[0]].N, gr.row0, 0});
-      for (int m : gr.members)
-        for (int32_t r = 0; r < cbs[m].M; ++r) {
-          row_off.push_back(cbs[m].c_off + r);
-          row_ld.push_back(cbs[m].ldc);
-        }
+      int32_t r = gr.row0;
+      for (int m : gr.members) {
+        runs.push_back(I8RowRun{cbs[m].c_off, cbs[m].ldc, cbs[m].M, r, 0});
+        r += cbs[m].M;
+      }
     }
     g.dgroup = upload(ctx, dg);
-    g.drow_off = upload(ctx, row_off);
-    g.drow_ld = upload(ctx, row_ld);
     g.dc = upload(ctx, cbs);
     g.dp = upload(ctx, pairs);
     g.dt = upload(ctx, tiles);
     g.dsplit = upload(ctx, splits);
     g.dpk = upload(ctx, pk);
-    g.dimg_a = upload(ctx, ia);
-    g.dimg_b = upload(ctx, ib);
-    g.nimg_a = static_cast<int64_t>(ia.size());
-    g.nimg_b = static_cast<int64_t>(ib.size());
+    g.nimg_a = na;
+    g.nimg_b = nb;
+    if (ctx->capturing) {  // before any replay, not in every one
+      auto images = [](const std::vector<I8Block>& blocks) {
+        std::vector<I8Image> v;
+        for (const I8Block& b : blocks)
+          for (int32_t p = 0, n = i8_entries(b); p < n; ++p) v.push_back(i8_entry(b, p));
+        return v;
+      };
+      g.dimg_a = upload(ctx, images(ia));
+      g.dimg_b = upload(ctx, images(ib));
+      std::vector<int64_t> row_off;
+      std::vector<int32_t> row_ld;
+      for (const I8RowRun& q : runs)
+        for (int32_t r = 0; r < q.M; ++r) {
+          row_off.push_back(q.c_off + r);
+          row_ld.push_back(q.ldc);
+        }
+      g.drow_off = upload(ctx, row_off);
+      g.drow_ld = upload(ctx, row_ld);
+    } else {
+      g.dimg_a = DevBuf(ctx, na * sizeof(I8Image));
+      g.dimg_b = DevBuf(ctx, nb * sizeof(I8Image));
+      g.drow_off = DevBuf(ctx, nrows * sizeof(int64_t));
+      g.drow_ld = DevBuf(ctx, nrows * sizeof(int32_t));
+      const DevBuf da = upload(ctx, ia), db = upload(ctx, ib), dr = upload(ctx, runs);
+      SB_CK(launch_i8_entries(da.as<I8Block>(), static_cast<int64_t>(ia.size()), g.dimg_a.as<I8Image>(), ctx->stream));
+      SB_CK(launch_i8_entries(db.as<I8Block>(), static_cast<int64_t>(ib.size()), g.dimg_b.as<I8Image>(), ctx->stream));
+      SB_CK(launch_i8_rows(dr.as<I8RowRun>(), static_cast<int64_t>(runs.size()), g.drow_off.as<int64_t>(),
+                           g.drow_ld.as<int32_t>(), ctx->stream));
+      ctx->note_launch(3);
+    }
     g.pack_a_bytes = total;
     g.pack_a_elems = elems_a;
     g.pack_b_elems = elems_b;

@@ -597,7 +597,38 @@ __global__ void __launch_bounds__(256) k_i8_reduce(const double* __restrict__ pa
   }
 }
 
+// One CTA per block / run; latency-bound, a few microseconds once per plan.
+__global__ void __launch_bounds__(256) k_i8_entries(const I8Block* __restrict__ blocks, I8Image* __restrict__ imgs) {
+  const I8Block b = blocks[blockIdx.x];
+  const int n = i8_entries(b);
+  for (int p = static_cast<int>(threadIdx.x); p < n; p += 256) imgs[b.first + p] = i8_entry(b, p);
+}
+
+__global__ void __launch_bounds__(256) k_i8_rows(const I8RowRun* __restrict__ runs, int64_t* __restrict__ row_off,
+                                                 int32_t* __restrict__ row_ld) {
+  const I8RowRun q = runs[blockIdx.x];
+  for (int r = static_cast<int>(threadIdx.x); r < q.M; r += 256) {
+    row_off[q.row0 + r] = q.c_off + r;
+    row_ld[q.row0 + r] = q.ldc;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_i8_entries(const I8Block* d_blocks, int64_t nblocks, I8Image* d_imgs, cudaStream_t s) {
+  if (nblocks <= 0) return cudaSuccess;
+  if (nblocks > 0x7fffffffLL) return cudaErrorInvalidValue;
+  k_i8_entries<<<static_cast<unsigned>(nblocks), 256, 0, s>>>(d_blocks, d_imgs);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_i8_rows(const I8RowRun* d_runs, int64_t nruns, int64_t* d_row_off, int32_t* d_row_ld,
+                           cudaStream_t s) {
+  if (nruns <= 0) return cudaSuccess;
+  if (nruns > 0x7fffffffLL) return cudaErrorInvalidValue;
+  k_i8_rows<<<static_cast<unsigned>(nruns), 256, 0, s>>>(d_runs, d_row_off, d_row_ld);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, int32_t strip_k, uint32_t* d_rowhi,
                            void* dst, int* d_flag, cudaStream_t s) {

@@ -124,6 +124,10 @@ struct Ctx {
   // result to.  Every call ends with a synchronisation, so one of each serves
   // the context's calls in turn.
   DevBuf dot_scratch;
+  // Workspace of the integer GEMM (at most kI8ScratchKeep bytes), kept between
+  // calls: used in stream order by one call at a time, given back when another
+  // allocation finds no memory and with the context.
+  DevBuf i8_scratch;
   double* host_scalar = nullptr;
   bool tc_launched = false;  // a tensor-core GEMM ran since the status was last read
   // Plan cache of the BS x BS contract_shared! path (sb_contract.cpp): the

@@ -176,6 +176,49 @@ struct I8Image {
   int32_t scale, row0, rows, row_end, rows_img, kv, kc, pad;
 };
 constexpr int32_t kI8StripK = 768;  // 16 rows of 768: two CTAs per SM
+// An operand block in its stack of rows: element (r, k) at src + r*ld + k when
+// kc, else src + r + k*ld; stack rows [at, at + rows) of total; the stack's
+// images from byte dst, its scales from index scale; the block's entries of the
+// image list begin at first.
+struct I8Block {
+  int64_t src, ld, dst;
+  int32_t scale, at, rows, total, tile, K, kc, strip, first, pad;
+};
+// Entries of a block, and its p-th: strips in row order, k-tiles row tile by row
+// tile.  Lists are written on the device, 56 bytes an entry from one block
+// descriptor: at chi = 2048 R*T3 has 14000 and their upload cost milliseconds.
+__host__ __device__ inline int32_t i8_entries(const I8Block& b) {
+  if (b.rows <= 0) return 0;
+  const int32_t unit = b.strip ? 16 : b.tile;
+  return ((b.at + b.rows - 1) / unit - b.at / unit + 1) * (b.strip ? 1 : (b.K + 63) / 64);
+}
+__host__ __device__ inline I8Image i8_entry(const I8Block& b, int32_t p) {
+  const int32_t nkt = (b.K + 63) / 64, unit = b.strip ? 16 : b.tile, per = b.strip ? 1 : nkt;
+  const int32_t u0 = (b.at / unit + p / per) * unit, kt = p % per;
+  const int32_t lo = b.at > u0 ? b.at : u0, hi = b.at + b.rows < u0 + unit ? b.at + b.rows : u0 + unit;
+  const int32_t t = lo / b.tile, r = lo - t * b.tile, left = b.K - 64 * kt;
+  const int64_t dr = lo - b.at, dk = 64 * kt;
+  return I8Image{b.src + (b.kc ? dr * b.ld + dk : dr + dk * b.ld),
+                 b.ld,
+                 b.dst + (static_cast<int64_t>(t) * nkt + kt) * 7 * 64 * b.tile,
+                 b.scale + lo,
+                 r,
+                 hi - lo,
+                 hi == b.total ? b.tile : r + hi - lo,
+                 b.tile,
+                 b.strip ? b.K : left < 64 ? left : 64,
+                 b.kc,
+                 0};
+}
+cudaError_t launch_i8_entries(const I8Block* d_blocks, int64_t nblocks, I8Image* d_imgs, cudaStream_t s);
+// Row tables of launch_gemm_i8 from the C blocks: rows [row0, row0 + M) are
+// C's at c_off, column stride ldc.
+struct I8RowRun {
+  int64_t c_off;
+  int32_t ldc, M, row0, pad;
+};
+cudaError_t launch_i8_rows(const I8RowRun* d_runs, int64_t nruns, int64_t* d_row_off, int32_t* d_row_ld,
+                           cudaStream_t s);
 cudaError_t launch_i8_pack(const double* src, const I8Image* d_imgs, int64_t nimg, int32_t strip_k, uint32_t* d_rowhi,
                            void* dst, int* d_flag, cudaStream_t s);
 // Per pair: byte offsets of the images of its X block (row tiles of 128, nkt

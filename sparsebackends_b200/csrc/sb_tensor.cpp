@@ -34,10 +34,10 @@ void Ctx::stage_copy(void* dst, const void* src, size_t bytes) {
   }
   if (!s.ev) SB_CK(cudaEventCreateWithFlags(&s.ev, cudaEventDisableTiming));
   if (s.cap < bytes) {
+    const size_t cap = std::max<size_t>(bytes, std::max<size_t>(64 << 10, 2 * s.cap));
     if (s.host) SB_CK(cudaFreeHost(s.host));
     s.host = nullptr;
     s.cap = 0;
-    const size_t cap = std::max<size_t>(bytes, std::max<size_t>(64 << 10, 2 * s.cap));
     SB_CK(cudaHostAlloc(&s.host, cap, cudaHostAllocDefault));
     s.cap = cap;
   }
@@ -89,7 +89,13 @@ DevBuf::DevBuf(Ctx* ctx, size_t bytes) : ctx_(ctx), n_(bytes) {
     SB_CK(cudaMalloc(&p_, bytes));
     plain_ = true;
   } else {
-    SB_CK(cudaMallocAsync(&p_, bytes, ctx->stream));
+    cudaError_t e = cudaMallocAsync(&p_, bytes, ctx->stream);
+    if (e == cudaErrorMemoryAllocation && ctx->i8_scratch.raw()) {  // give the kept workspace back
+      cudaGetLastError();
+      ctx->i8_scratch.reset();
+      e = cudaMallocAsync(&p_, bytes, ctx->stream);
+    }
+    SB_CK(e);
   }
 }
 DevBuf::~DevBuf() { reset(); }

@@ -197,3 +197,16 @@ def test_rows_stacked_over_output_blocks(ms, order):
         want = (a.astype(np.longdouble) @ b.astype(np.longdouble)).astype(float)
         scale = np.outer(np.sqrt((a ** 2).sum(1)), np.sqrt((b ** 2).sum(0)))
         assert np.max(np.abs(c - want) / scale) <= 8 * 2.0 ** -55, (i, j)
+
+
+def test_workspace_across_structures():
+    """The kept workspace grows, shrinks in use and serves other structures; every
+    result equals a fresh context's."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(5))
+    env = dict(SPARSEB_GEMM_I8=1, SPARSEB_GEMM_THIN=0, SPARSEB_POISON_OUTPUT=1)
+    ctx = _ctx(sb, **env)
+    for m, n, ks in [(40, 50, (70,)), (300, 260, (900, 65)), (33, 16, (20,)), (300, 260, (900, 65)), (301, 17, (64,))]:
+        A, B = _blocks(rng, m, n, ks)
+        got, want = _run(sb, ctx, A, B, "AB"), _run(sb, _ctx(sb, **env), A, B, "AB")
+        assert np.array_equal(got[1, 1], want[1, 1])
