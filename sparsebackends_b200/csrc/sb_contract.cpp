@@ -858,6 +858,8 @@ struct GemmPlan {
     }
     for (auto& c : cbs) nf += ((static_cast<int64_t>(c.M) + 63) / 64) * ((static_cast<int64_t>(c.N) + 63) / 64);
     if (nf >= (1LL << 31) || geo.size() >= (1ULL << 30)) return false;
+    const double t_mma = cycles / sms / 1.85e9 + 30e-6, t_f64 = flops / 27e12 + 5e-6;
+    if (ctx->gemm_i8 < 0 && t_mma > 0.95 * t_f64) return false;  // before any packing
     // packed images: every distinct Y block and every distinct stack of X blocks
     // once (finding the scales and packing 40 or 160 MB at a time, so that the
     // second read hits L2, was slower: 565 and 474 us against 402 for R*T3)
@@ -926,16 +928,16 @@ struct GemmPlan {
         if (nscale >= (1LL << 31) || total > (16LL << 30) || na + nb >= (1LL << 30)) return false;
       }
     const double pack = (strip > 0 ? 8.0 : 16.0) * (elems_a + elems_b) + total;
-    const double t_i8 = cycles / sms / 1.85e9 + pack / 4.5e12 + 30e-6;
-    const double t_f64 = flops / 27e12 + 5e-6;
+    const double t_i8 = t_mma + pack / 4.5e12;
     if (ctx->gemm_i8 < 0 && t_i8 > 0.95 * t_f64) return false;
     // k-segments when the tiles are fewer than four per SM, as in prepare_tc
     const int64_t target = 4LL * sms;
     int64_t seg = 0;
     if (static_cast<int64_t>(geo.size()) < target && total_kt > 0)
       seg = std::max<int64_t>(12, (total_kt + target - 1) / target);
-    struct W { TcTile t; double work; int64_t group; double sum; };
+    struct W { TcTile t; double work; int64_t group; };
     std::vector<W> items;
+    items.reserve(geo.size());
     std::vector<TcSplit> splits;
     int32_t nparts = 0;
     for (const Geo& t : geo) {
@@ -947,8 +949,7 @@ struct GemmPlan {
         const int64_t kb = kt * q / nseg, ke = kt * (q + 1) / nseg;
         items.push_back(W{TcTile{t.c, t.a0, t.b0, t.nb, p, k0, static_cast<int32_t>(ke - kb),
                                  nseg > 1 ? nparts + static_cast<int32_t>(q) : -1},
-                          (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q,
-                          0.0});
+                          (ke - kb) * mma_cycles(t.nb) + drain_cycles(t.nb), (static_cast<int64_t>(t.c) << 32) | q});
         if (q + 1 == nseg) break;
         for (int64_t left = ke - kb; left > 0;) {  // on to the next segment's first k-tile
           const int n = static_cast<int>(std::min<int64_t>(left, pk[p].nkt - kp));
@@ -963,32 +964,65 @@ struct GemmPlan {
       if (nseg > 1) nparts += static_cast<int32_t>(nseg);
     }
     // heaviest groups (C block, k-segment) first, a group's items together:
-    // they read the same images
-    std::unordered_map<int64_t, double> gwork;
-    for (const W& w : items) gwork[w.group] += w.work;
-    for (W& w : items) w.sum = gwork[w.group];
-    std::stable_sort(items.begin(), items.end(), [](const W& a, const W& b) {
-      return a.sum != b.sum ? a.sum > b.sum : a.group < b.group;
-    });
+    // they read the same images (buckets and one sift per item: sorting the
+    // items and a priority queue took 0.8 ms at chi = 2048)
+    struct G { double sum; int64_t group; int32_t n, at; };
+    std::vector<G> groups;
+    std::vector<int32_t> group_of(items.size()), rank;
+    {
+      std::unordered_map<int64_t, int32_t> index;
+      for (size_t i = 0; i < items.size(); ++i) {
+        const int32_t last = i > 0 ? group_of[i - 1] : -1;
+        if (last >= 0 && groups[last].group == items[i].group) {
+          group_of[i] = last;
+        } else {
+          const auto it = index.emplace(items[i].group, static_cast<int32_t>(groups.size()));
+          if (it.second) groups.push_back(G{0.0, items[i].group, 0, 0});
+          group_of[i] = it.first->second;
+        }
+        groups[group_of[i]].sum += items[i].work;
+        ++groups[group_of[i]].n;
+      }
+      rank.resize(groups.size());
+      std::iota(rank.begin(), rank.end(), 0);
+      std::sort(rank.begin(), rank.end(), [&](int32_t p, int32_t q) {
+        return groups[p].sum != groups[q].sum ? groups[p].sum > groups[q].sum : groups[p].group < groups[q].group;
+      });
+      int32_t at = 0;
+      for (int32_t r : rank) {
+        groups[r].at = at;
+        at += groups[r].n;
+      }
+    }
+    std::vector<int32_t> order(items.size());
+    for (size_t i = 0; i < items.size(); ++i) order[groups[group_of[i]].at++] = static_cast<int32_t>(i);
     // each item to the CTA with the least work so far: in this order neighbours
     // still run at about the same time, and the sums even out (the stride walk
     // left R*T3 at chi = 2048 with 51% to 77% busy tensor cores)
     const int32_t nctas = static_cast<int32_t>(std::max<size_t>(1, std::min<size_t>(sms, items.size())));
-    std::vector<std::vector<TcTile>> mine(nctas);
-    std::priority_queue<std::pair<double, int32_t>, std::vector<std::pair<double, int32_t>>, std::greater<>> least;
-    for (int32_t i = 0; i < nctas; ++i) least.emplace(0.0, i);
-    for (auto& w : items) {
-      auto [load, i] = least.top();
-      least.pop();
-      mine[i].push_back(w.t);
-      least.emplace(load + w.work, i);
+    std::vector<std::pair<double, int32_t>> least(nctas);  // min-heap
+    for (int32_t i = 0; i < nctas; ++i) least[i] = {0.0, i};
+    std::vector<int32_t> cta(items.size()), first(nctas + 1, 0);
+    for (size_t i = 0; i < order.size(); ++i) {
+      std::pair<double, int32_t> e = least[0];
+      cta[i] = e.second;
+      ++first[e.second + 1];
+      e.first += items[order[i]].work;
+      int32_t h = 0;
+      for (int32_t k = 1; k < nctas; k = 2 * h + 1) {
+        if (k + 1 < nctas && least[k + 1] < least[k]) ++k;
+        if (!(least[k] < e)) break;
+        least[h] = least[k];
+        h = k;
+      }
+      least[h] = e;
     }
-    std::vector<TcTile> tiles;
-    std::vector<int32_t> first(nctas + 1, 0);
+    for (int32_t i = 0; i < nctas; ++i) first[i + 1] += first[i];
+    std::vector<TcTile> tiles(items.size());
     tiles.reserve(items.size() + zero.size());
-    for (int32_t i = 0; i < nctas; ++i) {
-      tiles.insert(tiles.end(), mine[i].begin(), mine[i].end());
-      first[i + 1] = static_cast<int32_t>(tiles.size());
+    {
+      std::vector<int32_t> at(first.begin(), first.end() - 1);
+      for (size_t i = 0; i < order.size(); ++i) tiles[at[cta[i]]++] = items[order[i]].t;
     }
     for (auto& t : zero) tiles.push_back(TcTile{t.c, t.a0, t.b0, t.nb, 0, 0, 0, -1});
     require(tiles.size() < (1ULL << 31), SB_ERR_INVALID_ARG, "too many GEMM tiles in one launch");
