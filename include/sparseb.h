@@ -22,7 +22,9 @@
  * Threading: one sb_ctx per host thread.  Every call enqueues device work on
  * the context's stream; calls that must read device-computed structure flags
  * (value-dependent block creation) synchronise that stream internally.
- * No function allocates pinned host memory or blocks on other streams.
+ * A context keeps small pinned buffers (plan uploads, one scalar) and, after
+ * large FP64 block GEMMs, up to 2 GB of device workspace, which it gives back
+ * when an allocation finds no memory.  No function blocks on other streams.
  */
 #ifndef SPARSEB_H
 #define SPARSEB_H
