@@ -33,6 +33,13 @@ struct Seg {
 
 // Merge contiguous segments, cut into chunks, reduce on the device.
 double run_dot(Ctx* ctx, const double* X, const double* Y, const double* S, std::vector<Seg> segs) {
+  if (ctx->capturing) {
+    // The synchronisation fails and abandons the capture, as for every host
+    // read-back.  Before anything that outlives the call is made: in a capture
+    // the counter's memset below would be recorded and never run.
+    ctx->sync();
+    fail(SB_ERR_INVALID_ARG, "norm and dot read a value back and cannot be captured");
+  }
   std::vector<Seg> merged;
   merged.reserve(segs.size());
   for (const Seg& s : segs) {
@@ -63,8 +70,9 @@ double run_dot(Ctx* ctx, const double* X, const double* Y, const double* S, std:
   // longest vector (8 bytes per 1024 elements)
   const size_t need = static_cast<size_t>(nchunks) * sizeof(double) + 16;
   if (ctx->dot_scratch.bytes() < need) {
-    ctx->dot_scratch = DevBuf(ctx, std::max<size_t>(need, 2 * ctx->dot_scratch.bytes()));
-    SB_CK(cudaMemsetAsync(ctx->dot_scratch.raw(), 0, 16, ctx->stream));
+    DevBuf grown(ctx, std::max<size_t>(need, 2 * ctx->dot_scratch.bytes()));
+    SB_CK(cudaMemsetAsync(grown.raw(), 0, 16, ctx->stream));
+    ctx->dot_scratch = std::move(grown);
   }
   if (!ctx->host_scalar) SB_CK(cudaHostAlloc(&ctx->host_scalar, sizeof(double), cudaHostAllocMapped));
   double* out = nullptr;
