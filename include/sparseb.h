@@ -22,9 +22,10 @@
  * Threading: one sb_ctx per host thread.  Every call enqueues device work on
  * the context's stream; calls that must read device-computed structure flags
  * (value-dependent block creation) synchronise that stream internally.
- * A context keeps small pinned buffers (plan uploads, one scalar) and, after
- * large FP64 block GEMMs, up to 2 GB of device workspace, which it gives back
- * when an allocation finds no memory.  No function blocks on other streams.
+ * A context keeps small pinned buffers (plan uploads, one scalar) and, in
+ * SB_PRECISION_F64_I8 after large block GEMMs, up to 2 GB of device workspace,
+ * which it gives back when an allocation finds no memory.  No function blocks
+ * on other streams.
  */
 #ifndef SPARSEB_H
 #define SPARSEB_H
@@ -82,11 +83,18 @@ SB_API int64_t sb_ctx_launch_count(const sb_ctx* ctx);
  * ta/contract_bs_bs.jl:716-723 and ta/contract_bs_dense.jl:576-611, which the
  * reference runs in FP64).  Tensors stay FP64 unless created with
  * sb_tensor_create_bs_f32.
- *   SB_PRECISION_F64    FP64, the drop-in (default): DMMA tensor cores, and for
- *                       large launches exact 8-bit integer products on the
- *                       tcgen05 tensor cores (operands to 55 bits of each
- *                       row's and column's largest magnitude; rows beyond
- *                       2^+-400, infinities and NaN go to DMMA);
+ *   SB_PRECISION_F64    FP64, the drop-in (default): DMMA tensor cores;
+ *   SB_PRECISION_F64_I8 FP64 with norm-wise accuracy: large launches of FP64
+ *                       tensors run as exact 8-bit integer products on the
+ *                       tcgen05 tensor cores when that is estimated to be
+ *                       faster, the others as in SB_PRECISION_F64.  Each
+ *                       element of a block row of A and column of B is then
+ *                       held to 55 bits below the row's or column's largest
+ *                       magnitude, not to 53 bits of its own, so the error of
+ *                       an output is bounded against |row| |column| and no
+ *                       longer against sum_k |a_k| |b_k|: a small output next
+ *                       to large, unmatched entries loses its digits.  Rows
+ *                       beyond 2^+-400, infinities and NaN go to DMMA;
  *   SB_PRECISION_TF32X3 tcgen05 tensor cores: every operand value rounded
  *                       to FP32 and split into TF32 hi + lo, the three
  *                       significant products accumulated in FP32 chunks of
@@ -94,7 +102,8 @@ SB_API int64_t sb_ctx_launch_count(const sb_ctx* ctx);
  *                       a few 1e-6 relative per block);
  *   SB_PRECISION_TF32   tcgen05, one TF32 product (about 3e-4 relative).
  * Only the tiled GEMMs change; the K <= 16 (MPO) steps, outer products,
- * Kahan sums and axpys compute in FP64.  Operands must lie in FP32's range.
+ * Kahan sums and axpys compute in FP64.  In the TF32 precisions operands must
+ * lie in FP32's range.
  * The split operand images of a contraction are kept with its plan and
  * remade after the library writes the operand tensor or hands out its device
  * pointer (sb_tensor_device_data); inside a captured graph they are remade on
@@ -104,7 +113,8 @@ SB_API int64_t sb_ctx_launch_count(const sb_ctx* ctx);
 typedef enum sb_precision {
   SB_PRECISION_F64 = 0,
   SB_PRECISION_TF32X3 = 1,
-  SB_PRECISION_TF32 = 2
+  SB_PRECISION_TF32 = 2,
+  SB_PRECISION_F64_I8 = 3
 } sb_precision;
 SB_API sb_status sb_ctx_set_precision(sb_ctx* ctx, int precision);
 SB_API int sb_ctx_get_precision(const sb_ctx* ctx);

@@ -133,12 +133,14 @@ class Context:
     PROFILE_KINDS = {"gemm": 0, "permute": 1, "outer": 2, "axpy": 3, "other": 4, "vector": 5, "gemm_thin": 6,
                      "gemm_tc": 7, "tc_pack": 8}
 
-    PRECISIONS = {"f64": 0, "tf32x3": 1, "tf32": 2}
+    PRECISIONS = {"f64": 0, "tf32x3": 1, "tf32": 2, "f64i8": 3}
 
     @property
     def precision(self) -> str:
         """Arithmetic of the tiled block GEMMs: "f64" (default, the drop-in),
-        "tf32x3" (tcgen05, operands split into TF32 hi + lo) or "tf32"."""
+        "tf32x3" (tcgen05, operands split into TF32 hi + lo), "tf32", or "f64i8"
+        (FP64 of norm-wise accuracy: large launches as exact 8-bit integer
+        products, errors bounded against |row| |column|)."""
         v = int(self._lib.sb_ctx_get_precision(self._h))
         return {b: a for a, b in self.PRECISIONS.items()}[v]
 

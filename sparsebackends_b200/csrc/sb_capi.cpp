@@ -181,11 +181,12 @@ sb_status sb_ctx_synchronize(sb_ctx* ctx) {
 sb_status sb_ctx_set_precision(sb_ctx* ctx, int precision) {
   return guard(ctx, [&] {
     check_ctx(ctx);
-    require(precision == SB_PRECISION_F64 || precision == SB_PRECISION_TF32X3 || precision == SB_PRECISION_TF32,
+    require(precision == SB_PRECISION_F64 || precision == SB_PRECISION_TF32X3 || precision == SB_PRECISION_TF32 ||
+                precision == SB_PRECISION_F64_I8,
             SB_ERR_INVALID_ARG, "unknown precision");
     require(!ctx->impl.capturing, SB_ERR_INVALID_ARG, "precision cannot change while a capture is open");
     SB_CK(cudaSetDevice(ctx->impl.device));
-    if (precision != SB_PRECISION_F64 && !ctx->impl.tc_status.raw()) {
+    if (sb::is_tf32(precision) && !ctx->impl.tc_status.raw()) {
       ctx->impl.tc_status = sb::DevBuf(&ctx->impl, sizeof(int));
       SB_CK(cudaMemsetAsync(ctx->impl.tc_status.raw(), 0, sizeof(int), ctx->impl.stream));
     }

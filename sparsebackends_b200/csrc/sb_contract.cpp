@@ -540,7 +540,7 @@ struct GemmPlan {
       g.bytes = bytes;
       return g;
     }
-    if (ctx->precision != SB_PRECISION_F64) {
+    if (is_tf32(ctx->precision)) {
       prepare_tc(ctx, g, flops, bytes);
       return g;
     }
@@ -779,17 +779,21 @@ struct GemmPlan {
   // pairs of a link pair), so that rows pad to 128 once per stack: 14 to 20%
   // fewer clocks at chi = 2048 and 700.  Tiles of 128 rows by nbs columns of Y
   // (as few tiles of at most 128 columns as cover the block, of equal width
-  // rounded up to 16).  Returns false, leaving the launch to DMMA, unless the
-  // estimated time is below DMMA's.  The estimate: clocks per k-tile and per
-  // drained chunk over the SMs, the packing's bytes and 30 us of launches,
-  // against 27 TFLOP/s.  Measured (H_eff steps, us, with
+  // rounded up to 16).  Only for callers that chose SB_PRECISION_F64_I8: the
+  // operands are rounded to a common scale per row and column, which DMMA does
+  // not do (rows of one entry of 1 and others of 1e-14 against columns that are
+  // zero at the large one: 2.8e9 K 2^-53 sum|x||y| off, DMMA 1.5e-3).  Returns
+  // false, leaving the launch to DMMA, unless the estimated time is below
+  // DMMA's.  The estimate: clocks per k-tile and per drained chunk over the SMs,
+  // the packing's bytes and 30 us of launches, against 27 TFLOP/s.  Measured (H_eff steps, us, with
   // packing): psi*L at chi = 2048 946 against 1831 with DMMA, R*T3 1215 against
   // 1911; chi = 1024 psi*L 225 against 284, R*T3 366 against 318; chi = 700
   // 122 against 109: small blocks pad to 64-deep k-tiles and 16-wide columns,
   // every chunk pays its drain.
   bool prepare_i8(Ctx* ctx, GemmLaunch& g, double flops, double bytes) {
-    if (ctx->gemm_i8 == 0 || ctx->gemm_tile >= 0 || ctx->autotune) return false;
-    if (ctx->gemm_i8 < 0 && flops < 2e8) return false;
+    const bool forced = ctx->gemm_i8 == 1, chosen = ctx->precision == SB_PRECISION_F64_I8;
+    if (ctx->gemm_i8 == 0 || ctx->gemm_tile >= 0 || !(chosen || (forced && !ctx->autotune))) return false;
+    if (!forced && flops < 2e8) return false;
     auto up = [](int64_t v, int64_t m) { return (v + m - 1) / m * m; };
     auto width = [&](int64_t n) {
       const int64_t t = (n + kI8MaxN - 1) / kI8MaxN;
@@ -859,7 +863,7 @@ struct GemmPlan {
     for (auto& c : cbs) nf += ((static_cast<int64_t>(c.M) + 63) / 64) * ((static_cast<int64_t>(c.N) + 63) / 64);
     if (nf >= (1LL << 31) || geo.size() >= (1ULL << 30)) return false;
     const double t_mma = cycles / sms / 1.85e9 + 30e-6, t_f64 = flops / 27e12 + 5e-6;
-    if (ctx->gemm_i8 < 0 && t_mma > 0.95 * t_f64) return false;  // before any packing
+    if (!forced && t_mma > 0.95 * t_f64) return false;  // before any packing
     // packed images: every distinct Y block and every distinct stack of X blocks
     // once (finding the scales and packing 40 or 160 MB at a time, so that the
     // second read hits L2, was slower: 565 and 474 us against 402 for R*T3)
@@ -929,7 +933,7 @@ struct GemmPlan {
       }
     const double pack = (strip > 0 ? 8.0 : 16.0) * (elems_a + elems_b) + total;
     const double t_i8 = t_mma + pack / 4.5e12;
-    if (ctx->gemm_i8 < 0 && t_i8 > 0.95 * t_f64) return false;
+    if (!forced && t_i8 > 0.95 * t_f64) return false;
     // k-segments when the tiles are fewer than four per SM, as in prepare_tc
     const int64_t target = 4LL * sms;
     int64_t seg = 0;

@@ -55,6 +55,9 @@ class DevBuf {
   bool plain_ = false;  // cudaMalloc'd (allocated while a capture was open) instead of stream-ordered
 };
 
+// The precisions of the TF32 block GEMM (launch_gemm_tc).
+inline bool is_tf32(int precision) { return precision == SB_PRECISION_TF32X3 || precision == SB_PRECISION_TF32; }
+
 // Kernel classes reported by the in-library profiler.
 enum ProfKind : int {
   PROF_GEMM = 0, PROF_PERMUTE = 1, PROF_OUTER = 2, PROF_AXPY = 3, PROF_OTHER = 4, PROF_VECTOR = 5,
@@ -94,8 +97,8 @@ struct Ctx {
   // -1 = auto: column / row edges of <= 32 go to 64x32 / 32x64 tiles.
   int gemm_edges = -1;
   // SPARSEB_GEMM_I8=0 keeps FP64 launches on DMMA, =1 takes the integer
-  // tensor-core path for every launch it can serve (tests); -1 = by the
-  // estimated times (prepare_i8).
+  // tensor-core path for every launch it can serve (tests); -1 = in
+  // SB_PRECISION_F64_I8 by the estimated times (prepare_i8), otherwise never.
   int gemm_i8 = -1;
   // SPARSEB_AUTOTUNE=1: the first FP64 tiled block GEMM of a block-shape
   // histogram times the candidate tile shapes on its own operands and keeps the
@@ -105,7 +108,8 @@ struct Ctx {
   bool autotune = false;
   std::unordered_map<uint64_t, std::pair<int, int>> tune_table;
   // Arithmetic of the tiled block GEMMs (sb_ctx_set_precision): SB_PRECISION_F64
-  // (DMMA, the drop-in), SB_PRECISION_TF32X3 or SB_PRECISION_TF32 (tcgen05).
+  // (DMMA, the drop-in), SB_PRECISION_F64_I8 (large FP64 launches on the integer
+  // tensor cores), SB_PRECISION_TF32X3 or SB_PRECISION_TF32 (tcgen05).
   // The thin K <= 16 launches compute in FP64 in every mode (they are
   // HBM-bound); they read and write FP32-stored intermediates as FP32.
   int precision = SB_PRECISION_F64;

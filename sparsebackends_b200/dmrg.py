@@ -112,7 +112,8 @@ class DMRG:
     def __init__(self, n: int, delta: float = 1.0, ctx=None, precision: str = "f64", device_split="auto",
                  mpo=None, split_method: str = "svd"):
         """``precision``: the H_eff applies inside Lanczos run in that context
-        precision ("tf32x3": tcgen05 3xTF32 with FP32 intermediates); the
+        precision ("tf32x3": tcgen05 3xTF32 with FP32 intermediates; "f64i8":
+        FP64 of norm-wise accuracy, which needs no correction); the
         Lanczos vectors, orthogonalisation, the split and the environments stay
         FP64, and each bond's energy is the FP64 Rayleigh quotient of its Ritz
         vector (``krylov.eigsolve(..., correction=)``).  ``device_split``: True,
@@ -134,7 +135,7 @@ class DMRG:
         # per-apply accuracy: on the N = 100 Heisenberg chain (chi to 109) 1e-7
         # gives the FP64 energy to 1.7e-11, 1e-6 to 4.8e-10, 1e-5 to 2.3e-8
         # (bonds whose residual falls below it stop improving)
-        self.optol = {"f64": 0.0, "tf32x3": 1e-7, "tf32": 3e-2}[precision]
+        self.optol = {"f64": 0.0, "f64i8": 0.0, "tf32x3": 1e-7, "tf32": 3e-2}[precision]
         self.device_split = device_split
         self.split_method = split_method
         self.n = n
@@ -178,7 +179,7 @@ class DMRG:
         lay, x = self._two_site(i)
         ops = (lay, self.Lenv[i - 1], self.Ws[i - 1], self.Ws[i], self.Renv[i + 1], self.ctx)
         op = qn.HeffOperator(*ops, precision=self.precision)
-        corr = qn.HeffOperator(*ops) if self.precision != "f64" else None
+        corr = qn.HeffOperator(*ops) if self.precision in qn.TF32_PRECISIONS else None
         vals, vecs, _ = krylov.eigsolve(op, x, 1, "SR", krylovdim=krylovdim, maxiter=maxiter, tol=1e-14,
                                         correction=corr, optol=self.optol)
         self.energy = float(vals[0])

@@ -500,6 +500,9 @@ def hermitian_operators(layout: HeffLayout, rng: np.random.Generator, scales=Non
     return out
 
 
+TF32_PRECISIONS = ("tf32x3", "tf32")  # context precisions that round operands to FP32
+
+
 class HeffOperator:
     """x -> H_eff x as a new device tensor (the operator KrylovKit's eigsolve
     applies: ITensorMPS ``product(::ProjMPO, v)``).  Operands stay resident;
@@ -513,8 +516,8 @@ class HeffOperator:
         each call copies its input there and replays the graph.  ``w12`` picks
         the chain ψ·L·(W1·W2)·R (``HeffChain``).  ``precision``: the context
         precision the chain's block GEMMs run in (``Context.set_precision``;
-        set for each apply and restored after it); in a tensor-core precision
-        the intermediates are FP32 unless ``f32_intermediates`` is False."""
+        set for each apply and restored after it); in "tf32x3" and "tf32" the
+        intermediates are FP32 unless ``f32_intermediates`` is False."""
         import sparsebackends_b200 as sb
         self.sb = sb
         self.ctx = ctx or L.ctx
@@ -522,9 +525,9 @@ class HeffOperator:
         # relative accuracy of one apply (krylov.eigsolve's optol): measured
         # per-block errors of the tensor-core GEMMs are a few 1e-7 to 1e-6
         # (3xTF32) and 3e-4 (TF32); the bound leaves a margin
-        self.accuracy = {"f64": 0.0, "tf32x3": 1e-5, "tf32": 3e-2}[precision]
+        self.accuracy = {"f64": 0.0, "f64i8": 0.0, "tf32x3": 1e-5, "tf32": 3e-2}[precision]
         if f32_intermediates is None:
-            f32_intermediates = precision != "f64"
+            f32_intermediates = precision in TF32_PRECISIONS
         self.chain = HeffChain(layout, self.ctx, w12=w12, f32_intermediates=f32_intermediates)
         self.ops = (L, W1, W2, R)
         self.calls = 0

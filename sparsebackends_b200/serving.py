@@ -176,7 +176,7 @@ def _relative(results: List[Result], t: float) -> List[Result]:
 
 class Server:
     """``slots`` solves in flight under ``budget_bytes`` of estimated device
-    memory, each in ``precision`` ("f64" or "tf32x3"), one thread and one
+    memory, each in ``precision`` ("f64", "f64i8" or "tf32x3"), one thread and one
     library context (stream) per slot."""
 
     def __init__(self, slots: int = 4, budget_bytes: int = 64 << 30, precision: str = "f64", device: int = 0):
