@@ -279,6 +279,7 @@ struct GemmLaunch {
   int64_t n = 0;  // strips (thin) or tiles
   bool xT = false, yT = false, small_rows = false, persistent = false;
   int small_max = 0, k_max = 0, splitk = 1, bm = 64, bn = 64;
+  bool split_partials = false;  // split-K through partial tiles in memory
   GemmShape shape = GemmShape::T64x64;
   // tensor-core launches: explicit tile list, tiles [nz_begin, n) are the
   // pair-less C blocks; swap puts Y on the 128-row side; passes 3 or 1
@@ -440,16 +441,19 @@ struct GemmLaunch {
       ctx->note_launch();
       return;
     }
+    DevBuf part;
+    const int64_t tile = kind == EDGES ? 64 * 64 : static_cast<int64_t>(bm) * bn;
+    if (split_partials) part = DevBuf(ctx, static_cast<size_t>(splitk) * n * tile * sizeof(double));
     {
       ProfScope ps(ctx, PROF_GEMM, flops, bytes);
       if (kind == EDGES)
         SB_CK(launch_gemm_f64_edges(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), n, xT, yT, ctx->stream,
-                                    splitk));
+                                    splitk, part.d()));
       else
         SB_CK(launch_gemm_f64(X, Y, C, dc.as<GemmCBlock>(), ncb, dp.as<GemmPair>(), n, xT, yT, shape, ctx->stream,
-                              splitk));
+                              splitk, part.d()));
     }
-    ctx->note_launch();
+    ctx->note_launch(split_partials ? 2 : 1);
   }
 };
 
@@ -609,6 +613,7 @@ struct GemmPlan {
     g.bm = bm;
     g.bn = bn;
     g.splitk = splitk;
+    g.split_partials = splitk > 1 && beyond_l2(ctx, bytes);
     g.flops = flops;
     g.bytes = bytes;
     return g;
@@ -1170,8 +1175,31 @@ struct GemmPlan {
     return any;
   }
 
+  // Whether a split launch leaves partial tiles in memory, its segments
+  // outermost, instead of summing them inside clusters: when the operands take
+  // more than twice L2, so that CTAs running at the same time should work on one
+  // K range of many tiles (R*T3 of H_eff at chi = 2048, 900 MB: 2010 us in
+  // clusters, 1911 with partial tiles; the whole apply, us, clusters and partial
+  // tiles: chi = 1024 788 and 797, 1200 1193 and 1184, 1400 1662 and 1635, 2048
+  // 4521 and 4416).  bytes: every pair's blocks counted anew, an upper bound.
+  bool beyond_l2(Ctx* ctx, double bytes) const {
+    int l2 = 0;
+    cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
+    if (bytes <= 2.0 * l2) return false;
+    std::unordered_map<int64_t, int64_t> x, y;  // distinct operand blocks
+    for (const GemmCBlock& c : cbs)
+      for (int p = c.pair_begin; p < c.pair_end; ++p) {
+        x[pairs[p].x_off] = static_cast<int64_t>(c.M) * pairs[p].K;
+        y[pairs[p].y_off] = static_cast<int64_t>(c.N) * pairs[p].K;
+      }
+    double distinct = 0.0;
+    for (const auto* m : {&x, &y})
+      for (const auto& e : *m) distinct += 8.0 * static_cast<double>(e.second);
+    return distinct > 2.0 * l2;
+  }
+
   // Split-K factor for ntiles tiles with kt_avg k-tiles on average and kt_max
-  // at most (a power of two up to the cluster size): split while the tiles
+  // at most (a power of two): split while the tiles
   // fill less than ~6 waves of 148 SMs x 4 CTAs and every segment keeps >= 32
   // k-tiles (the shorter CTAs balance the uneven K loops), and, when there are
   // fewer CTAs than 4 per SM, as long as the longest K loop keeps >= 4 k-tiles
@@ -1296,6 +1324,7 @@ struct GemmPlan {
     g.ncb = static_cast<int32_t>(sc.size());
     g.n = ntiles;
     g.splitk = splitk;
+    g.split_partials = splitk > 1 && beyond_l2(ctx, bytes);
     g.flops = flops;
     g.bytes = bytes;
     return true;

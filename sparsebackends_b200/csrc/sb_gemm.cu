@@ -57,8 +57,17 @@ struct TileLayout {
   __device__ static int yidx(int k, int j) { return YT ? k * (BN + 4) + j : j * KP + k; }
 };
 
-// C block of tile `bid`, the last c with tile_begin <= bid, by a full warp
-// (every lane gets the result): each round
+// C block of tile `bid`: the last c with tile_begin <= bid.
+__device__ __forceinline__ int tile_cblock(const GemmCBlock* __restrict__ cblocks, int32_t ncb, int bid) {
+  int lo = 0, hi = ncb - 1;
+  while (lo < hi) {
+    const int mid = (lo + hi + 1) >> 1;
+    if (cblocks[mid].tile_begin <= bid) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// The same lookup by a full warp (every lane gets the result): each round
 // tests 32 evenly spaced candidates at once, so 120 blocks take two dependent
 // loads and 30000 take three, against 7 and 15 for a bisection.  The answer
 // stays in [lo, hi] with tile_begin[lo] <= bid; the lanes whose candidate
@@ -99,10 +108,11 @@ __device__ __noinline__ void sum_cluster_tile(double* smem, double* cbase, int M
 }
 
 // One CTA of the tiled GEMM: tile lt of C block cb, k-segment seg of splitk.
-// With splitk > 1 the tile's segments are the CTAs of one cluster: each leaves
-// its partial tile in its own shared memory (the pipeline's buffers, free by
-// then) and every CTA sums a slice of the tile over all of them, in segment
-// order, through distributed shared memory.
+// With splitk > 1 and partial NULL the tile's segments are the CTAs of one cluster:
+// each leaves its partial tile in its own shared memory (the pipeline's buffers,
+// free by then) and every CTA sums a slice of the tile over all of them, in
+// segment order, through distributed shared memory.  Otherwise the BMC x BNC
+// tile goes to the CTA's part_elems of partial (column-major), for k_splitk_reduce.
 // BM x BN is the staged (shared-memory) tile; the C tile BMC x BNC may be
 // narrower (48 of 64 rows or columns: the operand copies past BMC / BNC are
 // zero-filled without reading memory, and no warp multiplies them).
@@ -110,7 +120,7 @@ template <int BM, int BN, int WM, int WN, bool XT, bool YT, int BK, int ST, int 
 __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const double* __restrict__ Y,
                                          double* __restrict__ C, const GemmCBlock& cb,
                                          const GemmPair* __restrict__ pairs, int lt, int seg, int32_t splitk,
-                                         double* smem) {
+                                         double* __restrict__ partial, int part_elems, double* smem) {
   constexpr int kBK = BK;
   constexpr int kStages = ST;
   using TL = TileLayout<BM, BN, XT, YT, BK, ST>;
@@ -280,18 +290,19 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
   double* cbase = C + cb.c_off;
   if (splitk > 1) {
     static_assert(BMC * BNC <= ST * (TL::XSZ + TL::YSZ), "the partial tile must fit in the pipeline's buffers");
-    __syncthreads();  // every warp has read its last operand tile
+    double* const tile = partial ? partial + static_cast<int64_t>(blockIdx.x) * part_elems : smem;
+    if (!partial) __syncthreads();  // every warp has read its last operand tile
 #pragma unroll
     for (int a = 0; a < MT; ++a) {
       const int rl = wm * WM + a * 8 + g;
 #pragma unroll
       for (int b = 0; b < NTL; ++b) {
         const int cl = wn * WN + b * 8 + 2 * t;
-        smem[rl + cl * BMC] = acc[a][b][0];
-        smem[rl + (cl + 1) * BMC] = acc[a][b][1];
+        tile[rl + cl * BMC] = acc[a][b][0];
+        tile[rl + (cl + 1) * BMC] = acc[a][b][1];
       }
     }
-    sum_cluster_tile<BMC, BNC, NT>(smem, cbase, M, N, cb.ldc, m0, n0, seg, splitk);
+    if (!partial) sum_cluster_tile<BMC, BNC, NT>(smem, cbase, M, N, cb.ldc, m0, n0, seg, splitk);
     return;
   }
 #pragma unroll
@@ -307,20 +318,30 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
   }
 }
 
-// Split-K: CTA = (tile, segment), the segments of a tile adjacent: they form
-// the launch's clusters (at most 8 CTAs, the portable size).  The sum through
-// distributed shared memory replaces partial tiles in HBM and a second launch
-// (7.5 us of the chi = 512 R*T3), which makes splits of few k-tiles pay.
+// Split-K: CTA = (tile, segment).  In clusters the segments of a tile are
+// adjacent: they form the launch's clusters (at most 8 CTAs, the portable size), and the sum through distributed shared memory replaces partial tiles in
+// HBM and a second launch (7.5 us of the chi = 512 R*T3), which makes splits of
+// few k-tiles pay.  With partial tiles the segments are outermost, so that CTAs
+// running at the same time work on the same K range of neighbouring tiles and
+// find each other's operand panels in L2: R*T3 at chi = 2048 takes 1911 us,
+// 2010 in clusters.
+__device__ __forceinline__ void split_cta(int32_t splitk, int32_t ntiles, const double* partial, int& bid, int& seg) {
+  const int b = static_cast<int>(blockIdx.x);
+  bid = partial ? b % ntiles : b / splitk;
+  seg = partial ? b / ntiles : b % splitk;
+}
+
 template <int BM, int BN, int WM, int WN, bool XT, bool YT, int BK = kBK, int ST = kStages>
 __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32, 512 / ((BM / WM) * (BN / WN) * 32))
     k_gemm_f64(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ C,
                const GemmCBlock* __restrict__ cblocks, int32_t ncb, const GemmPair* __restrict__ pairs,
-               int32_t splitk) {
+               int32_t splitk, int32_t ntiles, double* __restrict__ partial) {
   extern __shared__ double smem[];
-  const int bid = static_cast<int>(blockIdx.x) / splitk;
-  const int seg = static_cast<int>(blockIdx.x) % splitk;
+  int bid, seg;
+  split_cta(splitk, ntiles, partial, bid, seg);
   const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
-  gemm_cta<BM, BN, WM, WN, XT, YT, BK, ST>(X, Y, C, cb, pairs, bid - cb.tile_begin, seg, splitk, smem);
+  gemm_cta<BM, BN, WM, WN, XT, YT, BK, ST>(X, Y, C, cb, pairs, bid - cb.tile_begin, seg, splitk, partial,
+                                           BM * BN, smem);
 }
 
 // Five tile shapes in one launch (launch_gemm_f64_edges): the tiles of every
@@ -328,32 +349,77 @@ __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32, 512 / ((BM / WM) *
 // sub-block's tshape picks the CTA's tile: 0 = 64x64 (32x32 warp tiles),
 // 1 = 64x32 (32x16), 2 = 32x64 (16x32), 3 = 64x48 (32x24), 4 = 48x64 (24x32),
 // all four warps and 3 stages (the 48-wide ones stage 64x64 operand tiles).
+// Partial tiles are kEdgePart doubles apart whatever their shape.
 constexpr int kEdgeThreads = 128;
+constexpr int kEdgePart = 64 * 64;
 template <bool XT, bool YT>
 __global__ void __launch_bounds__(kEdgeThreads, 4)
     k_gemm_f64_edges(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ C,
                      const GemmCBlock* __restrict__ cblocks, int32_t ncb, const GemmPair* __restrict__ pairs,
-                     int32_t splitk) {
+                     int32_t splitk, int32_t ntiles, double* __restrict__ partial) {
   extern __shared__ double smem[];
-  const int bid = static_cast<int>(blockIdx.x) / splitk;
-  const int seg = static_cast<int>(blockIdx.x) % splitk;
+  int bid, seg;
+  split_cta(splitk, ntiles, partial, bid, seg);
   const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
   const int lt = bid - cb.tile_begin;
   if (cb.tshape == 0)
-    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, smem);
+    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
   else if (cb.tshape == 1)
-    gemm_cta<64, 32, 32, 16, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, smem);
+    gemm_cta<64, 32, 32, 16, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
   else if (cb.tshape == 2)
-    gemm_cta<32, 64, 16, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, smem);
+    gemm_cta<32, 64, 16, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
   else if (cb.tshape == 3)
-    gemm_cta<64, 64, 32, 24, XT, YT, kBK, kStages, 64, 48>(X, Y, C, cb, pairs, lt, seg, splitk, smem);
+    gemm_cta<64, 64, 32, 24, XT, YT, kBK, kStages, 64, 48>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
   else
-    gemm_cta<64, 64, 24, 32, XT, YT, kBK, kStages, 48, 64>(X, Y, C, cb, pairs, lt, seg, splitk, smem);
+    gemm_cta<64, 64, 24, 32, XT, YT, kBK, kStages, 48, 64>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
 }
 
-// Launch with the segments of each tile as a cluster (splitk > 1).
+// Deterministic split-K reduction: C tile = sum over segments in order.
+// Element e: tile e / stride, offset e % stride in the column-major BM x BN
+// partial tile.
+__device__ __forceinline__ void splitk_reduce_elem(double* __restrict__ C, const GemmCBlock& cb, int bm, int bn,
+                                                   int lt, int w, int32_t splitk, int64_t seg_stride,
+                                                   const double* __restrict__ pt) {
+  if (w >= bm * bn) return;
+  const int rl = w % bm, cl = w / bm;
+  const int row = (lt % cb.mtiles) * bm + rl, col = (lt / cb.mtiles) * bn + cl;
+  if (row >= cb.M || col >= cb.N) return;
+  double acc = 0.0;
+  for (int sg = 0; sg < splitk; ++sg) acc += pt[sg * seg_stride + w];
+  C[cb.c_off + row + static_cast<int64_t>(col) * cb.ldc] = acc;
+}
+
+template <int BM, int BN>
+__global__ void k_splitk_reduce(double* __restrict__ C, const GemmCBlock* __restrict__ cblocks, int32_t ncb,
+                                int32_t splitk, int32_t ntiles, const double* __restrict__ partial) {
+  const int64_t total = static_cast<int64_t>(ntiles) * BM * BN;
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
+       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int bid = static_cast<int>(e / (BM * BN)), w = static_cast<int>(e % (BM * BN));
+    const GemmCBlock cb = cblocks[tile_cblock(cblocks, ncb, bid)];
+    splitk_reduce_elem(C, cb, BM, BN, bid - cb.tile_begin, w, splitk, static_cast<int64_t>(ntiles) * BM * BN,
+                       partial + static_cast<int64_t>(bid) * BM * BN);
+  }
+}
+
+__global__ void k_splitk_reduce_edges(double* __restrict__ C, const GemmCBlock* __restrict__ cblocks, int32_t ncb,
+                                      int32_t splitk, int32_t ntiles, const double* __restrict__ partial) {
+  const int64_t total = static_cast<int64_t>(ntiles) * kEdgePart;
+  for (int64_t e = static_cast<int64_t>(blockIdx.x) * blockDim.x + threadIdx.x; e < total;
+       e += static_cast<int64_t>(gridDim.x) * blockDim.x) {
+    const int bid = static_cast<int>(e / kEdgePart), w = static_cast<int>(e % kEdgePart);
+    const GemmCBlock cb = cblocks[tile_cblock(cblocks, ncb, bid)];
+    const int bm = cb.tshape == 2 ? 32 : cb.tshape == 4 ? 48 : 64;
+    const int bn = cb.tshape == 1 ? 32 : cb.tshape == 3 ? 48 : 64;
+    splitk_reduce_elem(C, cb, bm, bn, bid - cb.tile_begin, w, splitk, static_cast<int64_t>(ntiles) * kEdgePart,
+                       partial + static_cast<int64_t>(bid) * kEdgePart);
+  }
+}
+
+// Launch with the segments of each tile as a cluster (cluster) or on their own.
 template <class... P, class... A>
-cudaError_t launch_split(void (*kern)(P...), int64_t ntiles, int splitk, int threads, int smem, cudaStream_t s, A... args) {
+cudaError_t launch_split(void (*kern)(P...), int64_t ntiles, int splitk, bool cluster, int threads, int smem,
+                         cudaStream_t s, A... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(static_cast<unsigned>(ntiles * splitk));
   cfg.blockDim = dim3(static_cast<unsigned>(threads));
@@ -364,13 +430,13 @@ cudaError_t launch_split(void (*kern)(P...), int64_t ntiles, int splitk, int thr
   at.val.clusterDim.x = static_cast<unsigned>(splitk);
   at.val.clusterDim.y = at.val.clusterDim.z = 1;
   cfg.attrs = &at;
-  cfg.numAttrs = splitk > 1 ? 1 : 0;
+  cfg.numAttrs = cluster && splitk > 1 ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 template <int BM, int BN, int WM, int WN, bool XT, bool YT, int BK = kBK, int ST = kStages>
 cudaError_t launch_t(const double* X, const double* Y, double* C, const GemmCBlock* cb, int32_t ncb,
-                     const GemmPair* pr, int64_t ntiles, int splitk, cudaStream_t s) {
+                     const GemmPair* pr, int64_t ntiles, int splitk, double* partial, cudaStream_t s) {
   constexpr int threads = (BM / WM) * (BN / WN) * 32;
   constexpr int smem = TileLayout<BM, BN, XT, YT, BK, ST>::bytes();
   auto kern = k_gemm_f64<BM, BN, WM, WN, XT, YT, BK, ST>;
@@ -385,18 +451,23 @@ cudaError_t launch_t(const double* X, const double* Y, double* C, const GemmCBlo
     configured.fetch_or(bit);
   }
   if (ntiles <= 0) return cudaSuccess;
-  if (splitk < 1 || splitk > kMaxSplitK || ntiles * splitk > 0x7fffffffLL) return cudaErrorInvalidValue;
-  return launch_split(kern, ntiles, splitk, threads, smem, s, X, Y, C, cb, ncb, pr, splitk);
+  if (splitk < 1 || (!partial && splitk > kMaxSplitK) || ntiles * splitk > 0x7fffffffLL) return cudaErrorInvalidValue;
+  const int32_t nt = static_cast<int32_t>(ntiles);
+  e = launch_split(kern, ntiles, splitk, !partial, threads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
+  if (e != cudaSuccess || !partial) return e;
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>((ntiles * BM * BN + 255) / 256, 148LL * 64));
+  k_splitk_reduce<BM, BN><<<g, 256, 0, s>>>(C, cb, ncb, splitk, nt, partial);
+  return cudaGetLastError();
 }
 
 template <int BM, int BN, int WM, int WN, int BK = kBK, int ST = kStages>
 cudaError_t dispatch_t(bool xT, bool yT, const double* X, const double* Y, double* C,
-                       const GemmCBlock* cb, int32_t ncb, const GemmPair* pr, int64_t nt, int sk,
+                       const GemmCBlock* cb, int32_t ncb, const GemmPair* pr, int64_t nt, int sk, double* part,
                        cudaStream_t s) {
-  if (!xT && !yT) return launch_t<BM, BN, WM, WN, false, false, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, s);
-  if (!xT && yT) return launch_t<BM, BN, WM, WN, false, true, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, s);
-  if (xT && !yT) return launch_t<BM, BN, WM, WN, true, false, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, s);
-  return launch_t<BM, BN, WM, WN, true, true, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, s);
+  if (!xT && !yT) return launch_t<BM, BN, WM, WN, false, false, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, part, s);
+  if (!xT && yT) return launch_t<BM, BN, WM, WN, false, true, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, part, s);
+  if (xT && !yT) return launch_t<BM, BN, WM, WN, true, false, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, part, s);
+  return launch_t<BM, BN, WM, WN, true, true, BK, ST>(X, Y, C, cb, ncb, pr, nt, sk, part, s);
 }
 
 // 64x64 tiles walked by a resident grid, for a launch that another kernel has
@@ -411,7 +482,7 @@ __global__ void __launch_bounds__(128, 4)
   if (flag && *flag == 0) return;
   for (int bid = static_cast<int>(blockIdx.x); bid < ntiles; bid += static_cast<int>(gridDim.x)) {
     const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
-    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, bid - cb.tile_begin, 0, 1, smem);
+    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, bid - cb.tile_begin, 0, 1, nullptr, 0, smem);
     __syncthreads();  // the operand buffers are refilled by the next tile
   }
 }
@@ -907,7 +978,7 @@ cudaError_t launch_gemm_f64_skinny(const double* X, const double* Y, double* C, 
 
 template <bool XT, bool YT>
 cudaError_t launch_edges_t(const double* X, const double* Y, double* C, const GemmCBlock* cb, int32_t ncb,
-                           const GemmPair* pr, int64_t ntiles, int splitk, cudaStream_t s) {
+                           const GemmPair* pr, int64_t ntiles, int splitk, double* partial, cudaStream_t s) {
   constexpr int smem = std::max(std::max(TileLayout<64, 64, XT, YT>::bytes(), TileLayout<64, 32, XT, YT>::bytes()),
                                 TileLayout<32, 64, XT, YT>::bytes());
   auto kern = k_gemm_f64_edges<XT, YT>;
@@ -921,18 +992,23 @@ cudaError_t launch_edges_t(const double* X, const double* Y, double* C, const Ge
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
-  return launch_split(kern, ntiles, splitk, kEdgeThreads, smem, s, X, Y, C, cb, ncb, pr, splitk);
+  const int32_t nt = static_cast<int32_t>(ntiles);
+  e = launch_split(kern, ntiles, splitk, !partial, kEdgeThreads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
+  if (e != cudaSuccess || !partial) return e;
+  const unsigned g = static_cast<unsigned>(std::min<int64_t>((ntiles * kEdgePart + 255) / 256, 148LL * 64));
+  k_splitk_reduce_edges<<<g, 256, 0, s>>>(C, cb, ncb, splitk, nt, partial);
+  return cudaGetLastError();
 }
 
 cudaError_t launch_gemm_f64_edges(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,
                                   int32_t ncb, const GemmPair* d_pairs, int64_t ntiles, bool xT, bool yT,
-                                  cudaStream_t s, int splitk) {
+                                  cudaStream_t s, int splitk, double* partial) {
   if (ntiles <= 0) return cudaSuccess;
-  if (splitk < 1 || splitk > kMaxSplitK || ntiles * splitk > 0x7fffffffLL) return cudaErrorInvalidValue;
-  if (!xT && !yT) return launch_edges_t<false, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
-  if (!xT && yT) return launch_edges_t<false, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
-  if (xT && !yT) return launch_edges_t<true, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
-  return launch_edges_t<true, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+  if (splitk < 1 || (!partial && splitk > kMaxSplitK) || ntiles * splitk > 0x7fffffffLL) return cudaErrorInvalidValue;
+  if (!xT && !yT) return launch_edges_t<false, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
+  if (!xT && yT) return launch_edges_t<false, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
+  if (xT && !yT) return launch_edges_t<true, false>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
+  return launch_edges_t<true, true>(X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
 }
 
 cudaError_t launch_gemm_f64_fallback(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,
@@ -949,20 +1025,20 @@ cudaError_t launch_gemm_f64_fallback(const double* X, const double* Y, double* C
 cudaError_t launch_gemm_f64(const double* X, const double* Y, double* C,
                             const GemmCBlock* d_cblocks, int32_t ncb, const GemmPair* d_pairs,
                             int64_t ntiles, bool xT, bool yT, GemmShape shape, cudaStream_t s,
-                            int splitk) {
+                            int splitk, double* partial) {
   switch (shape) {
     case GemmShape::T128x32:
-      return dispatch_t<128, 32, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<128, 32, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
     case GemmShape::T32x128:
-      return dispatch_t<32, 128, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<32, 128, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
     case GemmShape::T128x64:
-      return dispatch_t<128, 64, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<128, 64, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
     case GemmShape::T64x128:
-      return dispatch_t<64, 128, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<64, 128, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
     case GemmShape::T64x32:
-      return dispatch_t<64, 32, 32, 16, 16, 4>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<64, 32, 32, 16, 16, 4>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
     default:
-      return dispatch_t<64, 64, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, s);
+      return dispatch_t<64, 64, 32, 32>(xT, yT, X, Y, C, d_cblocks, ncb, d_pairs, ntiles, splitk, partial, s);
   }
 }
 

@@ -47,13 +47,14 @@ struct GemmPair {
 enum class GemmShape : int { T64x64 = 0, T128x32 = 1, T32x128 = 2, T128x64 = 3, T64x128 = 4, T64x32 = 5 };
 
 // splitk > 1 (at most kMaxSplitK): the concatenated K range of every C tile is
-// cut into splitk segments, computed by the CTAs of one cluster and summed in
-// segment order through their shared memory (deterministic).
+// cut into splitk segments, each computed by a CTA of its own, and summed in
+// segment order (deterministic): through the shared memory of a cluster, or,
+// with partial (splitk * ntiles * BM*BN doubles), by a second kernel.
 constexpr int kMaxSplitK = 8;  // the portable cluster size
 cudaError_t launch_gemm_f64(const double* X, const double* Y, double* C,
                             const GemmCBlock* d_cblocks, int32_t ncblocks, const GemmPair* d_pairs,
                             int64_t ntiles, bool xT, bool yT, GemmShape shape, cudaStream_t s,
-                            int splitk = 1);
+                            int splitk = 1, double* partial = nullptr);
 
 // Tiled GEMM over C sub-blocks of five tile shapes in one launch: each
 // GemmCBlock's tshape gives its tile (0 = 64x64; 1 = 64x32 and 3 = 64x48 for
@@ -61,10 +62,10 @@ cudaError_t launch_gemm_f64(const double* X, const double* Y, double* C,
 // edges of height <= 32 and <= 48); tiles are
 // numbered through tile_begin / mtiles of that shape.  Sub-blocks carry their
 // own ldc and pairs whose offsets start at the sub-block's first row and
-// column.
+// column.  partial, if any: splitk * ntiles * 4096 doubles.
 cudaError_t launch_gemm_f64_edges(const double* X, const double* Y, double* C, const GemmCBlock* d_cblocks,
                                   int32_t ncblocks, const GemmPair* d_pairs, int64_t ntiles, bool xT, bool yT,
-                                  cudaStream_t s, int splitk = 1);
+                                  cudaStream_t s, int splitk = 1, double* partial = nullptr);
 
 // Thin variant for launches whose every pair has K <= 16 and whose C blocks
 // have min(M, N) <= 16 (HBM-bound): DMMA on 128 x 16 strips of the long side,
