@@ -1206,11 +1206,15 @@ struct GemmPlan {
   // per segment: one SM takes 0.5 us per 64x64x16 k-tile, so a few long
   // tiles leave the chip idle (R*T3 of H_eff, us, before and after: chi = 256,
   // 42 tiles of up to 130 k-tiles, 121 and 27; chi = 400 122 and 50; chi = 512
-  // 99 and 71; chi = 700 165 and 131; chi = 1024 332 and 318).
+  // 99 and 71; chi = 700 165 and 131; chi = 1024 332 and 318).  16 segments only
+  // while 8 leave SMs without a CTA (a 64x64 block with K = 8192, us, 8 and 16
+  // segments: 43 and 25; 18 tiles of K = 16384 151 and 130; 24 of K = 8192 94
+  // and 94; 32 of K = 8192 95 and 107).
   static int choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg, int64_t kt_max) {
     int splitk = 1;
     const int64_t wave = 148 * 4;
-    while (splitk < kMaxSplitK && ((ntiles * splitk < 6 * wave && kt_avg / (2 * splitk) >= 32) ||
+    const int cap = ntiles * kPortableCluster <= 148 ? kMaxSplitK : kPortableCluster;
+    while (splitk < cap && ((ntiles * splitk < 6 * wave && kt_avg / (2 * splitk) >= 32) ||
                                    (ntiles * splitk < wave && kt_max / (2 * splitk) >= 4)))
       splitk *= 2;
     if (ctx->gemm_splitk > 0) splitk = std::min(ctx->gemm_splitk, kMaxSplitK);

@@ -319,7 +319,8 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
 }
 
 // Split-K: CTA = (tile, segment).  In clusters the segments of a tile are
-// adjacent: they form the launch's clusters (at most 8 CTAs, the portable size), and the sum through distributed shared memory replaces partial tiles in
+// adjacent: they form the launch's clusters (up to 16 CTAs; 8 is the portable
+// size), and the sum through distributed shared memory replaces partial tiles in
 // HBM and a second launch (7.5 us of the chi = 512 R*T3), which makes splits of
 // few k-tiles pay.  With partial tiles the segments are outermost, so that CTAs
 // running at the same time work on the same K range of neighbouring tiles and
@@ -447,6 +448,8 @@ cudaError_t launch_t(const double* X, const double* Y, double* C, const GemmCBlo
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(configured & bit)) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
@@ -989,6 +992,8 @@ cudaError_t launch_edges_t(const double* X, const double* Y, double* C, const Ge
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(configured & bit)) {
     e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }

@@ -50,7 +50,7 @@ enum class GemmShape : int { T64x64 = 0, T128x32 = 1, T32x128 = 2, T128x64 = 3, 
 // cut into splitk segments, each computed by a CTA of its own, and summed in
 // segment order (deterministic): through the shared memory of a cluster, or,
 // with partial (splitk * ntiles * BM*BN doubles), by a second kernel.
-constexpr int kMaxSplitK = 8;  // the portable cluster size
+constexpr int kMaxSplitK = 16, kPortableCluster = 8;
 cudaError_t launch_gemm_f64(const double* X, const double* Y, double* C,
                             const GemmCBlock* d_cblocks, int32_t ncblocks, const GemmPair* d_pairs,
                             int64_t ntiles, bool xT, bool yT, GemmShape shape, cudaStream_t s,

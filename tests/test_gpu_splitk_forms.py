@@ -1,4 +1,5 @@
-"""Split-K through partial tiles (operands beyond twice L2), every tile shape, uneven K loops and both operand orders, against numpy in
+"""Split-K in clusters of 16 and through partial tiles (operands beyond twice
+L2), every tile shape, uneven K loops and both operand orders, against numpy in
 extended precision.  The tolerance is the sum's own rounding bound: K additions
 of relative error 2^-53 on the sum of magnitudes."""
 import os
@@ -57,6 +58,21 @@ def _check(sb, ctx, A, B, rows, launches=None):
             c = (c if tail[0] == "m" else c.T)[:rows]
             want = a.astype(np.longdouble) @ b.astype(np.longdouble)
             assert np.all(np.abs(c - want) <= a.shape[1] * 2.0 ** -53 * (np.abs(a) @ np.abs(b))), (i, tail)
+
+
+@pytest.mark.parametrize("tile", TILES)
+def test_clusters_of_sixteen(tile):
+    import sparsebackends_b200 as sb
+    env = dict(SPARSEB_GEMM_SPLITK=16, SPARSEB_GEMM_THIN=0, **({"SPARSEB_GEMM_TILE": tile} if tile else {}))
+    A, B = _blocks({1: 70, 2: 3, 3: 133}, {1: 5, 2: 200, 3: 17}, 66, ((2, 2), (2, 3)))
+    _check(sb, _ctx(sb, **env), A, B, 200, launches=1)
+
+
+def test_one_tile_with_a_long_k():
+    """Chosen by the launch rule: a single tile, 16 segments."""
+    import sparsebackends_b200 as sb
+    A, B = _blocks({1: 64}, {1: 8192}, 64, ())
+    _check(sb, sb.Context(0), A, B, 64, launches=1)
 
 
 @pytest.fixture(scope="module")
