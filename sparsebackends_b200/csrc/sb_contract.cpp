@@ -581,7 +581,11 @@ struct GemmPlan {
     if (ctx->gemm_tile >= 0) shape = static_cast<GemmShape>(ctx->gemm_tile);
     int bm, bn;
     gemm_tile_dims(shape, &bm, &bn);
-    // heavy C blocks first, as in prepare_edges
+    // Heavy C blocks first, so that the last CTAs to run are short ones; unlike in
+    // prepare_edges for long K loops too, where tiles of one shape already run
+    // together (blocks with 3 to 20 pairs, us, key order and this: 64x64x128 189
+    // and 168, 128x128x256 293 and 260, 32x256x512 353 and 299, 256x256x128 361
+    // and 320, 1024x512x512 1069 and 1026, 64x64x1024 beyond L2 1625 and 1562).
     std::stable_sort(cbs.begin(), cbs.end(),
                      [&](const GemmCBlock& a, const GemmCBlock& b) { return ktiles(pairs, a) > ktiles(pairs, b); });
     int64_t ntiles = 0;
