@@ -91,10 +91,14 @@ SB_API int64_t sb_ctx_launch_count(const sb_ctx* ctx);
  *                       element of a block row of A and column of B is then
  *                       held to 55 bits below the row's or column's largest
  *                       magnitude, not to 53 bits of its own, so the error of
- *                       an output is bounded against |row| |column| and no
- *                       longer against sum_k |a_k| |b_k|: a small output next
- *                       to large, unmatched entries loses its digits.  Rows
- *                       beyond 2^+-400, infinities and NaN go to DMMA;
+ *                       an output is bounded against |row| |column| (2-norms)
+ *                       and no longer against sum_k |a_k| |b_k|: a small
+ *                       output next to large, unmatched entries loses its
+ *                       digits.  About 2^-55 of |row| |column| on entries
+ *                       without a pattern; at most sqrt(K) 2^-53.9 + K 2^-59.6
+ *                       of it, besides the FP64 additions of the partial sums
+ *                       (K: length of a block pair's sum).  Rows beyond
+ *                       2^+-400, infinities and NaN go to DMMA;
  *   SB_PRECISION_TF32X3 tcgen05 tensor cores: every operand value rounded
  *                       to FP32 and split into TF32 hi + lo, the three
  *                       significant products accumulated in FP32 chunks of

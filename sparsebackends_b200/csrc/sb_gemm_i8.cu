@@ -13,10 +13,21 @@
 // bits and two more for the largest element.  In balanced radix 256 that is
 // seven signed 8-bit digits d_0 (most significant) .. d_6.  Products of digits
 // s and t weigh 256^(12-s-t); all products with s + t <= 7 are summed exactly
-// in INT32 accumulators, one per s + t ("diagonal"), 34 of the 49.  The ones
-// left out and the rounding of the integers are below 2^-55 of |row||column|
-// (2-norms), in the root mean square, whatever the entries; the sums of a DMMA
-// chain round at about 2^-55 of that too.  Four diagonals combine into one
+// in INT32 accumulators, one per s + t ("diagonal"), 34 of the 49.
+//
+// Error against |row||column| (2-norms), K the length of a pair's sum.  Worst
+// case: each side's rounding, at most 1.01 * 2^-55 of the row's largest magnitude
+// per element, adds up to 1.01 sqrt(K) 2^-55, and the digit products left out (at
+// most 5 * 2^14 * 2^32 units of 2^-108 per element, and little more) to
+// K 2^-59.6; rows of one large and many equal small entries come near it (x = y =
+// (1, c, ..., c), c with digits of 127: 27, 58 and 154 times 2^-55 at K = 700,
+// 1500 and 4000; bounds 82, 140 and 293).  With entries whose roundings and low
+// digits are independent of each other the two parts stay below 2^-55 in the
+// root mean square, where the sums of a DMMA chain round at about 2^-55 too.  It
+// is not a bound against sum_k |x_k||y_k|, which DMMA keeps: the path runs only
+// for callers that chose it (prepare_i8).
+//
+// Four diagonals combine into one
 // 64-bit integer, which converts to FP64 exactly; the sum over the chunks of K
 // and the pairs is in FP64.  Rows whose scale lies outside 2^+-400, infinities
 // and NaN set *flag, and the launch that follows (launch_gemm_f64_fallback)
