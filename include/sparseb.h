@@ -23,9 +23,10 @@
  * the context's stream; calls that must read device-computed structure flags
  * (value-dependent block creation) synchronise that stream internally.
  * A context keeps small pinned buffers (plan uploads, one scalar) and, in
- * SB_PRECISION_F64_I8 after large block GEMMs, up to 2 GB of device workspace,
- * which it gives back when an allocation finds no memory.  No function blocks
- * on other streams.
+ * SB_PRECISION_F64_I8 after large block GEMMs, up to 2 GB of device workspace.
+ * It gives that back when another allocation of the same context finds no
+ * memory, when a capture begins, and when its last tensor is freed; allocations
+ * of other contexts do not reclaim it.  No function blocks on other streams.
  */
 #ifndef SPARSEB_H
 #define SPARSEB_H

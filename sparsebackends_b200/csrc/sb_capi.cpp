@@ -73,6 +73,15 @@ void destroy_ctx_now(sb_ctx* ctx) {
   delete ctx;
 }
 
+// A tensor or graph of the context is gone.  With the last one goes the kept
+// workspace (an idle context holds no large memory), and the context itself if
+// it was waiting for this.
+void release_owner(sb_ctx* ctx) {
+  if (!ctx || --ctx->impl.live_tensors > 0) return;
+  if (!ctx->impl.capturing) ctx->impl.i8_scratch.reset();
+  if (ctx->impl.destroy_pending) destroy_ctx_now(ctx);
+}
+
 void check_keys_in_range(const std::vector<int64_t>& keys, int64_t n, int klen, const std::vector<int64_t>& dims) {
   for (int64_t i = 0; i < n; ++i)
     for (int j = 0; j < klen; ++j) {
@@ -484,7 +493,7 @@ sb_status sb_tensor_free(sb_tensor* t) {
     if (ctx) SB_CK(cudaSetDevice(ctx->impl.device));
     delete t;
   });
-  if (ctx && --ctx->impl.live_tensors == 0 && ctx->impl.destroy_pending) destroy_ctx_now(ctx);
+  release_owner(ctx);
   return st;
 }
 
@@ -891,7 +900,8 @@ sb_status sb_ctx_capture_begin(sb_ctx* ctx) {
     require(!c.capturing, SB_ERR_INVALID_ARG, "a capture is already open on this context");
     require(!c.profiling, SB_ERR_INVALID_ARG, "switch profiling off before capturing");
     SB_CK(cudaSetDevice(c.device));
-    c.sync();  // staged plan uploads of earlier calls are complete
+    c.i8_scratch.reset();  // the graph has a workspace of its own; its allocations may need this memory
+    c.sync();              // staged plan uploads of earlier calls are complete
     SB_CK(cudaStreamBeginCapture(c.stream, cudaStreamCaptureModeRelaxed));
     c.capturing = true;
     c.capture_keep.clear();
@@ -969,7 +979,7 @@ sb_status sb_graph_free(sb_graph* g) {
   if (ctx)
     for (void* p : g->keep_async) cudaFreeAsync(p, ctx->impl.stream);
   delete g;
-  if (ctx && --ctx->impl.live_tensors == 0 && ctx->impl.destroy_pending) destroy_ctx_now(ctx);
+  release_owner(ctx);
   return SB_OK;
 }
 

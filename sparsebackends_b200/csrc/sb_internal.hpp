@@ -130,7 +130,8 @@ struct Ctx {
   DevBuf dot_scratch;
   // Workspace of the integer GEMM (at most kI8ScratchKeep bytes), kept between
   // calls: used in stream order by one call at a time, given back when another
-  // allocation finds no memory and with the context.
+  // allocation of this context finds no memory, when a capture begins, and with
+  // the context's last tensor.
   DevBuf i8_scratch;
   double* host_scalar = nullptr;
   bool tc_launched = false;  // a tensor-core GEMM ran since the status was last read

@@ -58,12 +58,27 @@ class Result:
         return self.finish - self.arrival
 
 
-def footprint_bytes(req: Request) -> int:
+def footprint_bytes(req: Request, precision: str = "f64") -> int:
     """Upper estimate of a solve's device memory: site tensors (2 chi^2 per
     site), environments (5 chi^2 per bond: the MPO link of the XXZ chain), the
-    two-site H_eff intermediates (about 40 chi^2) and Lanczos vectors, in FP64."""
+    two-site H_eff intermediates (about 40 chi^2) and Lanczos vectors, in FP64;
+    in "f64i8" also the integer GEMM's workspace (``workspace_bytes``)."""
     chi2 = req.chi_max * req.chi_max
-    return 8 * chi2 * (2 * req.n + 5 * (req.n + 1) + 40 + 4 * (req.krylovdim + 2))
+    solve = 8 * chi2 * (2 * req.n + 5 * (req.n + 1) + 40 + 4 * (req.krylovdim + 2))
+    return solve + (workspace_bytes(req.chi_max) if precision == "f64i8" else 0)
+
+
+def workspace_bytes(chi: int) -> int:
+    """Upper estimate of the integer GEMM's workspace in a solve up to ``chi``:
+    seven digit planes of one byte per element of R and of the second
+    intermediate (5 + 20 chi^2 without charges), padded to tiles at most twofold;
+    two 128 x 128 FP64 partial tiles for each of the four work items per SM (148);
+    nothing while the largest contraction, below 80 chi^3 operations, stays under
+    the 2e8 that the path asks for.  The context gives it back with the solve's
+    last tensor."""
+    if 80 * chi ** 3 < 2e8:
+        return 0
+    return 7 * 25 * 2 * chi * chi + 2 * 4 * 148 * 128 * 128 * 8
 
 
 def poisson_arrivals(requests: List[Request], rate: float, seed: int) -> List[Request]:
@@ -91,13 +106,13 @@ def random_requests(count: int, seed: int, n_range=(8, 24), chi_range=(8, 64), s
     return out
 
 
-def _admit_loop(requests: List[Request], slots: int, budget: int, start_job) -> List[Result]:
+def _admit_loop(requests: List[Request], slots: int, budget: int, start_job, precision: str = "f64") -> List[Result]:
     """Replay the stream in real time and admit requests: ``start_job(req, slot,
-    on_done)`` starts a solve on a free slot and must call ``on_done(result or
-    exception)`` from any thread when it ends."""
+    on_done)`` starts a solve in ``precision`` on a free slot and must call
+    ``on_done(result or exception)`` from any thread when it ends."""
     for r in requests:
-        if footprint_bytes(r) > budget:
-            raise ValueError(f"request {r.rid} needs {footprint_bytes(r)} bytes, over the budget {budget}")
+        if footprint_bytes(r, precision) > budget:
+            raise ValueError(f"request {r.rid} needs {footprint_bytes(r, precision)} bytes, over the budget {budget}")
     pending = sorted(requests, key=lambda r: (r.arrival, r.rid))
     free = list(range(slots))
     state = {"used": 0, "running": 0}
@@ -128,12 +143,12 @@ def _admit_loop(requests: List[Request], slots: int, budget: int, start_job) -> 
             # admit the oldest queued request that fits
             admitted = None
             for q in queued:
-                if free and state["used"] + footprint_bytes(q) <= budget:
+                if free and state["used"] + footprint_bytes(q, precision) <= budget:
                     admitted = q
                     break
             if admitted is not None:
                 queued.remove(admitted)
-                slot, fp = free.pop(0), footprint_bytes(admitted)
+                slot, fp = free.pop(0), footprint_bytes(admitted, precision)
                 state["used"] += fp
                 state["running"] += 1
                 start_job(admitted, slot, done_for(slot, fp))
@@ -206,7 +221,7 @@ class Server:
                     on_done(exc)
             threading.Thread(target=work, daemon=True).start()
 
-        return _relative(_admit_loop(stream, self.slots, self.budget, start_job), t)
+        return _relative(_admit_loop(stream, self.slots, self.budget, start_job, self.precision), t)
 
 
 def summary(results: List[Result]) -> dict:
