@@ -421,8 +421,6 @@ __global__ void k_perm_block_rows(const double* __restrict__ src, double* __rest
 // of an environment with chi = 1024, w = 38 (88 MB moved): 53 us as a
 // per-element gather (1.65 TB/s), 29 us in tiles (3.0 TB/s); chi = 1500: 97 us
 // and 52 us (3.6 TB/s).
-constexpr int kPermTileElems = 64 * 65;
-constexpr int kPermTileRows = 1024;  // largest tv
 __global__ void __launch_bounds__(256, 6)
     k_perm_block_tiles(const double* __restrict__ src, double* __restrict__ dst,
                        const PermTileItem* __restrict__ items, int64_t n, int64_t total) {
@@ -770,54 +768,6 @@ cudaError_t launch_perm_block_rows(const double* src, double* dst, const BlockPe
   k_perm_block_rows<<<dim3(static_cast<unsigned>(gx), static_cast<unsigned>(gy)), kThreads, 0, s>>>(src, dst,
                                                                                                     d_items, n);
   return cudaGetLastError();
-}
-
-uint32_t perm_tile_cap(int64_t elems) {
-  const int64_t c = elems / (148LL * 12);
-  return static_cast<uint32_t>(c < 1056 ? 1056 : c > kPermTileElems ? kPermTileElems : c);
-}
-
-bool perm_tile_item(const BlockPerm& b, uint32_t cap, PermTileItem* out, int64_t* tiles) {
-  if (b.len <= 0 || b.len >= (int64_t{1} << 31) || b.rank < 1) return false;
-  PermTileItem p{};
-  p.src_off = b.src_off;
-  p.dst_off = b.dst_off;
-  p.rank = b.rank;
-  p.q = b.rank - 1;
-  for (int r = b.rank - 1; r >= 0; --r) {
-    if (b.in_lim[r] < b.out_dims[r] || (b.out_dims[r] > 1 && b.in_strides[r] >= (int64_t{1} << 31))) return false;
-    p.dims[r] = static_cast<uint32_t>(b.out_dims[r]);
-    p.strides[r] = b.out_dims[r] > 1 ? static_cast<uint32_t>(b.in_strides[r]) : 0;
-    if (b.in_strides[r] == 1 && b.out_dims[r] > 1) p.q = r;
-  }
-  if (b.out_dims[p.q] > 1 && b.in_strides[p.q] != 1) return false;
-  // output axis 0 contiguous in the source too (crops, outer-axis reorders):
-  // a tile would hold one row of axis 0, so only long rows qualify
-  if (p.q == 0 && p.dims[0] < 256 && b.len > p.dims[0]) return false;
-  int64_t nbatch = 1;
-  p.dv = 1;
-  for (int r = 0; r < p.q; ++r) p.dv *= p.dims[r];
-  p.du = p.dims[p.q];
-  for (int r = p.q + 1; r < b.rank; ++r) nbatch *= p.dims[r];
-  // about square; a short side is covered whole and the other takes what is
-  // left of cap; equal parts, so that no tile is a sliver
-  uint32_t side = 24;
-  while ((side + 8) * (side + 9) <= cap && side < 64) side += 8;
-  uint32_t tv = std::min(p.dv, side), tu = cap / (tv | 1);
-  if (p.du < tu) {
-    tu = p.du;
-    tv = std::min<uint32_t>((cap / tu - 1) | 1, kPermTileRows);
-  } else if (tv == side) {
-    tu = side;
-  }
-  tv = std::min(tv, p.dv);
-  p.tiles_u = (p.du + tu - 1) / tu;
-  p.tiles_v = (p.dv + tv - 1) / tv;
-  p.tu = (p.du + p.tiles_u - 1) / p.tiles_u;
-  p.tv = (p.dv + p.tiles_v - 1) / p.tiles_v;
-  *out = p;
-  *tiles = static_cast<int64_t>(p.tiles_u) * p.tiles_v * nbatch;
-  return true;
 }
 
 cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items, int64_t n,

@@ -333,7 +333,7 @@ cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* 
 // The same through shared-memory tiles, for items that neither pad nor crop.
 // perm_tile_item makes an item's geometry and its number of tiles, or returns
 // false when it does not qualify (limits below the output extents, 2^31
-// elements or more); cap = elements of shared memory per tile (perm_tile_cap:
+// elements or more, no axis to read contiguously); cap = elements of shared memory per tile (perm_tile_cap:
 // 1056 to 4160 by the elements moved, so that small operands make enough tiles
 // for the chip).  The caller sets tile_begin = tiles before the item; total =
 // all tiles.
@@ -343,8 +343,60 @@ struct PermTileItem {
   uint32_t dv, du, tv, tu, tiles_u, tiles_v;
   uint32_t dims[kMaxRank], strides[kMaxRank];
 };
-uint32_t perm_tile_cap(int64_t elems);
-bool perm_tile_item(const BlockPerm& it, uint32_t cap, PermTileItem* out, int64_t* tiles);
+constexpr int kPermTileElems = 64 * 65;  // largest cap
+constexpr int kPermTileRows = 1024;      // largest tv
+inline uint32_t perm_tile_cap(int64_t elems) {
+  const int64_t c = elems / (148LL * 12);
+  return static_cast<uint32_t>(c < 1056 ? 1056 : c > kPermTileElems ? kPermTileElems : c);
+}
+
+inline bool perm_tile_item(const BlockPerm& b, uint32_t cap, PermTileItem* out, int64_t* tiles) {
+  if (b.len <= 0 || b.len >= (int64_t{1} << 31) || b.rank < 1) return false;
+  PermTileItem p{};
+  p.src_off = b.src_off;
+  p.dst_off = b.dst_off;
+  p.rank = b.rank;
+  p.q = b.rank - 1;
+  for (int r = b.rank - 1; r >= 0; --r) {
+    if (b.in_lim[r] < b.out_dims[r] || (b.out_dims[r] > 1 && b.in_strides[r] >= (int64_t{1} << 31))) return false;
+    p.dims[r] = static_cast<uint32_t>(b.out_dims[r]);
+    p.strides[r] = b.out_dims[r] > 1 ? static_cast<uint32_t>(b.in_strides[r]) : 0;
+    if (b.in_strides[r] == 1 && b.out_dims[r] > 1) p.q = r;
+  }
+  if (b.len > 1 && (b.out_dims[p.q] == 1 || b.in_strides[p.q] != 1)) return false;
+  // output axis 0 contiguous in the source too (crops, outer-axis reorders):
+  // a tile would hold one row of axis 0, so only long rows qualify
+  if (p.q == 0 && p.dims[0] < 256 && b.len > p.dims[0]) return false;
+  // a tile row's source offset is a 32-bit sum; the strides may be those of a
+  // longer block, of which these are a part
+  int64_t reach = 0;
+  for (int r = 0; r < p.q; ++r) reach += (b.out_dims[r] - 1) * static_cast<int64_t>(p.strides[r]);
+  if (reach >= (int64_t{1} << 31)) return false;
+  int64_t nbatch = 1;
+  p.dv = 1;
+  for (int r = 0; r < p.q; ++r) p.dv *= p.dims[r];
+  p.du = p.dims[p.q];
+  for (int r = p.q + 1; r < b.rank; ++r) nbatch *= p.dims[r];
+  // about square; a short side is covered whole and the other takes what is
+  // left of cap; equal parts, so that no tile is a sliver
+  uint32_t side = 24;
+  while ((side + 8) * (side + 9) <= cap && side < 64) side += 8;
+  uint32_t tv = std::min(p.dv, side), tu = cap / (tv | 1);
+  if (p.du < tu) {
+    tu = p.du;
+    tv = std::min<uint32_t>((cap / tu - 1) | 1, kPermTileRows);
+  } else if (tv == side) {
+    tu = side;
+  }
+  tv = std::min(tv, p.dv);
+  p.tiles_u = (p.du + tu - 1) / tu;
+  p.tiles_v = (p.dv + tv - 1) / tv;
+  p.tu = (p.du + p.tiles_u - 1) / p.tiles_u;
+  p.tv = (p.dv + p.tiles_v - 1) / p.tiles_v;
+  *out = p;
+  *tiles = static_cast<int64_t>(p.tiles_u) * p.tiles_v * nbatch;
+  return true;
+}
 cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTileItem* d_items, int64_t n,
                                     int64_t total, uint32_t cap, cudaStream_t s);
 // The same for items whose out_dims[0] has in_strides[0] == 1 (one warp per
