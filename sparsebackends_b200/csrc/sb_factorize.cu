@@ -93,9 +93,71 @@ __global__ void __launch_bounds__(kFacThreads)
 // warp reduction, a square root, a division and the update per reflector, 1.35 us
 // each at 256 rows.  The 256 x 160 factorisation took 2.0 ms as a launch per
 // reflector and one per update (483), and takes 0.34 ms in 13 launches.
+// The products are those of x, scaled afterwards: they stay in range and meet
+// no infinity with x's zeros while every magnitude is at most 2^400; a panel
+// that holds a larger one, an infinity or NaN goes to house_panel_plain.
 constexpr int kPanelThreads = 512;
 constexpr int kPanelMax = 32;    // reflectors of a panel
 constexpr int kPanelRows = 1024;
+
+// The panel in memory, a warp per column, with products of v over the rows below
+// the pivot only and no step for a reflector with tau = 0, so that infinities
+// and NaN reach what the reflectors one at a time let them reach.
+__device__ __noinline__ void house_panel_plain(double* M, int64_t ld, int rows, int p0, int pb, double* T, double* taus,
+                                               double (*z)[kPanelMax + 1], double (*ts)[kPanelMax + 1]) {
+  const int warp = static_cast<int>(threadIdx.x) >> 5, lane = static_cast<int>(threadIdx.x) & 31;
+  auto column = [&](int c) { return M + p0 + static_cast<int64_t>(p0 + c) * ld; };
+  auto product = [&](const double* a, const double* b, int r0) {  // over rows [r0, rows)
+    double s = 0.0;
+    for (int r = r0 + lane; r < rows; r += 32) s = __fma_rn(a[r], b[r], s);
+    for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+    return s;
+  };
+  for (int j = 0; j < pb; ++j) {
+    double* const v = column(j);
+    const double alpha = v[j], xn2 = product(v, v, j + 1);
+    double tau = 0.0, beta = alpha, scal = 0.0;
+    if (xn2 != 0.0) {
+      const double nrm = sqrt(__fma_rn(alpha, alpha, xn2));
+      beta = alpha >= 0.0 ? -nrm : nrm;
+      tau = (beta - alpha) / beta;
+      scal = 1.0 / (alpha - beta);
+    }
+    __syncthreads();
+    if (warp == (j & 15)) {
+      if (scal != 0.0)
+        for (int r = j + 1 + lane; r < rows; r += 32) v[r] = __dmul_rn(v[r], scal);
+      if (lane == 0) {
+        v[j] = beta;
+        taus[j] = tau;
+      }
+    }
+    __syncthreads();
+    for (int c = warp; c < pb; c += kPanelThreads / 32) {
+      if (c == j || (c > j && tau == 0.0)) continue;
+      double* const col = column(c);
+      const double cj = col[j], d = __dadd_rn(cj, product(v, col, j + 1)), w = __dmul_rn(tau, d);
+      if (c < j) {
+        if (lane == 0) z[c][j] = d;
+        continue;
+      }
+      __syncwarp();
+      if (lane == 0) col[j] = __dsub_rn(cj, w);
+      for (int r = j + 1 + lane; r < rows; r += 32) col[r] = __fma_rn(-v[r], w, col[r]);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      double s = 0.0;
+      for (int i = lane; i < j; ++i)
+        if (taus[i] != 0.0) s = __fma_rn(ts[lane][i], z[i][j], s);
+      if (lane < j) ts[lane][j] = taus[lane] != 0.0 && tau != 0.0 ? -__dmul_rn(tau, s) : 0.0;
+      else if (lane == j) ts[j][j] = tau;
+      __syncwarp();
+    }
+  }
+  if (warp == 0)
+    for (int j = 0; j < pb; ++j) T[lane + kPanelMax * j] = lane <= j ? ts[lane][j] : 0.0;
+}
 template <int RPL, int CPW>
 __global__ void __launch_bounds__(kPanelThreads, 1)
     k_house_panel(double* __restrict__ M, int64_t ld, int m, int p0, int pb, double* __restrict__ T) {
@@ -113,6 +175,15 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
     const double* col = M + p0 + static_cast<int64_t>(p0 + c) * ld;
 #pragma unroll
     for (int i = 0; i < RPL; ++i) a[q][i] = c < pb && lane + 32 * i < rows ? col[lane + 32 * i] : 0.0;
+  }
+  bool odd = false;
+#pragma unroll
+  for (int q = 0; q < CPW; ++q)
+#pragma unroll
+    for (int i = 0; i < RPL; ++i) odd = odd || !(fabs(a[q][i]) <= 0x1p400);
+  if (__syncthreads_or(odd)) {
+    house_panel_plain(M, ld, rows, p0, pb, T, taus, z, ts);
+    return;
   }
   // T(0:j, j) = -tau_j * T(0:j, 0:j) * z(0:j, j), T(j, j) = tau_j, by one warp
   auto t_column = [&](int j) {
@@ -210,7 +281,8 @@ __global__ void __launch_bounds__(kPanelThreads, 1)
 // x <- (I - V op(T) V^T) x for one column x (rows [p0, m), in shared memory),
 // V the panel's reflectors in M (1 on the diagonal, 0 above).  A warp takes
 // the dot products of a stride of the reflectors; V is read from L2 twice,
-// coalesced along its columns.
+// coalesced along its columns.  A product that is not finite is taken again over
+// the rows from the pivot on, and T's zeros (reflectors with tau = 0) skip it.
 __device__ __forceinline__ void apply_block(const double* __restrict__ M, int64_t ld, int m, int p0, int pb,
                                             const double* __restrict__ T, bool trans, double* x, double* w, double* y) {
   const int tid = static_cast<int>(threadIdx.x), warp = tid >> 5, lane = tid & 31, rows = m - p0;
@@ -233,10 +305,28 @@ __device__ __forceinline__ void apply_block(const double* __restrict__ M, int64_
     for (int o = 16; o > 0; o >>= 1) s4[q] = __dadd_rn(s4[q], __shfl_xor_sync(0xffffffffu, s4[q], o));
     if (lane == 0) w[kPer * warp + q] = s4[q];
   }
-  __syncthreads();
+  bool odd = false;
+#pragma unroll
+  for (int q = 0; q < kPer; ++q) odd = odd || !isfinite(s4[q]);
+  odd = __syncthreads_or(odd);
+  if (odd) {
+    for (int j = kPer * warp; j < kPer * warp + kPer && j < pb; ++j) {
+      double s = 0.0;
+      for (int r = j + lane; r < rows; r += 32)
+        s = __fma_rn(r > j ? M[p0 + r + static_cast<int64_t>(p0 + j) * ld] : 1.0, x[r], s);
+      for (int o = 16; o > 0; o >>= 1) s = __dadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+      if (lane == 0) w[j] = s;
+    }
+    __syncthreads();
+  }
   if (tid < pb) {
     double s = 0.0;
-    if (trans)
+    if (odd)
+      for (int i = trans ? 0 : tid; i < (trans ? tid + 1 : pb); ++i) {
+        const double t = T[trans ? i + kPanelMax * tid : tid + kPanelMax * i];
+        if (t != 0.0) s = __fma_rn(t, w[i], s);
+      }
+    else if (trans)
       for (int i = 0; i <= tid; ++i) s = __fma_rn(T[i + kPanelMax * tid], w[i], s);
     else
       for (int j = tid; j < pb; ++j) s = __fma_rn(T[tid + kPanelMax * j], w[j], s);
@@ -270,17 +360,18 @@ __global__ void __launch_bounds__(kFacThreads)
   for (int r = threadIdx.x; r < m - p0; r += kFacThreads) col[r] = x[r];
 }
 
-// Column blockIdx.x of Q = H_0 H_1 ... H_{k-1} restricted to k columns: the
-// panels of nb reflectors applied to the unit vector, last one first.
+// Column blockIdx.x = c of Q = H_0 H_1 ... H_{k-1} restricted to k columns: the
+// panels of nb reflectors applied to the unit vector, last one first; the
+// reflectors behind the c-th leave it alone.
 __global__ void __launch_bounds__(kFacThreads)
-    k_house_q(const double* __restrict__ M, int64_t ld, int m, int k, int nb, const double* __restrict__ T,
+    k_house_q(const double* __restrict__ M, int64_t ld, int m, int nb, const double* __restrict__ T,
               double* __restrict__ Q) {
   __shared__ double x[kPanelRows], w[kPanelMax], y[kPanelMax];
   const int c = static_cast<int>(blockIdx.x);
   for (int r = threadIdx.x; r < m; r += kFacThreads) x[r] = r == c ? 1.0 : 0.0;
   __syncthreads();
   for (int p = c / nb; p >= 0; --p)
-    apply_block(M, ld, m, p * nb, min(nb, k - p * nb), T + static_cast<int64_t>(p) * kPanelMax * kPanelMax, false,
+    apply_block(M, ld, m, p * nb, min(nb, c + 1 - p * nb), T + static_cast<int64_t>(p) * kPanelMax * kPanelMax, false,
                 x + p * nb, w, y);
   for (int r = threadIdx.x; r < m; r += kFacThreads) Q[r + static_cast<int64_t>(c) * m] = x[r];
 }
@@ -470,7 +561,7 @@ cudaError_t launch_householder_form_q(const double* M, int64_t m, int64_t k, con
                                       cudaStream_t s, int64_t* launches) {
   if (m <= 0 || k <= 0) return cudaSuccess;
   if (const int nb = householder_panel(m); nb > 0) {
-    k_house_q<<<static_cast<unsigned>(k), kFacThreads, 0, s>>>(M, m, static_cast<int>(m), static_cast<int>(k), nb, tau, Q);
+    k_house_q<<<static_cast<unsigned>(k), kFacThreads, 0, s>>>(M, m, static_cast<int>(m), nb, tau, Q);
     ++*launches;
     return cudaGetLastError();
   }
