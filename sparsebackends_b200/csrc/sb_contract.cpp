@@ -21,14 +21,12 @@
 //                              contract_aliased_shared.jl
 //   bs_bs_to_dense()           contract_bs_bs.jl:736-754
 #include <algorithm>
-#include <array>
 #include <climits>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <tuple>
 #include <numeric>
-#include <queue>
 #include <unordered_map>
 
 #include "sb_internal.hpp"
@@ -586,8 +584,7 @@ struct GemmPlan {
     // together (blocks with 3 to 20 pairs, us, key order and this: 64x64x128 189
     // and 168, 128x128x256 293 and 260, 32x256x512 353 and 299, 256x256x128 361
     // and 320, 1024x512x512 1069 and 1026, 64x64x1024 beyond L2 1625 and 1562).
-    std::stable_sort(cbs.begin(), cbs.end(),
-                     [&](const GemmCBlock& a, const GemmCBlock& b) { return ktiles(pairs, a) > ktiles(pairs, b); });
+    heavy_first(cbs, pairs);
     int64_t ntiles = 0;
     for (auto& c : cbs) {
       const int64_t mt = (c.M + bm - 1) / bm, nt = (c.N + bn - 1) / bn;
@@ -1190,6 +1187,16 @@ struct GemmPlan {
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
     if (bytes <= 2.0 * l2) return false;
+    // the operands' spans first (27 000 pairs of small operands: 0.2 ms less)
+    int64_t x0 = INT64_MAX, x1 = 0, y0 = INT64_MAX, y1 = 0;
+    for (const GemmCBlock& c : cbs)
+      for (int p = c.pair_begin; p < c.pair_end; ++p) {
+        x0 = std::min(x0, pairs[p].x_off);
+        y0 = std::min(y0, pairs[p].y_off);
+        x1 = std::max(x1, pairs[p].x_off + static_cast<int64_t>(c.M) * pairs[p].K);
+        y1 = std::max(y1, pairs[p].y_off + static_cast<int64_t>(c.N) * pairs[p].K);
+      }
+    if (8.0 * static_cast<double>(x1 - x0) + 8.0 * static_cast<double>(y1 - y0) <= 2.0 * l2) return false;
     std::unordered_map<int64_t, int64_t> x, y;  // distinct operand blocks
     for (const GemmCBlock& c : cbs)
       for (int p = c.pair_begin; p < c.pair_end; ++p) {
@@ -1232,10 +1239,34 @@ struct GemmPlan {
   // launching nothing, when that saves < 3% of the padded 64x64 work.
   static int edge_rows(int shape) { return shape == 2 ? 32 : shape == 4 ? 48 : 64; }
   static int edge_cols(int shape) { return shape == 1 ? 32 : shape == 3 ? 48 : 64; }
-  static int64_t ktiles(const std::vector<GemmPair>& pr, const GemmCBlock& c) {
-    int64_t kt = 0;
-    for (int p = c.pair_begin; p < c.pair_end; ++p) kt += (static_cast<int64_t>(pr[p].K) + 15) / 16;
-    return kt;
+  // Blocks by falling number of k-tiles, equal ones in their order.  The k-tiles
+  // are counted once per block and the blocks dropped into one place per count:
+  // with a comparison sort that counted them anew, the plan of 10 000 blocks with
+  // 9 pairs each took 15.8 ms instead of 13.3.
+  static void heavy_first(std::vector<GemmCBlock>& blocks, const std::vector<GemmPair>& pr) {
+    std::vector<int64_t> kt(blocks.size(), 0);
+    bool sorted = true;
+    for (size_t i = 0; i < blocks.size(); ++i) {
+      for (int p = blocks[i].pair_begin; p < blocks[i].pair_end; ++p) kt[i] += (static_cast<int64_t>(pr[p].K) + 15) / 16;
+      sorted = sorted && (i == 0 || kt[i - 1] >= kt[i]);
+    }
+    if (sorted) return;
+    std::vector<int64_t> at(blocks.size());  // where each block goes
+    const int64_t most = *std::max_element(kt.begin(), kt.end());
+    if (most <= 16 * static_cast<int64_t>(blocks.size()) + 4096) {
+      std::vector<int64_t> next(most + 2, 0);  // next[most - kt + 1]: blocks with kt k-tiles
+      for (int64_t k : kt) ++next[most - k + 1];
+      std::partial_sum(next.begin(), next.end(), next.begin());
+      for (size_t i = 0; i < at.size(); ++i) at[i] = next[most - kt[i]]++;
+    } else {
+      std::vector<int64_t> order(blocks.size());
+      std::iota(order.begin(), order.end(), 0);
+      std::stable_sort(order.begin(), order.end(), [&](int64_t a, int64_t b) { return kt[a] > kt[b]; });
+      for (size_t i = 0; i < order.size(); ++i) at[order[i]] = static_cast<int64_t>(i);
+    }
+    std::vector<GemmCBlock> out(blocks.size());
+    for (size_t i = 0; i < at.size(); ++i) out[at[i]] = blocks[i];
+    blocks.swap(out);
   }
   bool prepare_edges(Ctx* ctx, GemmLaunch& g, double flops, double bytes) {
     const bool xT = g.xT, yT = g.yT;
@@ -1306,9 +1337,7 @@ struct GemmPlan {
       // Heavy C blocks first: CTAs start in this order, so the last ones to
       // run are the short ones (psi*L of H_eff, us, key order and this: chi =
       // 256 19.2 and 17.9, 400 41 and 37, 700 108 and 101).
-      std::stable_sort(sc.begin(), sc.end(), [&](const GemmCBlock& a, const GemmCBlock& b) {
-        return ktiles(ep, a) > ktiles(ep, b);
-      });
+      heavy_first(sc, ep);
       renumber();
     }
     if (kt_avg >= 64) {
