@@ -310,34 +310,44 @@ __global__ void k_copy_small_blocks(const double* __restrict__ src, double* __re
   for (int64_t e = threadIdx.x & 31; e < it.len; e += 32) dst[it.dst_off + e] = src[it.src_off + e];
 }
 
+// Gather, kPer elements per thread.
+template <int kPer>
 __global__ void k_perm_blocks(const double* __restrict__ src, double* __restrict__ dst,
                               const BlockPerm* __restrict__ items, int64_t n) {
   for (int64_t b = blockIdx.y; b < n; b += gridDim.y) {
     const BlockPerm& it = items[b];
     if (it.len < (int64_t{1} << 31)) {
-      // a block below 2^31 elements: 32-bit indices, divided by multiplication;
-      // four elements per thread, their loads in flight together.  With the
-      // divisions in hardware the index work bound it: cropping the zero-padded
-      // T3 of a chi = 1023 H_eff (rows of 12 to 14) took 181 us, now 107.
-      constexpr int kPer = 4;
+      // a block below 2^31 elements: 32-bit indices, divided by multiplication,
+      // an axis' descriptor read once for a thread's elements, whose loads are in
+      // flight together.  With the divisions in hardware the index work bound it:
+      // cropping the zero-padded T3 of a chi = 1023 H_eff (rows of 12 to 14) took
+      // 181 us, now 107.
       const int64_t stride = static_cast<int64_t>(gridDim.x) * blockDim.x;
       for (int64_t e0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e0 < it.len; e0 += kPer * stride) {
-        double v[kPer];
+        uint32_t e[kPer];
+        int64_t so[kPer];
+        bool in[kPer];
 #pragma unroll
         for (int q = 0; q < kPer; ++q) {
           const int64_t e1 = e0 + q * stride;
-          uint32_t e = static_cast<uint32_t>(e1 < it.len ? e1 : 0);
-          int64_t so = it.src_off;
-          bool in = e1 < it.len;
-          for (int r = 0; r < it.rank; ++r) {
-            const uint32_t d = static_cast<uint32_t>(it.out_dims[r]);
-            const uint32_t next = (__umulhi(e, it.div_mul[r]) + e) >> it.div_shift[r], c = e - next * d;
-            e = next;
-            in = in && c < it.in_lim[r];
-            so += static_cast<int64_t>(c) * it.in_strides[r];
-          }
-          v[q] = in ? src[so] : 0.0;
+          in[q] = e1 < it.len;
+          e[q] = static_cast<uint32_t>(in[q] ? e1 : 0);
+          so[q] = it.src_off;
         }
+        for (int r = 0; r < it.rank; ++r) {
+          const uint32_t d = static_cast<uint32_t>(it.out_dims[r]), mul = it.div_mul[r], shift = it.div_shift[r];
+          const int64_t lim = it.in_lim[r], st = it.in_strides[r];
+#pragma unroll
+          for (int q = 0; q < kPer; ++q) {
+            const uint32_t next = (__umulhi(e[q], mul) + e[q]) >> shift, c = e[q] - next * d;
+            e[q] = next;
+            in[q] = in[q] && c < lim;
+            so[q] += static_cast<int64_t>(c) * st;
+          }
+        }
+        double v[kPer];
+#pragma unroll
+        for (int q = 0; q < kPer; ++q) v[q] = in[q] ? src[so[q]] : 0.0;
 #pragma unroll
         for (int q = 0; q < kPer; ++q)
           if (e0 + q * stride < it.len) dst[it.dst_off + e0 + q * stride] = v[q];
@@ -466,9 +476,24 @@ __global__ void __launch_bounds__(256, 6)
     __syncthreads();
     const uint32_t pitch = tv | 1;  // odd: no bank conflicts along u or along v
     const double* s0 = src + sb;
-    for (uint32_t v = warp; v < nv; v += 8) {
-      const double* row = s0 + row_off[v];
-      for (uint32_t u = lane; u < nu; u += 32) cp_async8(&ptile[u * pitch + v], row + u);
+    if (nu < 32) {  // rows shorter than a warp: their elements in a row, 256 at a time
+      uint32_t v = threadIdx.x / nu, u = threadIdx.x % nu;
+      const uint32_t sv = 256 / nu, su = 256 % nu;
+#pragma unroll 4
+      while (v < nv) {
+        cp_async8(&ptile[u * pitch + v], s0 + row_off[v] + u);
+        v += sv;
+        u += su;
+        if (u >= nu) {
+          u -= nu;
+          ++v;
+        }
+      }
+    } else {
+      for (uint32_t v = warp; v < nv; v += 8) {
+        const double* row = s0 + row_off[v];
+        for (uint32_t u = lane; u < nu; u += 32) cp_async8(&ptile[u * pitch + v], row + u);
+      }
     }
     // element i of the tile: u = i / nv, v = i % nv, advanced without dividing again
     uint32_t u = threadIdx.x / nv, v = threadIdx.x % nv;
@@ -783,9 +808,13 @@ cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTi
 cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* d_items, int64_t n, int64_t max_len,
                                cudaStream_t s) {
   if (n <= 0 || max_len <= 0) return cudaSuccess;
-  dim3 grid(grid_for(max_len), static_cast<unsigned>(n < 65535 ? n : 65535));
-  if ((int64_t)grid.x * grid.y > 148LL * 64) grid.x = static_cast<unsigned>(std::max<int64_t>(1, 148LL * 64 / grid.y));
-  k_perm_blocks<<<grid, kThreads, 0, s>>>(src, dst, d_items, n);
+  const int64_t gy = std::min<int64_t>(n, 65535), quarter = grid_for(max_len, 4 * kThreads);
+  // four elements per thread once that leaves eight CTAs per SM
+  const bool wide = quarter * gy >= 148LL * 8;
+  const int64_t gx = std::min<int64_t>(wide ? quarter : grid_for(max_len), std::max<int64_t>(1, 148LL * 64 / gy));
+  const dim3 grid(static_cast<unsigned>(gx), static_cast<unsigned>(gy));
+  if (wide) k_perm_blocks<4><<<grid, kThreads, 0, s>>>(src, dst, d_items, n);
+  else k_perm_blocks<1><<<grid, kThreads, 0, s>>>(src, dst, d_items, n);
   return cudaGetLastError();
 }
 
@@ -919,7 +948,7 @@ __global__ void __launch_bounds__(kThreads)
       d[r] = b.dims[r];
       len *= d[r];
       m[r] = 0;
-      sh[r] = d[r] <= 1 ? 0 : 32 - __clz(d[r] - 1);  // as set_divisors
+      sh[r] = d[r] <= 1 ? 0 : 32 - __clz(d[r] - 1);  // as Divisors
       mul[r] = static_cast<uint32_t>((((uint64_t{1} << sh[r]) - d[r]) << 32) / d[r] + 1);
     }
     const uint32_t e0 = static_cast<uint32_t>((w - b.task_begin) * budget);

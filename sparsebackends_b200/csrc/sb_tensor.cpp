@@ -251,11 +251,16 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
   // which is also the quicker one on small operands, where a tile's two
   // dependent phases cost more than they save (11 000 elements: 6.6 to 8.0 us
   // against 7.7 to 8.8; 215 000: 11.5 to 11.9 against 8.8 to 10.3; 89 000: the
-  // whole call 19.9 us against 20.6)
+  // whole call 19.9 us against 20.6), where the geometry leaves tiles below half
+  // their capacity (60 blocks (6, 700, 50) to (50, 6, 700), 50 x 6 tiles: 214 us,
+  // gather 86; 30 x 31: 88, 77; 2 x 48: 7300, 72), and where rows of one or two
+  // elements are most of the work (400 of (2, 50, 700) reversed: 260, 173; rows
+  // of three: 70, 83)
   std::vector<PermTileItem> pt;
-  int64_t tiles = 0;
-  const uint32_t cap = perm_tile_cap(static_cast<int64_t>(bytes / 16));
-  if (!rows && bytes >= 16.0 * (1 << 17)) {
+  int64_t tiles = 0, narrow = 0;
+  const int64_t moved = static_cast<int64_t>(bytes / 16);
+  const uint32_t cap = perm_tile_cap(moved);
+  if (!rows && moved >= 1 << 17) {
     pt.resize(items.size());
     for (size_t i = 0; i < items.size(); ++i) {
       int64_t t = 0;
@@ -265,7 +270,9 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
       }
       pt[i].tile_begin = tiles;
       tiles += t;
+      if (pt[i].du < 3) narrow += items[i].len;
     }
+    if (2 * moved < cap * tiles || 2 * narrow > moved) pt.clear();
   }
   if (!pt.empty()) {
     DevBuf d = upload(ctx, pt);
@@ -275,7 +282,8 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
     ctx->note_launch();
     return;
   }
-  for (auto& it : items) set_divisors(it);
+  Divisors div;
+  for (auto& it : items) div.set(it);
   DevBuf d = upload(ctx, items);
   ProfScope ps(ctx, PROF_PERMUTE, 0.0, bytes);
   if (rows)
@@ -286,10 +294,14 @@ static void perm_blocks(Ctx* ctx, const double* src, double* dst, std::vector<Bl
   ctx->note_launch();
 }
 
-static BlockPerm make_block_perm(int64_t src_off, int64_t dst_off, const std::vector<int64_t>& out_dims,
-                                 const std::vector<int64_t>& in_strides, const std::vector<int64_t>& in_lim) {
+// Appends an item to the list, written in place (400 blocks through a temporary
+// and vectors of their own: 25 us of a call's host time).
+static void add_block_perm(std::vector<BlockPerm>& items, int64_t src_off, int64_t dst_off,
+                           const std::vector<int64_t>& out_dims, const std::vector<int64_t>& in_strides,
+                           const std::vector<int64_t>& in_lim) {
   require(out_dims.size() <= static_cast<size_t>(kMaxRank), SB_ERR_INVALID_ARG, "tail rank too large");
-  BlockPerm b{};
+  items.emplace_back();
+  BlockPerm& b = items.back();
   b.src_off = src_off;
   b.dst_off = dst_off;
   b.len = 1;
@@ -300,7 +312,6 @@ static BlockPerm make_block_perm(int64_t src_off, int64_t dst_off, const std::ve
     b.in_lim[r] = in_lim[r];
     b.len *= out_dims[r];
   }
-  return b;
 }
 
 // The uniform (zero-padded) blocks of A, in key order, written to dst
@@ -315,15 +326,16 @@ void bs_pad_into(Ctx* ctx, const Tensor& A, double* dst) {
   const int P = A.P();
   std::vector<int64_t> od(A.dims.begin() + P, A.dims.end());
   std::vector<BlockPerm> items;
+  items.reserve(A.nkeys);
+  std::vector<int64_t> st(A.n2), lim(A.n2);
   for (int64_t i = 0; i < A.nkeys; ++i) {
-    std::vector<int64_t> st(A.n2), lim(A.n2);
     int64_t acc = 1;
     for (int t = 0; t < A.n2; ++t) {
       st[t] = acc;
       lim[t] = A.block_dim(i, t);
       acc *= lim[t];
     }
-    items.push_back(make_block_perm(A.block_off(i), i * blk, od, st, lim));
+    add_block_perm(items, A.block_off(i), i * blk, od, st, lim);
   }
   perm_blocks(ctx, A.payload(), dst, items);
 }
@@ -439,8 +451,8 @@ TensorPtr bs_to_ragged(Ctx* ctx, const Tensor& A, const std::vector<int64_t>& bd
   else out->data = DevBuf(ctx, need);
   std::vector<BlockPerm> items, checks;
   items.reserve(A.nkeys);
+  std::vector<int64_t> od(A.n2), st(A.n2), full(A.n2);
   for (int64_t i = 0; i < A.nkeys; ++i) {
-    std::vector<int64_t> od(A.n2), st(A.n2), full(A.n2);
     int64_t acc = 1;
     for (int t = 0; t < A.n2; ++t) {
       od[t] = bd[i * A.n2 + t];
@@ -448,8 +460,8 @@ TensorPtr bs_to_ragged(Ctx* ctx, const Tensor& A, const std::vector<int64_t>& bd
       st[t] = acc;
       acc *= full[t];
     }
-    items.push_back(make_block_perm(A.block_off(i), out->boff[i], od, st, od));
-    if (check_zero) checks.push_back(make_block_perm(A.block_off(i), 0, full, st, od));
+    add_block_perm(items, A.block_off(i), out->boff[i], od, st, od);
+    if (check_zero) add_block_perm(checks, A.block_off(i), 0, full, st, od);
   }
   if (check_zero && !checks.empty()) {
     int64_t mx = 0;
@@ -511,8 +523,8 @@ TensorPtr bs_permute(Ctx* ctx, const Tensor& A, const std::vector<int>& perm) {
     } else {
       std::vector<BlockPerm> items;
       items.reserve(n);
+      std::vector<int64_t> sst(A.n2), od(A.n2), is(A.n2);
       for (int64_t i = 0; i < n; ++i) {
-        std::vector<int64_t> sst(A.n2), od(A.n2), is(A.n2);
         int64_t acc = 1;
         for (int t = 0; t < A.n2; ++t) {
           sst[t] = acc;
@@ -522,7 +534,7 @@ TensorPtr bs_permute(Ctx* ctx, const Tensor& A, const std::vector<int>& perm) {
           od[r] = out->bdims[i * A.n2 + r];
           is[r] = sst[perm[P + r] - 1 - P];
         }
-        items.push_back(make_block_perm(A.block_off(p[i]), out->boff[i], od, is, od));
+        add_block_perm(items, A.block_off(p[i]), out->boff[i], od, is, od);
       }
       perm_blocks(ctx, A.payload(), out->data.d(), items);
     }
