@@ -603,7 +603,7 @@ struct GemmPlan {
       kt_max = std::max(kt_max, kt);
     }
     kt_avg = ntiles ? kt_avg / ntiles : 0;
-    const int splitk = choose_splitk(ctx, ntiles, kt_avg, kt_max);
+    const auto [splitk, partials] = choose_splitk(ctx, ntiles, kt_avg, kt_max, bytes);
     std::snprintf(g.desc, sizeof(g.desc), "tiled %dx%d sk%d", bm, bn, splitk);
     g.kind = GemmLaunch::TILED;
     g.dc = upload(ctx, cbs);
@@ -614,7 +614,7 @@ struct GemmPlan {
     g.bm = bm;
     g.bn = bn;
     g.splitk = splitk;
-    g.split_partials = splitk > 1 && beyond_l2(ctx, bytes);
+    g.split_partials = partials;
     g.flops = flops;
     g.bytes = bytes;
     return g;
@@ -1176,13 +1176,8 @@ struct GemmPlan {
     return any;
   }
 
-  // Whether a split launch leaves partial tiles in memory, its segments
-  // outermost, instead of summing them inside clusters: when the operands take
-  // more than twice L2, so that CTAs running at the same time should work on one
-  // K range of many tiles (R*T3 of H_eff at chi = 2048, 900 MB: 2010 us in
-  // clusters, 1911 with partial tiles; the whole apply, us, clusters and partial
-  // tiles: chi = 1024 788 and 797, 1200 1193 and 1184, 1400 1662 and 1635, 2048
-  // 4521 and 4416).  bytes: every pair's blocks counted anew, an upper bound.
+  // Whether the operands of a launch take more than twice L2.  bytes: every
+  // pair's blocks counted anew, an upper bound.
   bool beyond_l2(Ctx* ctx, double bytes) const {
     int l2 = 0;
     cudaDeviceGetAttribute(&l2, cudaDevAttrL2CacheSize, ctx->device);
@@ -1209,27 +1204,46 @@ struct GemmPlan {
     return distinct > 2.0 * l2;
   }
 
-  // Split-K factor for ntiles tiles with kt_avg k-tiles on average and kt_max
-  // at most (a power of two): split while the tiles
-  // fill less than ~6 waves of 148 SMs x 4 CTAs and every segment keeps >= 32
-  // k-tiles (the shorter CTAs balance the uneven K loops), and, when there are
-  // fewer CTAs than 4 per SM, as long as the longest K loop keeps >= 4 k-tiles
-  // per segment: one SM takes 0.5 us per 64x64x16 k-tile, so a few long
-  // tiles leave the chip idle (R*T3 of H_eff, us, before and after: chi = 256,
-  // 42 tiles of up to 130 k-tiles, 121 and 27; chi = 400 122 and 50; chi = 512
-  // 99 and 71; chi = 700 165 and 131; chi = 1024 332 and 318).  16 segments only
-  // while 8 leave SMs without a CTA (a 64x64 block with K = 8192, us, 8 and 16
-  // segments: 43 and 25; 18 tiles of K = 16384 151 and 130; 24 of K = 8192 94
-  // and 94; 32 of K = 8192 95 and 107).
-  static int choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg, int64_t kt_max) {
+  // Split-K of ntiles tiles with kt_avg k-tiles on average and kt_max at most.
+  //
+  // partials: the segments leave partial tiles in memory, segments outermost,
+  // instead of summing them inside clusters.  When the operands take more than
+  // twice L2, so that CTAs running at the same time work on one K range of many
+  // tiles (R*T3 of H_eff at chi = 2048, 900 MB: 2010 us in clusters, 1911 with
+  // partial tiles).  And when the loops are long enough to pay for the second
+  // launch: clusters start only where their CTAs fit at once, which leaves SMs
+  // idle (64x64 tiles, us, clusters and partial tiles: 25 with K = 16000 149 and
+  // 138, 36 with K = 24000 400 and 343, 64 with K = 12000 329 and 309; 128x32
+  // tiles: 64 with K = 5400 148 and 120, 100 with K = 12000 443 and 352; but 25
+  // with K = 2000 66 and 70, one with K = 24000 62 and 66).
+  //
+  // splitk (a power of two): split while the tiles fill less than ~6 waves of 148
+  // SMs x 4 CTAs and every segment keeps >= 32 k-tiles, 20 with partial tiles (the
+  // shorter CTAs balance the uneven K loops; 49 64x64 tiles with K = 8000, 8 and 16
+  // segments: 208 us and 199), and, when there are fewer CTAs than 4 per SM, as long as
+  // the longest K loop keeps >= 4 k-tiles per segment: one SM takes 0.5 us per
+  // 64x64x16 k-tile, so a few long tiles leave the chip idle (R*T3 of H_eff, us,
+  // before and after: chi = 256, 42 tiles of up to 130 k-tiles, 121 and 27; chi =
+  // 400 122 and 50; chi = 512 99 and 71; chi = 700 165 and 131; chi = 1024 332 and
+  // 318).  Clusters of 16 only while 8 leave SMs without a CTA (a 64x64 block with
+  // K = 8192, us, 8 and 16 segments: 43 and 25; 24 of K = 8192 94 and 94; 32 of K
+  // = 8192 95 and 107).
+  struct Split {
     int splitk = 1;
+    bool partials = false;
+  };
+  Split choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg, int64_t kt_max, double bytes) const {
+    Split r;
     const int64_t wave = 148 * 4;
-    const int cap = ntiles * kPortableCluster <= 148 ? kMaxSplitK : kPortableCluster;
-    while (splitk < cap && ((ntiles * splitk < 6 * wave && kt_avg / (2 * splitk) >= 32) ||
-                                   (ntiles * splitk < wave && kt_max / (2 * splitk) >= 4)))
-      splitk *= 2;
-    if (ctx->gemm_splitk > 0) splitk = std::min(ctx->gemm_splitk, kMaxSplitK);
-    return splitk;
+    r.partials = (kt_avg >= 256 && ntiles * kt_avg >= 12 * 256) || beyond_l2(ctx, bytes);
+    const int cap = r.partials || ntiles * kPortableCluster <= 148 ? kMaxSplitK : kPortableCluster;
+    const int least = r.partials ? 20 : 32;
+    while (r.splitk < cap && ((ntiles * r.splitk < 6 * wave && kt_avg / (2 * r.splitk) >= least) ||
+                              (ntiles * r.splitk < wave && kt_max / (2 * r.splitk) >= 4)))
+      r.splitk *= 2;
+    if (ctx->gemm_splitk > 0) r.splitk = std::min(ctx->gemm_splitk, kMaxSplitK);
+    r.partials = r.partials && r.splitk > 1;
+    return r;
   }
   // 64x64 tiles with the edges cut off: a column remainder N mod 64 of <= 32
   // or <= 48 (the whole block when N is that small) goes to 64x32 or 64x48
@@ -1349,7 +1363,7 @@ struct GemmPlan {
                        [](const GemmCBlock& a, const GemmCBlock& b) { return a.tshape < b.tshape; });
       renumber();
     }
-    const int splitk = choose_splitk(ctx, ntiles, kt_avg, kt_max);
+    const auto [splitk, partials] = choose_splitk(ctx, ntiles, kt_avg, kt_max, bytes);
     long long nshape[5] = {0, 0, 0, 0, 0};
     for (auto& b : sc) nshape[b.tshape] += static_cast<long long>(b.mtiles) * ((b.N + edge_cols(b.tshape) - 1) /
                                                                                 edge_cols(b.tshape));
@@ -1361,7 +1375,7 @@ struct GemmPlan {
     g.ncb = static_cast<int32_t>(sc.size());
     g.n = ntiles;
     g.splitk = splitk;
-    g.split_partials = splitk > 1 && beyond_l2(ctx, bytes);
+    g.split_partials = partials;
     g.flops = flops;
     g.bytes = bytes;
     return true;
