@@ -39,3 +39,16 @@ def test_crops_and_pads_through_the_gather(tail, kept, blocks):
     for i, f in enumerate(full):
         assert np.array_equal(got[(i + 1,)], f[tuple(slice(0, e) for e in kept)].reshape(-1, order="F"))
         assert np.array_equal(back[(i + 1,)], f.reshape(-1, order="F"))
+
+
+@pytest.mark.parametrize("length", [32, 33, 63, 64, 65, 255, 256, 257, 511, 513, 2047, 2048])
+def test_run_copies(length):
+    """Runs around a warp's batch of loads, whole and with a rest."""
+    import sparsebackends_b200 as sb
+    rng = np.random.Generator(np.random.PCG64(length))
+    v = [rng.standard_normal((length, 3, 5)) for _ in range(4)]
+    A = sb.NewBlockSparseSorted((4, length, 3, 5), 3, [(i + 1,) for i in range(4)], None,
+                                np.concatenate([x.reshape(-1, order="F") for x in v]))
+    got = sb.permutedims(A, [1, 2, 4, 3]).blocks_by_key()
+    for i, x in enumerate(v):
+        assert np.array_equal(got[(i + 1,)], np.transpose(x, (0, 2, 1)).reshape(-1, order="F")), i
