@@ -1215,7 +1215,11 @@ struct GemmPlan {
   // idle (64x64 tiles, us, clusters and partial tiles: 25 with K = 16000 149 and
   // 138, 36 with K = 24000 400 and 343, 64 with K = 12000 329 and 309; 128x32
   // tiles: 64 with K = 5400 148 and 120, 100 with K = 12000 443 and 352; but 25
-  // with K = 2000 66 and 70, one with K = 24000 62 and 66).
+  // with K = 2000 66 and 70, one with K = 24000 62 and 66).  Not beyond a tile
+  // per SM, where clusters find room (200 with K = 8000 513 and 512) and allocating
+  // the partial tiles, more than 77 MB, stalls calls that hold other temporaries
+  // (R*T3 of the zero-padded chi = 1023 H_eff, 208 tiles: the apply 1825 and 1913
+  // to 2240).
   //
   // splitk (a power of two): split while the tiles fill less than ~6 waves of 148
   // SMs x 4 CTAs and every segment keeps >= 32 k-tiles, 20 with partial tiles (the
@@ -1235,7 +1239,7 @@ struct GemmPlan {
   Split choose_splitk(Ctx* ctx, int64_t ntiles, int64_t kt_avg, int64_t kt_max, double bytes) const {
     Split r;
     const int64_t wave = 148 * 4;
-    r.partials = (kt_avg >= 256 && ntiles * kt_avg >= 12 * 256) || beyond_l2(ctx, bytes);
+    r.partials = (kt_avg >= 256 && ntiles * kt_avg >= 12 * 256 && ntiles <= 148) || beyond_l2(ctx, bytes);
     const int cap = r.partials || ntiles * kPortableCluster <= 148 ? kMaxSplitK : kPortableCluster;
     const int least = r.partials ? 20 : 32;
     while (r.splitk < cap && ((ntiles * r.splitk < 6 * wave && kt_avg / (2 * r.splitk) >= least) ||

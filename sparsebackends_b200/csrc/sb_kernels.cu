@@ -837,7 +837,7 @@ cudaError_t launch_perm_blocks(const double* src, double* dst, const BlockPerm* 
 
 // Smallest tail extents of every block that keep all its nonzero entries:
 // ext[b*n2 + r] = 1 + the largest axis-r coordinate of a nonzero element
-// (ext holds 1s on entry).  A block is a column-major matrix of d0 rows
+// (0 if there is none: ext holds 0s on entry).  A block is a column-major matrix of d0 rows
 // (axis 0) and cols columns (the other axes, flattened).  Work comes in warp
 // tasks of about `budget` elements, task_begin[b] .. task_begin[b+1] for block
 // b, in one of three forms fixed by (d0, cols): rows of one column split into

@@ -413,8 +413,8 @@ cudaError_t launch_perm_block_tiles(const double* src, double* dst, const PermTi
 cudaError_t launch_perm_block_rows(const double* src, double* dst, const BlockPerm* d_items, int64_t n,
                                    int64_t max_rows, cudaStream_t s);
 // ext[b*n2 + r] = smallest axis-r extent of block b (payload at d_off[b],
-// extents d_dims[b*n2 ..]) that keeps all its nonzero entries (>= 1; d_ext
-// holds 1s on entry).  The scan runs in warp tasks: block b has
+// extents d_dims[b*n2 ..]) that keeps all its nonzero entries, 0 for a block of
+// zeros (d_ext holds 0s on entry).  The scan runs in warp tasks: block b has
 // block_extent_tasks(d0, cols, ...) of them (d0 = its first extent, cols =
 // the product of the others), starting at d_task_begin[b]; d_task_begin has
 // nblocks + 1 entries, the last = ntasks.  budget: elements per task, 512 to
