@@ -108,19 +108,20 @@ __device__ __noinline__ void sum_cluster_tile(double* smem, double* cbase, int M
 }
 
 // One CTA of the tiled GEMM: tile lt of C block cb, k-segment seg of splitk.
-// With splitk > 1 and partial NULL the tile's segments are the CTAs of one cluster:
-// each leaves its partial tile in its own shared memory (the pipeline's buffers,
-// free by then) and every CTA sums a slice of the tile over all of them, in
-// segment order, through distributed shared memory.  Otherwise the BMC x BNC
-// tile goes to the CTA's part_elems of partial (column-major), for k_splitk_reduce.
+// With splitk > 1 the tile's segments are the CTAs of one cluster: each leaves its
+// partial tile in its own shared memory (the pipeline's buffers, free by then)
+// and every CTA sums a slice of the tile over all of them, in segment order,
+// through distributed shared memory.  PARTS: the BMC x BNC tile goes to pt
+// (column-major), for k_splitk_reduce; kernels of their own, since with both in
+// one the chi = 600 H_eff apply took 255 us instead of 251.
 // BM x BN is the staged (shared-memory) tile; the C tile BMC x BNC may be
 // narrower (48 of 64 rows or columns: the operand copies past BMC / BNC are
 // zero-filled without reading memory, and no warp multiplies them).
-template <int BM, int BN, int WM, int WN, bool XT, bool YT, int BK, int ST, int BMC = BM, int BNC = BN>
+template <bool PARTS, int BM, int BN, int WM, int WN, bool XT, bool YT, int BK, int ST, int BMC = BM, int BNC = BN>
 __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const double* __restrict__ Y,
                                          double* __restrict__ C, const GemmCBlock& cb,
                                          const GemmPair* __restrict__ pairs, int lt, int seg, int32_t splitk,
-                                         double* __restrict__ partial, int part_elems, double* smem) {
+                                         double* __restrict__ pt, double* smem) {
   constexpr int kBK = BK;
   constexpr int kStages = ST;
   using TL = TileLayout<BM, BN, XT, YT, BK, ST>;
@@ -290,8 +291,8 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
   double* cbase = C + cb.c_off;
   if (splitk > 1) {
     static_assert(BMC * BNC <= ST * (TL::XSZ + TL::YSZ), "the partial tile must fit in the pipeline's buffers");
-    double* const tile = partial ? partial + static_cast<int64_t>(blockIdx.x) * part_elems : smem;
-    if (!partial) __syncthreads();  // every warp has read its last operand tile
+    double* const tile = PARTS ? pt : smem;
+    if (!PARTS) __syncthreads();  // every warp has read its last operand tile
 #pragma unroll
     for (int a = 0; a < MT; ++a) {
       const int rl = wm * WM + a * 8 + g;
@@ -302,7 +303,7 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
         tile[rl + (cl + 1) * BMC] = acc[a][b][1];
       }
     }
-    if (!partial) sum_cluster_tile<BMC, BNC, NT>(smem, cbase, M, N, cb.ldc, m0, n0, seg, splitk);
+    if constexpr (!PARTS) sum_cluster_tile<BMC, BNC, NT>(smem, cbase, M, N, cb.ldc, m0, n0, seg, splitk);
     return;
   }
 #pragma unroll
@@ -326,23 +327,24 @@ __device__ __forceinline__ void gemm_cta(const double* __restrict__ X, const dou
 // running at the same time work on the same K range of neighbouring tiles and
 // find each other's operand panels in L2: R*T3 at chi = 2048 takes 1911 us,
 // 2010 in clusters.
-__device__ __forceinline__ void split_cta(int32_t splitk, int32_t ntiles, const double* partial, int& bid, int& seg) {
+template <bool PARTS>
+__device__ __forceinline__ void split_cta(int32_t splitk, int32_t ntiles, int& bid, int& seg) {
   const int b = static_cast<int>(blockIdx.x);
-  bid = partial ? b % ntiles : b / splitk;
-  seg = partial ? b / ntiles : b % splitk;
+  bid = PARTS ? b % ntiles : b / splitk;
+  seg = PARTS ? b / ntiles : b % splitk;
 }
 
-template <int BM, int BN, int WM, int WN, bool XT, bool YT, int BK = kBK, int ST = kStages>
+template <bool PARTS, int BM, int BN, int WM, int WN, bool XT, bool YT, int BK = kBK, int ST = kStages>
 __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32, 512 / ((BM / WM) * (BN / WN) * 32))
     k_gemm_f64(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ C,
                const GemmCBlock* __restrict__ cblocks, int32_t ncb, const GemmPair* __restrict__ pairs,
                int32_t splitk, int32_t ntiles, double* __restrict__ partial) {
   extern __shared__ double smem[];
   int bid, seg;
-  split_cta(splitk, ntiles, partial, bid, seg);
+  split_cta<PARTS>(splitk, ntiles, bid, seg);
   const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
-  gemm_cta<BM, BN, WM, WN, XT, YT, BK, ST>(X, Y, C, cb, pairs, bid - cb.tile_begin, seg, splitk, partial,
-                                           BM * BN, smem);
+  double* const pt = PARTS ? partial + static_cast<int64_t>(blockIdx.x) * (BM * BN) : nullptr;
+  gemm_cta<PARTS, BM, BN, WM, WN, XT, YT, BK, ST>(X, Y, C, cb, pairs, bid - cb.tile_begin, seg, splitk, pt, smem);
 }
 
 // Five tile shapes in one launch (launch_gemm_f64_edges): the tiles of every
@@ -353,26 +355,27 @@ __global__ void __launch_bounds__((BM / WM) * (BN / WN) * 32, 512 / ((BM / WM) *
 // Partial tiles are kEdgePart doubles apart whatever their shape.
 constexpr int kEdgeThreads = 128;
 constexpr int kEdgePart = 64 * 64;
-template <bool XT, bool YT>
+template <bool PARTS, bool XT, bool YT>
 __global__ void __launch_bounds__(kEdgeThreads, 4)
     k_gemm_f64_edges(const double* __restrict__ X, const double* __restrict__ Y, double* __restrict__ C,
                      const GemmCBlock* __restrict__ cblocks, int32_t ncb, const GemmPair* __restrict__ pairs,
                      int32_t splitk, int32_t ntiles, double* __restrict__ partial) {
   extern __shared__ double smem[];
   int bid, seg;
-  split_cta(splitk, ntiles, partial, bid, seg);
+  split_cta<PARTS>(splitk, ntiles, bid, seg);
   const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
+  double* const pt = PARTS ? partial + static_cast<int64_t>(blockIdx.x) * kEdgePart : nullptr;
   const int lt = bid - cb.tile_begin;
   if (cb.tshape == 0)
-    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
+    gemm_cta<PARTS, 64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, pt, smem);
   else if (cb.tshape == 1)
-    gemm_cta<64, 32, 32, 16, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
+    gemm_cta<PARTS, 64, 32, 32, 16, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, pt, smem);
   else if (cb.tshape == 2)
-    gemm_cta<32, 64, 16, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
+    gemm_cta<PARTS, 32, 64, 16, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, lt, seg, splitk, pt, smem);
   else if (cb.tshape == 3)
-    gemm_cta<64, 64, 32, 24, XT, YT, kBK, kStages, 64, 48>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
+    gemm_cta<PARTS, 64, 64, 32, 24, XT, YT, kBK, kStages, 64, 48>(X, Y, C, cb, pairs, lt, seg, splitk, pt, smem);
   else
-    gemm_cta<64, 64, 24, 32, XT, YT, kBK, kStages, 48, 64>(X, Y, C, cb, pairs, lt, seg, splitk, partial, kEdgePart, smem);
+    gemm_cta<PARTS, 64, 64, 24, 32, XT, YT, kBK, kStages, 48, 64>(X, Y, C, cb, pairs, lt, seg, splitk, pt, smem);
 }
 
 // Deterministic split-K reduction: C tile = sum over segments in order.
@@ -440,23 +443,26 @@ cudaError_t launch_t(const double* X, const double* Y, double* C, const GemmCBlo
                      const GemmPair* pr, int64_t ntiles, int splitk, double* partial, cudaStream_t s) {
   constexpr int threads = (BM / WM) * (BN / WN) * 32;
   constexpr int smem = TileLayout<BM, BN, XT, YT, BK, ST>::bytes();
-  auto kern = k_gemm_f64<BM, BN, WM, WN, XT, YT, BK, ST>;
+  auto clusters = k_gemm_f64<false, BM, BN, WM, WN, XT, YT, BK, ST>;
+  auto partials = k_gemm_f64<true, BM, BN, WM, WN, XT, YT, BK, ST>;
   static std::atomic<unsigned long long> configured{0};  // one bit per device ordinal (host threads may race)
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(configured & bit)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(clusters, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(clusters, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(partials, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
   if (ntiles <= 0) return cudaSuccess;
   if (splitk < 1 || (!partial && splitk > kMaxSplitK) || ntiles * splitk > 0x7fffffffLL) return cudaErrorInvalidValue;
   const int32_t nt = static_cast<int32_t>(ntiles);
-  e = launch_split(kern, ntiles, splitk, !partial, threads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
+  e = launch_split(partial ? partials : clusters, ntiles, splitk, !partial, threads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
   if (e != cudaSuccess || !partial) return e;
   const unsigned g = static_cast<unsigned>(std::min<int64_t>((ntiles * BM * BN + 255) / 256, 148LL * 64));
   k_splitk_reduce<BM, BN><<<g, 256, 0, s>>>(C, cb, ncb, splitk, nt, partial);
@@ -485,7 +491,7 @@ __global__ void __launch_bounds__(128, 4)
   if (flag && *flag == 0) return;
   for (int bid = static_cast<int>(blockIdx.x); bid < ntiles; bid += static_cast<int>(gridDim.x)) {
     const GemmCBlock cb = cblocks[tile_cblock_warp(cblocks, ncb, bid)];
-    gemm_cta<64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, bid - cb.tile_begin, 0, 1, nullptr, 0, smem);
+    gemm_cta<false, 64, 64, 32, 32, XT, YT, kBK, kStages>(X, Y, C, cb, pairs, bid - cb.tile_begin, 0, 1, nullptr, smem);
     __syncthreads();  // the operand buffers are refilled by the next tile
   }
 }
@@ -984,21 +990,24 @@ cudaError_t launch_edges_t(const double* X, const double* Y, double* C, const Ge
                            const GemmPair* pr, int64_t ntiles, int splitk, double* partial, cudaStream_t s) {
   constexpr int smem = std::max(std::max(TileLayout<64, 64, XT, YT>::bytes(), TileLayout<64, 32, XT, YT>::bytes()),
                                 TileLayout<32, 64, XT, YT>::bytes());
-  auto kern = k_gemm_f64_edges<XT, YT>;
+  auto clusters = k_gemm_f64_edges<false, XT, YT>;
+  auto partials = k_gemm_f64_edges<true, XT, YT>;
   static std::atomic<unsigned long long> configured{0};  // one bit per device ordinal (host threads may race)
   int dev = 0;
   cudaError_t e = cudaGetDevice(&dev);
   if (e != cudaSuccess) return e;
   const unsigned long long bit = 1ull << (dev & 63);
   if (!(configured & bit)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    e = cudaFuncSetAttribute(clusters, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    e = cudaFuncSetAttribute(clusters, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    e = cudaFuncSetAttribute(partials, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
     configured.fetch_or(bit);
   }
   const int32_t nt = static_cast<int32_t>(ntiles);
-  e = launch_split(kern, ntiles, splitk, !partial, kEdgeThreads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
+  e = launch_split(partial ? partials : clusters, ntiles, splitk, !partial, kEdgeThreads, smem, s, X, Y, C, cb, ncb, pr, splitk, nt, partial);
   if (e != cudaSuccess || !partial) return e;
   const unsigned g = static_cast<unsigned>(std::min<int64_t>((ntiles * kEdgePart + 255) / 256, 148LL * 64));
   k_splitk_reduce_edges<<<g, 256, 0, s>>>(C, cb, ncb, splitk, nt, partial);
