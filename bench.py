@@ -155,14 +155,15 @@ def measured_hbm_gbs():
         return 6650.0
 
 
-# DRAM bytes (read + write) per launch from one ncu capture of this bench at the
-# given chi (--metrics dram__bytes_read.sum,dram__bytes_write.sum), averaged
+# DRAM bytes (read + write) per launch from one ncu capture of the H_eff apply at
+# the given chi (--metrics dram__bytes_read.sum,dram__bytes_write.sum), averaged
 # over the captured launches of each kernel.  A constant of that capture (its
 # date below), not a measurement of this run: it goes stale when the kernel
 # changes.
 TRAFFIC = {
-    (2048, "k_gemm_i8"): (913.0e6, "ncu capture of 2026-12-05, mean of the psi*L and R*T3 launches"),
-    (2048, "k_gemm_thin"): (1315.3e6, "ncu capture of 2026-12-03, mean of the T1*W1 and T2*W2 launches"),
+    (2048, "k_gemm_f64"): (1180.8e6, "ncu capture of 2026-12-05, mean of the psi*L and R*T3 launches, without the "
+                                     "split-K sums (160.5e6)"),
+    (2048, "k_gemm_thin"): (1315.6e6, "ncu capture of 2026-12-05, mean of the T1*W1 and T2*W2 launches"),
 }
 
 
@@ -974,14 +975,12 @@ def run_ours(args, world, rank, local):
                    "parallelism": f"replicas x{world}" if world > 1 else "single GPU",
                    "l2": "inputs larger than L2 (operators ~0.6 GB, intermediates ~2.3 GB each)"},
         "gflops_algorithmic": flops_alg * value / 1e9,
-        "roofline": {"bound": "tensor", "kernel": "k_gemm_i8 (tcgen05.mma kind::i8, 34 exact digit products per FP64 "
-                                                       "multiply-add; steps psi*L and R*T3; DMMA k_gemm_f64_edges where "
-                                                       "that is the faster, as at small chi)",
+        "roofline": {"bound": "tensor", "kernel": "k_gemm_f64_edges (DMMA m8n8k4, 64x64 tiles with 64x32 / 64x48 / "
+                                                       "32x64 / 48x64 edge tiles; steps psi*L and R*T3)",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak if peak else None,
-                     "peak_source": "measured live: torch.matmul float64 8192^3, best of 10 (cuBLAS DGEMM, DMMA; the "
-                                    "integer tensor cores can exceed it)",
+                     "peak_source": "measured live: torch.matmul float64 8192^3, best of 10 (cuBLAS DGEMM)",
                      "flops_per_launch": g["flops"] / max(g["launches"], 1),
-                     "traffic": traffic_per_launch(args.chi, "k_gemm_i8"), "launches": g["launches"],
+                     "traffic": traffic_per_launch(args.chi, "k_gemm_f64"), "launches": g["launches"],
                      "kernel_ms_per_step": g["ms"] / args.steps},
         "roofline_mpo_steps": {"bound": "hbm", "kernel": "k_gemm_thin_p (steps T1*W1 and T2*W2, K <= 16)",
                                "achieved": thin_gbs, "peak": hbm_peak, "unit": "GB/s",
